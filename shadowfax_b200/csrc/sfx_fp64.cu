@@ -5,8 +5,9 @@
  * This translation unit is compiled with -fmad=false (no a*b+c contraction)
  * and IEEE division / square root, and keeps the reference's expression
  * order, so each value is rounded exactly as the reference rounds it.  pow()
- * is sfx_pow (sfx_pow.h), shared with the CPU oracle, because glibc's and
- * CUDA's pow differ in the last bit.
+ * has the values of sfx_pow (sfx_pow.h), shared with the CPU oracle, because
+ * glibc's and CUDA's pow differ in the last bit; it is evaluated by sfx_powq
+ * (sfx_powq.h).
  *
  * Kernels (one step = three or four launches):
  *   k_gradients  one thread per cell: VorCell::estimate_gradient
@@ -27,7 +28,14 @@
 
 #include "sfx_internal.h"
 #include "sfx_limiter.h"
-#include "sfx_pow.h"
+
+/* sfx_pow for the arguments sfx_powq does not settle, out of line */
+__host__ __device__ __noinline__ double sfx_pow_rare64(double x, double y);
+#define SFX_POWQ_RARE sfx_pow_rare64
+#include "sfx_powq.h"
+__host__ __device__ __noinline__ double sfx_pow_rare64(double x, double y) {
+    return sfx_pow(x, y);
+}
 
 namespace {
 
@@ -445,15 +453,49 @@ __device__ __forceinline__ double sound(const sfx_solver_params& s, const double
     return W[0] != 0. ? sqrt(s.gamma * W[D + 1] / W[0]) : 0.;
 }
 
+/* The solver's powers, sfx_pow's values (sfx_powq.h) in two out-of-line parts:
+ * ln x as a pair, and x^y from it.  The iteration takes several powers of one
+ * ratio p / p_K (f, f', the sampling), which share the logarithm.  Out of line
+ * because the solver has some twenty power sites: inlined, its code overran
+ * the instruction cache (21.5 of 27 stall cycles per issue were instruction
+ * fetch; 807,000 random-field faces took 6.1 ms, now 0.82 ms). */
+struct LogPair {
+    double x, h, l; /* h is NaN where x is not a positive normal number */
+};
+
+__device__ __noinline__ LogPair xlog(double x) {
+    LogPair p;
+    p.x = x;
+    p.l = 0.;
+    if(!sfx_powq_log(x, &p.h, &p.l)) p.h = __longlong_as_double(0x7ff8000000000000ll);
+    return p;
+}
+
+__device__ __noinline__ double xexp(LogPair p, double y) {
+    const double th = y * p.h;
+    const double tl = sfx_fma(y, p.h, -th) + y * p.l;
+    double r;
+    if(fabs(th) < 22. && sfx_powq_exp(th, tl, &r)) return r;
+    return sfx_pow_rare64(p.x, y);
+}
+
+__device__ __forceinline__ double xpow(double x, double y) {
+    return xexp(xlog(x), y);
+}
+
+/* f_K(p) and, on a rarefaction side, ln(p / p_K) and z_K = (p/p_K)^((g-1)/(2g)) */
 template <int D>
-__device__ __forceinline__ double fb(const sfx_solver_params& s, double p,
-                                     const double* Wb, double a) {
+__device__ __forceinline__ double fb(const sfx_solver_params& s, double p, const double* Wb,
+                                     double a, double* z, LogPair* lr) {
     if(p > Wb[D + 1]) {
         double A = s.tdgp1 / Wb[0];
         double B = s.gm1dgp1 * Wb[D + 1];
+        *z = 0.;
         return (p - Wb[D + 1]) * sqrt(A / (p + B));
     }
-    return s.tdgm1 * a * (sfx_pow(p / Wb[D + 1], s.gm1d2g) - 1.);
+    *lr = xlog(p / Wb[D + 1]);
+    *z = xexp(*lr, s.gm1d2g);
+    return s.tdgm1 * a * (*z - 1.);
 }
 
 template <int D>
@@ -464,64 +506,44 @@ __device__ __forceinline__ double gbf(const sfx_solver_params& s, double p,
     return sqrt(A / (p + B));
 }
 
+/* f_K'(p), with lr = ln(p / p_K) on a rarefaction side */
 template <int D>
 __device__ __forceinline__ double fprimeb(const sfx_solver_params& s, double p,
-                                          const double* Wb, double a) {
+                                          const double* Wb, double a, const LogPair& lr) {
     if(p > Wb[D + 1]) {
         double A = s.tdgp1 / Wb[0];
         double B = s.gm1dgp1 * Wb[D + 1];
         return (1. - 0.5 * (p - Wb[D + 1]) / (B + p)) * sqrt(A / (p + B));
     }
-    return 1. / (Wb[0] * a) * sfx_pow(p / Wb[D + 1], -s.gp1d2g);
-}
-
-template <int D>
-__device__ __forceinline__ double ff(const sfx_solver_params& s, double p,
-                                     const double* WL, const double* WR,
-                                     double vL, double vR, double aL, double aR) {
-    return fb<D>(s, p, WL, aL) + fb<D>(s, p, WR, aR) + (vR - vL);
+    return 1. / (Wb[0] * a) * xexp(lr, -s.gp1d2g);
 }
 
 /* The last f(p) of the iteration, per side, with its power
- * sfx_pow(p / p_K, (g-1)/(2g)) on a rarefaction side.  The reference
- * evaluates f_K(p) again for the wave velocity and that power again for the
- * sampling at the same p (ExactRiemannSolver.cpp:207-265): the kept values
- * are the same operations on the same operands, so reusing them changes no
- * bit and saves the double-double powers. */
+ * sfx_pow(p / p_K, (g-1)/(2g)) and the ratio's logarithm on a rarefaction
+ * side.  The reference evaluates f_K(p) again for the wave velocity and that
+ * power again for the sampling at the same p (ExactRiemannSolver.cpp:207-265):
+ * the kept values are the same operations on the same operands, so reusing
+ * them changes no bit. */
 struct FLast {
     double p, fL, fR, zL, zR;
-    bool ok;
+    LogPair lL, lR;
 };
-
-template <int D>
-__device__ __forceinline__ double fbz(const sfx_solver_params& s, double p, const double* Wb,
-                                      double a, double* z) {
-    if(p > Wb[D + 1]) {
-        double A = s.tdgp1 / Wb[0];
-        double B = s.gm1dgp1 * Wb[D + 1];
-        *z = 0.;
-        return (p - Wb[D + 1]) * sqrt(A / (p + B));
-    }
-    *z = sfx_pow(p / Wb[D + 1], s.gm1d2g);
-    return s.tdgm1 * a * (*z - 1.);
-}
 
 template <int D>
 __device__ __forceinline__ double ffl(const sfx_solver_params& s, double p, const double* WL,
                                       const double* WR, double vL, double vR, double aL,
                                       double aR, FLast& c) {
     c.p = p;
-    c.fL = fbz<D>(s, p, WL, aL, &c.zL);
-    c.fR = fbz<D>(s, p, WR, aR, &c.zR);
-    c.ok = true;
+    c.fL = fb<D>(s, p, WL, aL, &c.zL, &c.lL);
+    c.fR = fb<D>(s, p, WR, aR, &c.zR, &c.lR);
     return c.fL + c.fR + (vR - vL);
 }
 
 template <int D>
-__device__ __forceinline__ double fprime(const sfx_solver_params& s, double p,
-                                         const double* WL, const double* WR,
-                                         double aL, double aR) {
-    return fprimeb<D>(s, p, WL, aL) + fprimeb<D>(s, p, WR, aR);
+__device__ __forceinline__ double fprime(const sfx_solver_params& s, const double* WL,
+                                         const double* WR, double aL, double aR,
+                                         const FLast& c) {
+    return fprimeb<D>(s, c.p, WL, aL, c.lL) + fprimeb<D>(s, c.p, WR, aR, c.lR);
 }
 
 /* ExactRiemannSolver.cpp:644-673 */
@@ -540,8 +562,8 @@ __device__ double guess_p(const sfx_solver_params& s, const double* WL,
     if(qmax <= 2. && pmin <= ppv && ppv <= pmax) {
         pguess = ppv;
     } else if(ppv < pmin) {
-        pguess = sfx_pow((aL + aR - s.gm1d2 * (vR - vL)) /
-                                 (aL / sfx_pow(pL, s.gm1d2g) + aR / sfx_pow(pR, s.gm1d2g)),
+        pguess = xpow((aL + aR - s.gm1d2 * (vR - vL)) /
+                                 (aL / xpow(pL, s.gm1d2g) + aR / xpow(pR, s.gm1d2g)),
                          s.tgdgm1);
     } else {
         const double gL = gbf<D>(s, ppv, WL), gR = gbf<D>(s, ppv, WR);
@@ -551,20 +573,18 @@ __device__ double guess_p(const sfx_solver_params& s, const double* WL,
     return (fl < pguess) ? pguess : fl;
 }
 
-/* ExactRiemannSolver.cpp:462-546, capped at SFX_MAX_ITER steps */
+/* ExactRiemannSolver.cpp:462-546, capped at SFX_MAX_ITER steps.  The limits'
+ * function values fa and fbv come from the caller, which has evaluated f at
+ * both of them. */
 template <int D>
 __device__ double brent(const sfx_solver_params& s, double lowerLimit,
-                        double upperLimit, double errorTol, const double* WL,
-                        const double* WR, double vL, double vR, double aL,
-                        double aR, int* iters, int* errexit, int* noconv) {
+                        double upperLimit, double fa, double fbv, double errorTol,
+                        const double* WL, const double* WR, double vL, double vR, double aL,
+                        double aR, FLast& last, int& iters, bool& errexit, bool& noconv) {
     double a = lowerLimit, b = upperLimit, c = 0., d = 1e230;
-    double fa = ff<D>(s, a, WL, WR, vL, vR, aL, aR);
-    double fbv = ff<D>(s, b, WL, WR, vL, vR, aL, aR);
     double fc = 0., sv = 0., fs = 0.;
-    *iters = 0;
-    *errexit = 0;
     if(fa * fbv >= 0) {
-        *errexit = 1;
+        errexit = true;
         return (fa < fbv) ? a : b;
     }
     if(fabs(fa) < fabs(fbv)) {
@@ -579,11 +599,11 @@ __device__ double brent(const sfx_solver_params& s, double lowerLimit,
     fc = fa;
     bool mflag = true;
     while(!(fbv == 0) && (fabs(a - b) > errorTol * (a + b) * 0.5)) {
-        if(*iters >= SFX_MAX_ITER) {
-            *noconv = 1;
+        if(iters >= SFX_MAX_ITER) {
+            noconv = true;
             break;
         }
-        ++*iters;
+        ++iters;
         if((fa != fc) && (fbv != fc))
             sv = a * fbv * fc / (fa - fbv) / (fa - fc) +
                  b * fa * fc / (fbv - fa) / (fbv - fc) +
@@ -601,7 +621,7 @@ __device__ double brent(const sfx_solver_params& s, double lowerLimit,
         } else {
             mflag = false;
         }
-        fs = ff<D>(s, sv, WL, WR, vL, vR, aL, aR);
+        fs = ffl<D>(s, sv, WL, WR, vL, vR, aL, aR, last);
         d = c;
         c = b;
         fc = fbv;
@@ -638,19 +658,19 @@ __device__ __forceinline__ bool bad_state(const double* sol) {
 template <int D>
 __device__ __forceinline__ void fan_left(double g, const double* WL, double vL,
                                          double aL, double* sol, double* vhalf) {
-    sol[0] = WL[0] * sfx_pow(2. / (g + 1.) + (g - 1.) / (g + 1.) / aL * vL, 2. / (g - 1.));
+    const LogPair base = xlog(2. / (g + 1.) + (g - 1.) / (g + 1.) / aL * vL);
+    sol[0] = WL[0] * xexp(base, 2. / (g - 1.));
     *vhalf = 2. / (g + 1.) * (aL + 0.5 * (g - 1.) * vL) - vL;
-    sol[D + 1] = WL[D + 1] *
-                 sfx_pow(2. / (g + 1.) + (g - 1.) / (g + 1.) / aL * vL, 2. * g / (g - 1.));
+    sol[D + 1] = WL[D + 1] * xexp(base, 2. * g / (g - 1.));
 }
 
 template <int D>
 __device__ __forceinline__ void fan_right(double g, const double* WR, double vR,
                                           double aR, double* sol, double* vhalf) {
-    sol[0] = WR[0] * sfx_pow(2. / (g + 1.) - (g - 1.) / (g + 1.) / aR * vR, 2. / (g - 1.));
+    const LogPair base = xlog(2. / (g + 1.) - (g - 1.) / (g + 1.) / aR * vR);
+    sol[0] = WR[0] * xexp(base, 2. / (g - 1.));
     *vhalf = 2. / (g + 1.) * (-aR + 0.5 * (g - 1.) * vR) - vR;
-    sol[D + 1] = WR[D + 1] *
-                 sfx_pow(2. / (g + 1.) - (g - 1.) / (g + 1.) / aR * vR, 2. * g / (g - 1.));
+    sol[D + 1] = WR[D + 1] * xexp(base, 2. * g / (g - 1.));
 }
 
 /* vacuum sampling shared by ExactRiemannSolver::solve_vacuum
@@ -765,54 +785,48 @@ __device__ ExactOut exact_solve(const sfx_solver_params& s, double* WL, double* 
     const double tol = s.tol;
     double p = 0.;
     double pguess = guess_p<D>(s, WL, WR, vL, vR, aL, aR);
+    FLast last;
+    last.lL = last.lR = LogPair{0., 0., 0.};
     /* f(0): on both sides the rarefaction branch with sfx_pow(0, e) = +0
      * (e > 0), i.e. (2/(g-1) a_K) * (0 - 1) exactly */
     const double fp = WL[D + 1] > 0. && WR[D + 1] > 0.
                               ? s.tdgm1 * aL * (0. - 1.) + s.tdgm1 * aR * (0. - 1.) + (vR - vL)
-                              : ff<D>(s, p, WL, WR, vL, vR, aL, aR);
-    FLast last;
-    last.ok = false;
+                              : ffl<D>(s, p, WL, WR, vL, vR, aL, aR, last);
     double fpguess = ffl<D>(s, pguess, WL, WR, vL, vR, aL, aR, last);
-    int newton = 0, brent_it = 0, errexit = 0, noconv = 0, mode;
-    if(fp < s.cutoff) {
-        mode = 1 << 3;
-        while(fabs(p - pguess) > tol * 0.5 * (p + pguess)) {
+    int newton = 0, brent_it = 0, mode;
+    bool errexit = false, noconv = false;
+    /* The reference has one Newton loop per mode: below the cutoff it runs to
+     * the tolerance with p kept non-negative; above it, only while f < 0 (and
+     * not at all when f(0) and f(guess) differ in sign).  One loop here. */
+    const bool only_newton = fp < s.cutoff;
+    if(only_newton || fp * fpguess >= 0.) {
+        while(fabs(p - pguess) > tol * 0.5 * (p + pguess) && (only_newton || fpguess < 0.)) {
             if(newton >= SFX_MAX_ITER) {
-                noconv = 1;
+                noconv = true;
                 break;
             }
             ++newton;
             p = pguess;
-            pguess = pguess - fpguess / fprime<D>(s, pguess, WL, WR, aL, aR);
-            if(pguess < 0.) pguess = 0.;
+            pguess = pguess - fpguess / fprime<D>(s, WL, WR, aL, aR, last);
+            if(only_newton && pguess < 0.) pguess = 0.;
             fpguess = ffl<D>(s, pguess, WL, WR, vL, vR, aL, aR, last);
         }
+    }
+    if(only_newton) {
+        mode = 1 << 3;
         p = pguess;
     } else {
         mode = 2 << 3;
-        if(fp * fpguess >= 0.) {
-            while(fabs(p - pguess) > tol * 0.5 * (p + pguess) && fpguess < 0.) {
-                if(newton >= SFX_MAX_ITER) {
-                    noconv = 1;
-                    break;
-                }
-                ++newton;
-                p = pguess;
-                pguess = pguess - fpguess / fprime<D>(s, pguess, WL, WR, aL, aR);
-                fpguess = ffl<D>(s, pguess, WL, WR, vL, vR, aL, aR, last);
-            }
-        }
         if(!noconv && fabs(p - pguess) > tol * 0.5 * (p + pguess) && fpguess > 0.) {
             mode = 3 << 3;
-            p = brent<D>(s, 0., pguess, tol, WL, WR, vL, vR, aL, aR, &brent_it,
-                         &errexit, &noconv);
+            p = brent<D>(s, 0., pguess, fp, fpguess, tol, WL, WR, vL, vR, aL, aR, last, brent_it,
+                         errexit, noconv);
         } else {
             p = pguess;
         }
     }
-    const bool at_p = last.ok && last.p == p;
-    const double u = 0.5 * (vL + vR) + 0.5 * ((at_p ? last.fR : fb<D>(s, p, WR, aR)) -
-                                             (at_p ? last.fL : fb<D>(s, p, WL, aL)));
+    if(last.p != p) ffl<D>(s, p, WL, WR, vL, vR, aL, aR, last);
+    const double u = 0.5 * (vL + vR) + 0.5 * (last.fR - last.fL);
     double vhalf;
     int region;
     if(u < 0) {
@@ -833,14 +847,15 @@ __device__ ExactOut exact_solve(const sfx_solver_params& s, double* WL, double* 
         } else {
             const double SHR = vR + aR;
             if(SHR > 0) {
-                const double STR = u + aR * (at_p ? last.zR : sfx_pow(pdpR, s.gm1d2g));
+                const double STR = u + aR * last.zR;
                 if(STR <= 0) {
-                    sol[0] = WR[0] * sfx_pow(s.tdgp1 - s.gm1dgp1 / aR * vR, s.tdgm1);
+                    const LogPair base = xlog(s.tdgp1 - s.gm1dgp1 / aR * vR);
+                    sol[0] = WR[0] * xexp(base, s.tdgm1);
                     vhalf = s.tdgp1 * (-aR + s.gm1d2 * vR) - vR;
-                    sol[D + 1] = WR[D + 1] * sfx_pow(s.tdgp1 - s.gm1dgp1 / aR * vR, s.tgdgm1);
+                    sol[D + 1] = WR[D + 1] * xexp(base, s.tgdgm1);
                     region = SFX_BRANCH_S_RFAN;
                 } else {
-                    sol[0] = WR[0] * sfx_pow(pdpR, s.ginv);
+                    sol[0] = WR[0] * xexp(last.lR, s.ginv);
                     sol[D + 1] = p;
                     vhalf = u - vR;
                     region = SFX_BRANCH_S_RRARE_STAR;
@@ -868,14 +883,15 @@ __device__ ExactOut exact_solve(const sfx_solver_params& s, double* WL, double* 
         } else {
             const double SHL = vL - aL;
             if(SHL < 0) {
-                const double STL = u - aL * (at_p ? last.zL : sfx_pow(pdpL, s.gm1d2g));
+                const double STL = u - aL * last.zL;
                 if(STL > 0) {
-                    sol[0] = WL[0] * sfx_pow(s.tdgp1 + s.gm1dgp1 / aL * vL, s.tdgm1);
+                    const LogPair base = xlog(s.tdgp1 + s.gm1dgp1 / aL * vL);
+                    sol[0] = WL[0] * xexp(base, s.tdgm1);
                     vhalf = s.tdgp1 * (aL + s.gm1d2 * vL) - vL;
-                    sol[D + 1] = WL[D + 1] * sfx_pow(s.tdgp1 + s.gm1dgp1 / aL * vL, s.tgdgm1);
+                    sol[D + 1] = WL[D + 1] * xexp(base, s.tgdgm1);
                     region = SFX_BRANCH_S_LFAN;
                 } else {
-                    sol[0] = WL[0] * sfx_pow(pdpL, s.ginv);
+                    sol[0] = WL[0] * xexp(last.lL, s.ginv);
                     vhalf = u - vL;
                     sol[D + 1] = p;
                     region = SFX_BRANCH_S_LRARE_STAR;
