@@ -128,6 +128,11 @@ int setup_self(sfx_mesh* m, cudaStream_t s) {
     return h2d(m->self_tab, &e, 1, s);
 }
 
+/* doubles of one of the plain-FP64 pass's records */
+size_t rec_doubles(int dim, int what) {
+    return (size_t)sfx_fp64_record_bytes(dim, what) / sizeof(double);
+}
+
 int run_phase(sfx_mesh* m, int phase, double dt, int write_branch, cudaStream_t s) {
     sfx_ctx* c = m->ctx;
     if(c->cfg.precision == SFX_PREC_SPLIT) {
@@ -160,7 +165,7 @@ int run_phase(sfx_mesh* m, int phase, double dt, int write_branch, cudaStream_t 
     }
     switch(phase) {
     case 0:
-        return sfx_fp64_gradients(&m->d, s);
+        return sfx_fp64_gradients(&m->d, &c->sp, s);
     case 1:
         return sfx_fp64_faces(&m->d, &c->sp, dt, write_branch, s);
     default:
@@ -179,6 +184,34 @@ int reset_err_on(sfx_mesh* m, cudaStream_t s) {
 int reset_err(sfx_mesh* m) {
     return reset_err_on(m, m->ctx->stream);
 }
+
+/* Arrays carved from one device block (256-byte aligned each): a mesh has
+ * about thirty, and an allocation of its own for each cost more than the
+ * copies that fill them on small meshes. */
+struct Carver {
+    struct Slot {
+        void** p;
+        size_t bytes;
+    };
+    std::vector<Slot> slots;
+    template <typename T>
+    void add(T** p, size_t count) {
+        slots.push_back({(void**)p, (count ? count : 1) * sizeof(T)});
+    }
+    int allocate(sfx_mesh* m) {
+        size_t total = 0;
+        for(const Slot& sl : slots) total = ((total + 255) & ~(size_t)255) + sl.bytes;
+        uint8_t* block = nullptr;
+        SFX_TRY(dalloc(m, &block, total));
+        size_t off = 0;
+        for(const Slot& sl : slots) {
+            off = (off + 255) & ~(size_t)255;
+            *sl.p = block + off;
+            off += sl.bytes;
+        }
+        return SFX_OK;
+    }
+};
 
 /* a state on base's geometry: one device block carved into the arrays,
  * set up on stream s (waited for when `wait`) */
@@ -202,7 +235,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     sfx_dmesh& d = m->d;
     const int64_t n = d.n_cells, F = d.n_faces;
     const int S = d.S, dim = d.dim;
-    d.W = d.Q = d.grad = d.dQf = d.gterm = nullptr;
+    d.W = d.Q = d.dQf = d.ws = d.grec = nullptr;
     d.branch = nullptr;
     d.err = nullptr;
     d.totals_scratch = nullptr;
@@ -212,12 +245,8 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     d.slowq = nullptr;
     d.slowq_n = nullptr;
     d.slowq_cap = 0;
-    struct Slot {
-        void** p;
-        size_t bytes;
-    };
-    std::vector<Slot> slots;
-    auto A = [&](auto** p, size_t c) { slots.push_back({(void**)p, c * sizeof(**p)}); };
+    Carver arrays;
+    auto A = [&](auto** p, size_t c) { arrays.add(p, c); };
     A(&d.W, n * S);
     A(&d.Q, n * S);
     A(&d.err, 1);
@@ -234,26 +263,12 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
         A(&m->self_tab, 1);
         A(&m->self_pre, 6);
     } else {
-        A(&d.grad, n * dim * S);
-        if(d.gshare)
-            A(&d.gterm, F * sfx_grad_term_stride(dim));
-        else
-            A(&d.dQf, F * S);
+        A(&d.ws, n * rec_doubles(dim, SFX_REC_WS));
+        A(&d.grec, n * rec_doubles(dim, SFX_REC_GREC));
+        A(&d.dQf, F * rec_doubles(dim, SFX_REC_DQ));
         A(&d.branch, F);
     }
-    size_t total = 0;
-    for(const Slot& sl : slots) total = ((total + 255) & ~(size_t)255) + sl.bytes;
-    uint8_t* block = nullptr;
-    int rc = dalloc(m, &block, total);
-    if(!rc) {
-        size_t off = 0;
-        for(const Slot& sl : slots) {
-            off = (off + 255) & ~(size_t)255;
-            *sl.p = block + off;
-            off += sl.bytes;
-        }
-        if(d.gterm) d.dQf = d.gterm;
-    }
+    int rc = arrays.allocate(m);
     if(!rc) rc = reset_err_on(m, s);
     if(!rc && split) rc = cuda_ok(cudaMemsetAsync(d.slowq_n, 0, sizeof(int32_t), s));
     if(!rc && split) rc = setup_self(m, s);
@@ -374,20 +389,26 @@ int sfx_ctx_synchronize(sfx_ctx* ctx) {
 int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
                               int64_t nnz, int32_t precision) {
     const int64_t S = dim + 2, n = n_cells, F = n_faces;
-    int64_t cells = n * (8 * (2 * dim + 2 + 2 * S + dim * S) + 4) + 4;
-    int64_t faces = F * (8 * (1 + 3 * dim + S) + 4 * 4);
+    int64_t cells = n * (8 * (2 * dim + 2 + 2 * S) + 4) + 4;
+    int64_t faces = F * (8 * (1 + 2 * dim) + 4 * 4);
     int64_t bytes = cells + faces + nnz * 4 + 8 * 8 * 1024 + 4096;
-    if(precision != SFX_PREC_SPLIT) /* the gradient terms, dQf inside them; the
-                                       update's CSR copy (cells not in ascending
-                                       face order) */
-        bytes += F * 8 * (sfx_grad_term_stride(dim) - S) + nnz * 4;
+    if(precision != SFX_PREC_SPLIT) {
+        /* the records; the update's CSR copy (cells not in ascending face
+         * order); face velocities */
+        auto rec = [&](int what) { return (int64_t)sfx_fp64_record_bytes(dim, what); };
+        bytes += n * (rec(SFX_REC_WS) + rec(SFX_REC_GREC)) +
+                 F * (rec(SFX_REC_DQ) + rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO) + 8 * dim) +
+                 nnz * 4;
+    } else {
+        bytes += F * 8 * (dim + S); /* face velocities, dQf */
+    }
     if(precision == SFX_PREC_SPLIT) {
-        /* fg, fi, fsh, an, dqm, dqv, queue; cw, cg, cx, self table; nbe */
+        /* fg, fi, fsh, an, dqm, dqv, queue; cw, cg, cx, self table */
         bytes += F * (32 + 8 + 1 + 8 * dim + 8 + 8 * dim) + 4 * slowq_capacity(F) + 4;
         bytes += n * (32 + 16 * (sfx_split_grad_vec4((int)dim) + sfx_split_dwdt_vec4((int)dim)) +
                       16) + 256;
-        bytes += nnz * 4;
     }
+    bytes += nnz * 8; /* ent */
     return bytes;
 }
 
@@ -594,10 +615,8 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
                        sizeof(double) * dim) != 0)
             d.gshare = 0;
     const int S = d.S;
-    int rc = SFX_OK;
-    auto A = [&](auto** p, size_t c) {
-        if(rc == SFX_OK) rc = dalloc(m, p, c);
-    };
+    Carver arrays;
+    auto A = [&](auto** p, size_t c) { arrays.add(p, c); };
     A(&d.pos, n * dim);
     A(&d.cen, n * dim);
     A(&d.vol, n);
@@ -607,7 +626,6 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!aidx.empty()) A(&d.aidx, nnz);
     A(&d.W, n * S);
     A(&d.Q, n * S);
-    A(&d.grad, n * dim * S);
     A(&d.area, F);
     A(&d.mid, F * dim);
     A(&d.left, F);
@@ -616,12 +634,16 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     A(&d.rpos, F * dim);
     if(d.has_velocity) A(&d.vel, F * dim);
     const bool split = ctx->cfg.precision == SFX_PREC_SPLIT;
-    if(!split && d.gshare) {
-        A(&d.gterm, F * sfx_grad_term_stride(dim));
-        d.dQf = d.gterm;
+    if(!split) {
+        A(&d.ws, n * rec_doubles(dim, SFX_REC_WS));
+        A(&d.grec, n * rec_doubles(dim, SFX_REC_GREC));
+        A(&d.dQf, F * rec_doubles(dim, SFX_REC_DQ));
+        A(&d.ggeo, F * rec_doubles(dim, SFX_REC_GGEO));
+        A(&d.fgeo, F * rec_doubles(dim, SFX_REC_FGEO));
     } else {
         A(&d.dQf, F * S);
     }
+    A(&d.ent, nnz);
     A(&d.branch, F);
     A(&d.err, 1);
     A(&d.totals_scratch, (size_t)(S + 1) * 1024);
@@ -637,7 +659,6 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         A(&d.cg, (size_t)sfx_split_grad_vec4(dim) * n);
         A(&d.cdw, (size_t)sfx_split_dwdt_vec4(dim) * n);
         A(&d.cx, n);
-        A(&d.nbe, nnz);
         A(&d.an, (size_t)dim * F);
         A(&d.dqm, F);
         A(&d.dqv, (size_t)dim * F);
@@ -645,6 +666,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         A(&d.slowq, (size_t)d.slowq_cap);
         A(&d.slowq_n, 1);
     }
+    int rc = arrays.allocate(m);
     if(rc != SFX_OK) {
         sfx_mesh_free(m);
         return rc;
@@ -664,19 +686,6 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!rc) rc = h2d(d.idx, split ? idx_split.data() : idx.data(), nnz, s);
     if(!rc && !aidx.empty()) rc = h2d(d.aidx, aidx.data(), nnz, s);
     if(aidx.empty()) d.aidx = d.idx;
-    std::vector<int32_t> nbe;
-    if(split) {
-        /* the neighbour of each CSR entry, so the gradient kernel loads it
-         * beside the face id instead of after it */
-        nbe.resize(nnz);
-        for(int64_t j = 0; j < nnz; ++j) {
-            const uint32_t e = (uint32_t)idx_split[j];
-            const int32_t f = (int32_t)(e & 0x7fffffffu);
-            nbe[j] = (e >> 31) ? desc->face_left[f]
-                               : (desc->face_kind[f] == SFX_FACE_MIRROR ? -1 : desc->face_right[f]);
-        }
-        if(!rc) rc = h2d(d.nbe, nbe.data(), nnz, s);
-    }
     if(!rc) rc = h2d(d.area, desc->face_area, F, s);
     if(!rc) rc = h2d(d.mid, t3.data(), t3.size(), s);
     if(!rc) rc = h2d(d.left, desc->face_left, F, s);
@@ -688,8 +697,11 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!rc) rc = cuda_ok(cudaMemsetAsync(d.Q, 0, sizeof(double) * n * S, s));
     if(!rc) rc = reset_err(m);
     if(!rc && split) rc = cuda_ok(cudaMemsetAsync(d.slowq_n, 0, sizeof(int32_t), s));
+    if(!rc) rc = sfx_fp64_csr_neighbours(&d, s);
     if(!rc && split) rc = sfx_split_prepare(&d, s);
     if(!rc && split) rc = setup_self(m, s);
+    if(!rc && !split) rc = sfx_fp64_face_records(&d, s);
+    if(!rc && !split) rc = sfx_fp64_state_records(&d, s);
     /* host staging buffers go out of scope: wait for the copies */
     if(!rc) rc = cuda_ok(cudaStreamSynchronize(s));
     if(rc != SFX_OK) {
@@ -737,7 +749,10 @@ int sfx_state_upload_WQ(sfx_mesh* m, const double* W, const double* Q) {
     SFX_TRY(reset_err(m));
     SFX_TRY(h2d(m->d.W, t1.data(), t1.size(), s));
     SFX_TRY(h2d(m->d.Q, t2.data(), t2.size(), s));
-    if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_load_state(&m->d, s));
+    if(m->ctx->cfg.precision == SFX_PREC_SPLIT)
+        SFX_TRY(sfx_split_load_state(&m->d, s));
+    else
+        SFX_TRY(sfx_fp64_state_records(&m->d, s));
     return cuda_ok(cudaStreamSynchronize(s));
 }
 
@@ -868,29 +883,36 @@ int sfx_mesh_get_timesteps(sfx_mesh* m, uint64_t* start, uint64_t* end) {
     return cuda_ok(cudaStreamSynchronize(s));
 }
 
+/* the cells' gradient records [n][rec]: gradients [l][k] first */
+static int download_grec(sfx_mesh* m, std::vector<double>& t) {
+    cudaStream_t s = m->ctx->stream;
+    t.resize((size_t)m->d.n_cells * rec_doubles(m->d.dim, SFX_REC_GREC));
+    SFX_TRY(cuda_ok(cudaMemcpyAsync(t.data(), m->d.grec, sizeof(double) * t.size(),
+                                    cudaMemcpyDeviceToHost, s)));
+    return cuda_ok(cudaStreamSynchronize(s));
+}
+
 int sfx_mesh_set_gradients(sfx_mesh* m, const double* grad) {
     if(!m || !grad) return SFX_ERR_INVALID;
-    if(m->ctx->cfg.precision != SFX_PREC_FP64 || !m->d.grad) return SFX_ERR_UNSUPPORTED;
+    if(m->ctx->cfg.precision != SFX_PREC_FP64 || !m->d.grec) return SFX_ERR_UNSUPPORTED;
     const int64_t n = m->d.n_cells;
-    const int w = m->d.dim * m->d.S;
+    const size_t w = (size_t)m->d.dim * m->d.S, rec = rec_doubles(m->d.dim, SFX_REC_GREC);
     std::vector<double> t;
-    transpose_in(grad, n, w, t);
+    SFX_TRY(download_grec(m, t)); /* the records' dW/dt stays */
+    for(int64_t i = 0; i < n; ++i) std::memcpy(&t[i * rec], grad + i * w, w * sizeof(double));
     cudaStream_t s = m->ctx->stream;
-    SFX_TRY(h2d(m->d.grad, t.data(), t.size(), s));
+    SFX_TRY(h2d(m->d.grec, t.data(), t.size(), s));
     return cuda_ok(cudaStreamSynchronize(s));
 }
 
 int sfx_mesh_get_gradients(sfx_mesh* m, double* grad) {
     if(!m || !grad) return SFX_ERR_INVALID;
-    if(m->ctx->cfg.precision != SFX_PREC_FP64 || !m->d.grad) return SFX_ERR_UNSUPPORTED;
+    if(m->ctx->cfg.precision != SFX_PREC_FP64 || !m->d.grec) return SFX_ERR_UNSUPPORTED;
     const int64_t n = m->d.n_cells;
-    const int w = m->d.dim * m->d.S;
-    std::vector<double> t((size_t)n * w);
-    cudaStream_t s = m->ctx->stream;
-    SFX_TRY(cuda_ok(cudaMemcpyAsync(t.data(), m->d.grad, sizeof(double) * t.size(),
-                                    cudaMemcpyDeviceToHost, s)));
-    SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
-    transpose_out(t, n, w, grad);
+    const size_t w = (size_t)m->d.dim * m->d.S, rec = rec_doubles(m->d.dim, SFX_REC_GREC);
+    std::vector<double> t;
+    SFX_TRY(download_grec(m, t));
+    for(int64_t i = 0; i < n; ++i) std::memcpy(grad + i * w, &t[i * rec], w * sizeof(double));
     return SFX_OK;
 }
 
@@ -1003,21 +1025,21 @@ int sfx_flux_pass(sfx_mesh* m, double dt, double* grad, double* dQ_face,
     SFX_TRY(run_phase(m, 0, dt, 1, s));
     SFX_TRY(run_phase(m, 1, dt, 1, s));
     if(split) SFX_TRY(sfx_split_export_dQ(&m->d, s));
-    std::vector<double> tg(grad ? n * D * S : 0), tq(dQ_face ? F * S : 0);
     if(grad && split) {
-        /* FP32 gradient records [n][G float4] -> [D*S][n] */
+        /* FP32 gradient records [n][G float4] */
         const int G = sfx_split_grad_vec4(D);
         std::vector<float> tf((size_t)n * G * 4);
         SFX_TRY(cuda_ok(cudaMemcpyAsync(tf.data(), m->d.cg, sizeof(float) * tf.size(),
                                         cudaMemcpyDeviceToHost, s)));
         SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
         for(int64_t i = 0; i < n; ++i)
-            for(int q = 0; q < D * S; ++q) tg[(size_t)q * n + i] = tf[(size_t)i * G * 4 + q];
+            for(int q = 0; q < D * S; ++q) grad[i * D * S + q] = tf[(size_t)i * G * 4 + q];
     } else if(grad) {
-        SFX_TRY(cuda_ok(cudaMemcpyAsync(tg.data(), m->d.grad, sizeof(double) * tg.size(),
-                                        cudaMemcpyDeviceToHost, s)));
+        SFX_TRY(sfx_mesh_get_gradients(m, grad));
     }
     if(branch && split && F) SFX_TRY(cuda_ok(cudaMemsetAsync(m->d.branch, 0, 4 * F, s)));
+    const size_t dq = split ? (size_t)S : rec_doubles(D, SFX_REC_DQ);
+    std::vector<double> tq(dQ_face ? F * dq : 0);
     if(dQ_face)
         SFX_TRY(cuda_ok(cudaMemcpyAsync(tq.data(), m->d.dQf, sizeof(double) * tq.size(),
                                         cudaMemcpyDeviceToHost, s)));
@@ -1025,8 +1047,10 @@ int sfx_flux_pass(sfx_mesh* m, double dt, double* grad, double* dQ_face,
         SFX_TRY(cuda_ok(cudaMemcpyAsync(branch, m->d.branch, sizeof(int32_t) * F,
                                         cudaMemcpyDeviceToHost, s)));
     SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
-    if(grad) transpose_out(tg, n, D * S, grad);
-    if(dQ_face) transpose_out(tq, F, S, dQ_face);
+    if(dQ_face && split) transpose_out(tq, F, S, dQ_face);
+    if(dQ_face && !split)
+        for(int64_t f = 0; f < F; ++f)
+            std::memcpy(dQ_face + f * S, &tq[f * dq], S * sizeof(double));
     sfx_stats local;
     return check_err(m, st ? st : &local);
 }
@@ -1085,8 +1109,9 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
                  F * 8 + F * D * 8 +
                  4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 24;
     else
-        bytes += n * D * S * 8 + F * 4 +
-                 F * 8 * (b.gshare ? sfx_grad_term_stride((int)D) : S) + 256;
+        bytes += n * (int64_t)(sfx_fp64_record_bytes((int)D, SFX_REC_WS) +
+                               sfx_fp64_record_bytes((int)D, SFX_REC_GREC)) +
+                 F * (4 + (int64_t)sfx_fp64_record_bytes((int)D, SFX_REC_DQ)) + 512;
     return bytes;
 }
 

@@ -9,17 +9,17 @@
  * glibc's and CUDA's pow differ in the last bit; it is evaluated by sfx_powq
  * (sfx_powq.h).
  *
- * Kernels (one step = three or four launches):
- *   k_gradients  one thread per cell: VorCell::estimate_gradient
- *                (src/VorCell.cpp:464-530); or k_grad_terms (one thread
- *                per face) + k_grad_sum (one per cell and variable), the
- *                same values with each face's terms computed once
+ * Kernels (one step = three launches):
+ *   k_grad_cells one thread per cell and variable: VorCell::estimate_gradient
+ *                (src/VorCell.cpp:464-530); k_gradients, one thread per
+ *                cell, for meshes whose faces do not sit between their
+ *                cells' positions and for caller-owned arrays
  *   k_faces      one thread per face: VorFace::calculate_flux
  *                (src/VorFace.cpp:670-1024) with the Exact or HLLC solver;
  *                writes the limited dQ of the left cell once per face
- *   k_apply      one thread per cell: the face contributions in ascending
- *                face order (the order of VorTessManager::hydro's loop,
- *                src/VorTessManager.cpp:205-209), Q -= dQ
+ *   k_apply      one thread per cell: the face contributions in
+ *                ascending face order (the order of VorTessManager::hydro's
+ *                loop, src/VorTessManager.cpp:205-209), Q -= dQ
  *                (GasParticle::update_Q, GasParticle.cpp:617-624), get_W.
  * No floating-point atomics: every cell sums its own faces in a fixed order,
  * so reruns are bitwise identical.
@@ -112,14 +112,13 @@ __device__ __forceinline__ void reconstruct(double* W, const double (*g)[D + 2],
 
 /* VorFace.hpp:92-137 */
 template <int D>
-__device__ __forceinline__ double limit1(double phimid0, double phiL, double phiR,
-                                         double dnrm, double r) {
+__device__ __forceinline__ double limit1(double phimid0, double phiL, double phiR, double w) {
     const double psi1 = 0.5, psi2 = 0.25;
     double delta1 = psi1 * fabs(phiL - phiR);
     double delta2 = psi2 * fabs(phiL - phiR);
     double phimin = fmin(phiL, phiR);
     double phimax = fmax(phiL, phiR);
-    double phibar = phiL + dnrm / r * (phiR - phiL);
+    double phibar = phiL + w * (phiR - phiL);
     if(phiL == phiR) return phiL;
     /* only the bound the result uses (phi- when phiL < phiR, else phi+), with
      * the sign-preserving fallback where the shifted extreme changes sign:
@@ -134,15 +133,14 @@ __device__ __forceinline__ double limit1(double phimid0, double phiL, double phi
 
 /* mirror a state across a reflective face: transform, flip the normal
  * velocity, invtransform (VorFace.cpp:417-542, VorCell.cpp:479-485) */
+/* from r = left - right and its norm (right - left is -r exactly) */
 template <int D>
-__device__ __forceinline__ void mirror_state(double* W, const double* left,
-                                             const double* right);
+__device__ __forceinline__ void mirror_across(double* W, const double* r, double rnorm);
 
 template <>
-__device__ __forceinline__ void mirror_state<3>(double* W, const double* left,
-                                                const double* right) {
-    double n0 = right[0] - left[0], n1 = right[1] - left[1], n2 = right[2] - left[2];
-    double n3 = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
+__device__ __forceinline__ void mirror_across<3>(double* W, const double* r, double rnorm) {
+    double n0 = -r[0], n1 = -r[1], n2 = -r[2];
+    const double n3 = rnorm;
     n0 /= n3;
     n1 /= n3;
     n2 /= n3;
@@ -174,10 +172,8 @@ __device__ __forceinline__ void mirror_state<3>(double* W, const double* left,
 }
 
 template <>
-__device__ __forceinline__ void mirror_state<2>(double* W, const double* left,
-                                                const double* right) {
-    double d0 = left[0] - right[0], d1 = left[1] - right[1];
-    double d2 = sqrt(d0 * d0 + d1 * d1);
+__device__ __forceinline__ void mirror_across<2>(double* W, const double* r, double rnorm) {
+    const double d0 = r[0], d1 = r[1], d2 = rnorm;
     double cost = -d0 / d2;
     double sint = -d1 / d2;
     double W1 = W[1] * cost + W[2] * sint;
@@ -187,9 +183,155 @@ __device__ __forceinline__ void mirror_state<2>(double* W, const double* left,
     W[2] = W1 * sint + W2 * cost;
 }
 
-/* ------------------------------ gradients ------------------------------ */
 template <int D>
-__global__ void __launch_bounds__(128) k_gradients(sfx_dmesh m) {
+__device__ __forceinline__ void mirror_state(double* W, const double* left,
+                                             const double* right) {
+    double r[D];
+#pragma unroll
+    for(int l = 0; l < D; ++l) r[l] = left[l] - right[l];
+    mirror_across<D>(W, r, norm<D>(r));
+}
+
+/* ------------------------------- records -------------------------------
+ * A mesh's step reads three records laid out for it (a gather of one variable
+ * at a time from field-major arrays touches a 32-byte sector per double):
+ *   ws   [n][8]   the cell's W, then its mass Q[0]
+ *   grec [n][20] (3D), [n][12] (2D): gradients [l][k], then dW/dt at W
+ *   dQf  [F][6] (3D), [F][4] (2D): the limited dQ of the left cell
+ * and two per face that hold what the reference forms from positions on
+ * every step, in its operation order (the mesh is static between uploads):
+ *   ggeo gradient: A, 1/|r|, |r|, c, r, midpoint (NaN for a face of zero
+ *        area); c = mid - (x_L + x_R)/2 and r = x_L - x_R
+ *   fgeo flux: {left, right or -1}, A, A/area_L, A/area_R, |d_L|/|c_LR|,
+ *        |d_R|/|c_LR|, d_L, d_R, normal */
+template <int D>
+struct Rec {
+    static constexpr int S = D + 2;
+    static constexpr int ws = 8;
+    static constexpr int grec = D == 3 ? 20 : 12;
+    static constexpr int dq = D == 3 ? 6 : 4;
+    static constexpr int ggeo = D == 3 ? 12 : 10;
+    static constexpr int fgeo = D == 3 ? 16 : 12;
+    /* cells per warp of the kernels with one lane per cell and variable */
+    static constexpr int cells = 32 / S;
+};
+
+template <int N>
+__device__ __forceinline__ void load_record(const double* p, double* out) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+#pragma unroll
+    for(int i = 0; i < N / 2; ++i) {
+        const double2 v = __ldg(q + i);
+        out[2 * i] = v.x;
+        out[2 * i + 1] = v.y;
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void store_record(double* p, const double* v) {
+    double2* q = reinterpret_cast<double2*>(p);
+#pragma unroll
+    for(int i = 0; i < N / 2; ++i) q[i] = make_double2(v[2 * i], v[2 * i + 1]);
+}
+
+/* a length, or a difference of positions, for which sfx_div_by's products and
+ * residuals stay far from underflow and overflow */
+__device__ __forceinline__ bool plain_size(double x) {
+    return x == 0. || (fabs(x) > 0x1p-200 && fabs(x) < 0x1p200);
+}
+
+template <int D>
+__global__ void __launch_bounds__(128) k_face_records(sfx_dmesh m) {
+    using R = Rec<D>;
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if(f >= m.n_faces) return;
+    const int n = m.n_cells, F = m.n_faces;
+    const int iL = m.left[f];
+    const bool has_right = m.kind[f] != SFX_FACE_MIRROR;
+    const int iR = has_right ? m.right[f] : 0;
+    const double A = m.area[f];
+    double mid[D], xL[D], xRi[D], cenL[D], r[D], c[D], dL[D], dR[D], dd[D], cd[D];
+    bool plain = true;
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        mid[l] = m.mid[(size_t)l * F + f];
+        xL[l] = m.pos[(size_t)l * n + iL];
+        xRi[l] = m.rpos[(size_t)l * F + f];
+        cenL[l] = m.cen[(size_t)l * n + iL];
+        c[l] = mid[l] - 0.5 * (xL[l] + xRi[l]);
+        r[l] = xL[l] - xRi[l];
+        plain = plain && plain_size(c[l]) && plain_size(r[l]);
+        dL[l] = mid[l] - cenL[l] + (xL[l] - xL[l]);
+        dR[l] = 0.;
+        cd[l] = 0.;
+        if(has_right) {
+            const double cenR = m.cen[(size_t)l * n + iR], xR = m.pos[(size_t)l * n + iR];
+            dR[l] = mid[l] - cenR + (xR - xRi[l]);
+            cd[l] = cenL[l] - cenR;
+        }
+        dd[l] = xL[l] - xRi[l];
+    }
+    const double rn = norm<D>(r);
+    double g[R::ggeo];
+    g[0] = A;
+    g[1] = plain && plain_size(rn) && rn > 0. ? 1. / rn : 0.;
+    g[2] = rn;
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        g[3 + l] = c[l];
+        g[3 + D + l] = r[l];
+        /* a NaN offset takes no part in the slope limiter */
+        g[3 + 2 * D + l] = A == 0. ? __longlong_as_double(0x7ff8000000000000ll) : mid[l];
+    }
+    if(D == 2) g[R::ggeo - 1] = 0.;
+    store_record<R::ggeo>(m.ggeo + (size_t)f * R::ggeo, g);
+    const double cn = norm<D>(cd);
+    const double dn = norm<D>(dd);
+    double h[R::fgeo];
+    h[0] = __hiloint2double(has_right ? iR : -1, iL);
+    h[1] = A;
+    h[2] = A / m.tarea[iL];
+    h[3] = has_right ? A / m.tarea[iR] : 0.;
+    h[4] = has_right ? sqrt(dot<D>(dL, dL)) / cn : 0.;
+    h[5] = has_right ? sqrt(dot<D>(dR, dR)) / cn : 0.;
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        h[6 + l] = dL[l];
+        h[6 + D + l] = dR[l];
+        /* VorFace::get_normal (VorFace.cpp:553-571) */
+        h[6 + 2 * D + l] = -dd[l] / dn;
+    }
+    if(D == 3) h[R::fgeo - 1] = 0.;
+    store_record<R::fgeo>(m.fgeo + (size_t)f * R::fgeo, h);
+}
+
+/* each CSR entry with its neighbour cell, so that the gradient kernels load
+ * it beside the face id instead of after it */
+__global__ void __launch_bounds__(256) k_csr_neighbours(sfx_dmesh m) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(j >= m.nnz) return;
+    const unsigned e = (unsigned)m.idx[j];
+    const int f = (int)(e & ~kRightBit);
+    const int nb = e & kRightBit ? m.left[f] : (m.kind[f] == SFX_FACE_MIRROR ? -1 : m.right[f]);
+    m.ent[j] = make_int2((int)e, nb);
+}
+
+/* W and Q[0] (field-major) -> ws */
+template <int D>
+__global__ void k_state_records(sfx_dmesh m) {
+    constexpr int S = D + 2;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= m.n_cells) return;
+    double* w = m.ws + (size_t)i * Rec<D>::ws;
+    for(int k = 0; k < S; ++k) w[k] = m.W[(size_t)k * m.n_cells + i];
+    w[S] = m.Q[i];
+}
+
+/* ------------------------------ gradients ------------------------------ */
+/* REC: the gradients and dW/dt go to the cell's record (field-major
+ * gradients otherwise, for caller-owned arrays) */
+template <int D, bool REC>
+__global__ void __launch_bounds__(128) k_gradients(sfx_dmesh m, double gamma) {
     constexpr int S = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= sfx_grad_cells(m) || failed(m.err)) return;
@@ -290,156 +432,258 @@ __global__ void __launch_bounds__(128) k_gradients(sfx_dmesh m) {
             alpha[k] = (mx < alpha[k]) ? mx : alpha[k];
         }
     }
+    if constexpr(REC) {
+        double out[Rec<D>::grec];
 #pragma unroll
-    for(int l = 0; l < D; ++l)
+        for(int l = 0; l < D; ++l)
 #pragma unroll
-        for(int k = 0; k < S; ++k)
-            m.grad[((size_t)l * S + k) * n + i] = delta[l][k] * alpha[k];
-}
-
-constexpr int kGradBlock = 128;
-
-/* The same gradients in two kernels, when every local face's right position
- * is its right cell's position (gshare).  The first loop's term of a face,
- *   t = A ((W_j - W_i) c / |r| - (W_i + W_j) / 2 r / |r|),
- * is then exactly negated between the face's two cells: c is the same for
- * both (the midpoint sum commutes), r and W_j - W_i change sign, and IEEE
- * rounding is symmetric under negation, so the right cell's term equals -t
- * bit for bit, except that a zero term may carry the other sign, which no
- * sum starting at +0 can tell apart.  k_grad_terms evaluates t once per face
- * (its 2 D S divisions, the bulk of the gradients' cost, are no longer done
- * twice); k_grad_sum adds the terms in each cell's face order exactly as the
- * one-kernel loop does, and runs the limiter. */
-template <int D>
-__global__ void __launch_bounds__(128) k_grad_terms(sfx_dmesh m) {
-    constexpr int S = D + 2, TS = D == 3 ? 16 : 8;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if(f >= m.n_faces || failed(m.err)) return;
-    const double A = m.area[f];
-    if(A == 0.) return; /* skipped by both cells */
-    const int n = m.n_cells, F = m.n_faces;
-    const int i = m.left[f];
-    double W[S], Wj[S], xi[D], xj[D], c[D], rij[D];
-#pragma unroll
-    for(int k = 0; k < S; ++k) W[k] = m.W[(size_t)k * n + i];
-#pragma unroll
-    for(int l = 0; l < D; ++l) {
-        xi[l] = m.pos[(size_t)l * n + i];
-        xj[l] = m.rpos[(size_t)l * F + f];
-    }
-    if(m.kind[f] == SFX_FACE_MIRROR) {
-#pragma unroll
-        for(int k = 0; k < S; ++k) Wj[k] = W[k];
-        mirror_state<D>(Wj, xi, xj);
+            for(int k = 0; k < S; ++k) {
+                delta[l][k] = delta[l][k] * alpha[k];
+                out[l * S + k] = delta[l][k];
+            }
+        time_derivative<D>(gamma, W, delta, out + D * S);
+        store_record<Rec<D>::grec>(m.grec + (size_t)i * Rec<D>::grec, out);
     } else {
-        const int r = m.right[f];
 #pragma unroll
-        for(int k = 0; k < S; ++k) Wj[k] = m.W[(size_t)k * n + r];
+        for(int l = 0; l < D; ++l)
+#pragma unroll
+            for(int k = 0; k < S; ++k)
+                m.grad[((size_t)l * S + k) * n + i] = delta[l][k] * alpha[k];
     }
-#pragma unroll
-    for(int l = 0; l < D; ++l) {
-        c[l] = m.mid[(size_t)l * F + f] - 0.5 * (xi[l] + xj[l]);
-        rij[l] = xi[l] - xj[l];
-    }
-    const double rnorm = norm<D>(rij);
-    double t[TS];
-#pragma unroll
-    for(int l = 0; l < D; ++l)
-#pragma unroll
-        for(int k = 0; k < S; ++k)
-            t[l * S + k] =
-                A * ((Wj[k] - W[k]) * c[l] / rnorm - 0.5 * (W[k] + Wj[k]) * rij[l] / rnorm);
-#pragma unroll
-    for(int q = D * S; q < TS; ++q) t[q] = 0.;
-    double2* out = reinterpret_cast<double2*>(m.gterm + (size_t)f * TS);
-#pragma unroll
-    for(int q = 0; q < TS / 2; ++q) out[q] = make_double2(t[2 * q], t[2 * q + 1]);
 }
 
-/* one thread per (cell, primitive variable): the first loop adds the
- * faces' terms (subtracts them where the cell is the face's right one) in
- * the cell's face order, the second is the limiter; the variables are
- * independent in both loops, so each thread rounds exactly as the
- * one-kernel loop does */
+/* a / b from y = 1 / b (rounded to nearest): two corrections of a y, the
+ * second of them with an exact residual of a quotient within an ulp, give the
+ * correctly rounded quotient (P. Markstein, "Computation of elementary
+ * functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990)
+ * where nothing under- or overflows; a zero quotient may lose its sign */
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+/* 0, or a normal size between 2^-300 and 2^300: with plain_size lengths,
+ * every dividend of the gradient is then 0 or between 2^-560 and 2^520 */
+__device__ __forceinline__ bool plain_state(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return h - 0x2d300000u < 0x25800000u || (h | (unsigned)__double2loint(x)) == 0u;
+}
+
+/* asynchronous copy of BYTES (8 or 16) bytes to shared memory, both aligned to them */
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(BYTES)
+                 : "memory");
+}
+
+/* One lane per (cell, primitive variable), Rec::cells whole cells per warp:
+ * the variables are independent in both loops, so each lane adds the terms
+ *   A ((W_j - W_i) c / |r| - (W_i + W_j) / 2 r / |r|)
+ * in the cell's face order, as the reference rounds them; the right cell of a
+ * face sees the same c and |r| and the opposite r (the mesh qualifies when
+ * every local face's right position is its right cell's position, gshare).
+ * Bound by FP64 issue and the latency of the gathers.  The 2 D divisions by
+ * |r| use the face's stored reciprocal (div_by: 5 operations; a zero term's
+ * sign cannot change a sum that starts at +0), the limiter's minimum over the
+ * faces takes two divisions per cell (sfx_limiter_min), and the face's
+ * geometry and the neighbour's state come through a shared-memory ring filled
+ * kGradStages faces ahead (lane k of a cell copies 16 bytes of the geometry
+ * and one variable): no registers hold loads in flight.  Both loops divided
+ * per face before, the first one in a kernel of its own that wrote 128 bytes
+ * per face: 220 -> 88 us on 65,537 cells in 3D, 104 -> 66 us on 150,001 in 2D
+ * (109 and 68 us without the ring).  Cells sorted by face count so that a
+ * warp's lanes run equally long: 83 us, but the update in that order lost
+ * more than that to a lower L1 hit rate. */
+constexpr int kGradBlock = 128, kGradStages = 4;
+
 template <int D>
-__global__ void __launch_bounds__(kGradBlock, 8) k_grad_sum(sfx_dmesh m) {
-    constexpr int S = D + 2, TS = D == 3 ? 16 : 8;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = (int)(t / S), k = (int)(t % S);
-    if(i >= sfx_grad_cells(m) || failed(m.err)) return;
-    if(m.local && m.tstart[i] != m.t_now) return;
-    const int n = m.n_cells, F = m.n_faces;
-    const double W = m.W[(size_t)k * n + i];
+struct GradSlot {
+    static constexpr int S = D + 2;
+    double2 geo[S];  /* A, 1/|r|, |r|, c, r (and, 2D, the midpoint's x) */
+    double W[S];     /* the neighbour's state */
+    int2 ent;        /* CSR entry, neighbour (-1: mirror) */
+    /* to 144 bytes (3D) and 112 (2D): a warp's cells on different banks */
+    double pad[D == 3 ? 2 : 1];
+};
+
+template <int D>
+__global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double gamma) {
+    using R = Rec<D>;
+    constexpr int S = R::S;
+    static_assert(sizeof(GradSlot<D>) == (D == 3 ? 144 : 112), "slot layout");
+    __shared__ __align__(16) GradSlot<D> ring[kGradBlock / 32][kGradStages][R::cells];
+    const int lane = threadIdx.x & 31;
+    const int slot = lane / S, k = lane - slot * S;
+    const int i = ((blockIdx.x * kGradBlock + threadIdx.x) >> 5) * R::cells + slot;
+    /* local time steps: an inactive cell keeps its gradients (src/Simulation.cpp:414-420) */
+    const bool live = slot < R::cells && i < sfx_grad_cells(m) && !failed(m.err) &&
+                      !(m.local && m.tstart[i] != m.t_now);
+    if(!__any_sync(0xffffffffu, live)) return;
+    const int ic = live ? i : 0;
+    const double* own = m.ws + (size_t)ic * R::ws;
+    const double W = own[k];
     double delta[D];
     double Wmax = W, Wmin = W;
+    bool plain = plain_state(W);
 #pragma unroll
     for(int l = 0; l < D; ++l) delta[l] = 0.;
-    const int beg = m.off[i], end = m.off[i + 1];
-    for(int j = end - 1; j >= beg; --j) {
-        const unsigned e = (unsigned)m.idx[j];
-        const int f = (int)(e & ~kRightBit);
-        const bool rside = (e & kRightBit) != 0;
-        /* the face's loads all issued before the area test (the record of a
-         * face of zero area holds stale values, never used) */
-        const double A = m.area[f];
-        const int kd = m.kind[f];
-        const int nb = rside ? m.left[f] : m.right[f];
-        const double* tf = m.gterm + (size_t)f * TS + k;
-        double tv[D];
-#pragma unroll
-        for(int l = 0; l < D; ++l) tv[l] = tf[l * S];
-        if(A == 0.) continue;
-        double Wj;
-        if(!rside && kd == SFX_FACE_MIRROR) {
-            double Wm[S], xi[D], xj[D];
-#pragma unroll
-            for(int q = 0; q < S; ++q) Wm[q] = m.W[(size_t)q * n + i];
-#pragma unroll
-            for(int l = 0; l < D; ++l) {
-                xi[l] = m.pos[(size_t)l * n + i];
-                xj[l] = m.rpos[(size_t)l * F + f];
-            }
-            mirror_state<D>(Wm, xi, xj);
-            Wj = Wm[0];
-#pragma unroll
-            for(int q = 1; q < S; ++q)
-                if(q == k) Wj = Wm[q];
-        } else {
-            Wj = m.W[(size_t)k * n + nb];
+    const int beg = live ? m.off[ic] : 0, end = live ? m.off[ic + 1] : 0;
+    const int count = end - beg;
+    const int most = __reduce_max_sync(0xffffffffu, count);
+    /* face `it` of the cell (from its last to its first) into its ring slot;
+     * the CSR entry was loaded one call before */
+    int2 next = make_int2(0, -1);
+    if(count > 0) next = __ldg(m.ent + end - 1);
+    GradSlot<D>(*mine)[R::cells] = ring[threadIdx.x >> 5];
+    auto fetch = [&](int it) {
+        if(it < count) {
+            const int2 v = next;
+            if(it + 1 < count) next = __ldg(m.ent + end - 2 - it);
+            GradSlot<D>& q = mine[it % kGradStages][slot];
+            copy_async<16>(&q.geo[k],
+                           m.ggeo + (size_t)((unsigned)v.x & ~kRightBit) * R::ggeo + 2 * k);
+            copy_async<8>(&q.W[k], m.ws + (size_t)(v.y < 0 ? ic : v.y) * R::ws + k);
+            if(k == 0) q.ent = v;
         }
-        if(!rside) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-            for(int l = 0; l < D; ++l) delta[l] = delta[l] + tv[l];
+    for(int it = 0; it < kGradStages - 1; ++it) fetch(it);
+#pragma unroll 1
+    for(int it = 0; it < most; ++it) {
+        /* this lane's copies for face `it` have landed; then every lane's */
+        asm volatile("cp.async.wait_group %0;" ::"n"(kGradStages - 2) : "memory");
+        __syncwarp();
+        /* the slot refilled here was read before the barrier above */
+        fetch(it + kGradStages - 1);
+        if(it >= count) continue;
+        const GradSlot<D>& q = mine[it % kGradStages][slot];
+        double g[2 * S];
+#pragma unroll
+        for(int t = 0; t < S; ++t) {
+            g[2 * t] = q.geo[t].x;
+            g[2 * t + 1] = q.geo[t].y;
+        }
+        double Wj = q.W[k];
+        const double A = g[0], y = g[1], rn = g[2];
+        if(A == 0.) continue;
+        const int2 ent = q.ent;
+        if(ent.y < 0) {
+            double Wm[S], r[D];
+#pragma unroll
+            for(int t = 0; t < S; ++t) Wm[t] = own[t];
+#pragma unroll
+            for(int l = 0; l < D; ++l) r[l] = g[3 + D + l];
+            mirror_across<D>(Wm, r, rn);
+#pragma unroll
+            for(int t = 1; t <= D; ++t)
+                if(t == k) Wj = Wm[t];
+        }
+        const double dW = Wj - W;
+        double sW = 0.5 * (W + Wj);
+        if((unsigned)ent.x & kRightBit) sW = -sW; /* r changes sign */
+        plain = plain && plain_state(Wj);
+        if(plain && y != 0.) {
+#pragma unroll
+            for(int l = 0; l < D; ++l)
+                delta[l] = delta[l] + A * (div_by(dW * g[3 + l], rn, y) -
+                                           div_by(sW * g[3 + D + l], rn, y));
         } else {
 #pragma unroll
-            for(int l = 0; l < D; ++l) delta[l] = delta[l] - tv[l];
+            for(int l = 0; l < D; ++l)
+                delta[l] = delta[l] + A * (dW * g[3 + l] / rn - sW * g[3 + D + l] / rn);
         }
         Wmax = (Wmax < Wj) ? Wj : Wmax;
         Wmin = (Wj < Wmin) ? Wj : Wmin;
     }
-    const double V = m.vol[i];
+    const double V = m.vol[ic];
     double cen[D];
 #pragma unroll
     for(int l = 0; l < D; ++l) {
         delta[l] = delta[l] / V;
-        cen[l] = m.cen[(size_t)l * n + i];
+        cen[l] = m.cen[(size_t)l * m.n_cells + ic];
     }
     const double a = Wmax - W, b = Wmin - W;
-    double alpha = 1.;
-    for(int j = end - 1; j >= beg; --j) {
-        const int f = (int)((unsigned)m.idx[j] & ~kRightBit);
-        const double A = m.area[f];
+    /* the offsets' projections on the gradient: the extremes decide the limiter */
+    auto offset = [&](int j) {
+        const unsigned f = (unsigned)__ldg(m.idx + j) & ~kRightBit;
+        const double* p = m.ggeo + (size_t)f * R::ggeo;
         double d[D];
+        if(D == 3) {
+            double t[4];
+            load_record<4>(p + 8, t);
 #pragma unroll
-        for(int l = 0; l < D; ++l) d[l] = m.mid[(size_t)l * F + f] - cen[l];
-        if(A == 0.) continue;
+            for(int l = 0; l < D; ++l) d[l] = t[(l + 1) & 3] - cen[l];
+        } else {
+            d[0] = __ldg(p + 7) - cen[0];
+            d[1] = __ldg(p + 8) - cen[1];
+        }
         double dp = delta[0] * d[0] + delta[1] * d[1];
-        if(D == 3) dp = dp + delta[2] * d[2];
-        const double mx = sfx_limiter_ratio(a, b, dp);
-        alpha = (mx < alpha) ? mx : alpha;
+        if(D == 3) dp = dp + delta[D - 1] * d[D - 1];
+        return dp;
+    };
+    double dmax = 0., dmin = 0.;
+    int first = 0;
+#pragma unroll 4
+    for(int j = end - 1; j >= beg; --j) {
+        const double dp = offset(j);
+        if(dp > dmax) dmax = dp;
+        if(dp < dmin) dmin = dp;
+        if(first == 0) first = dp > 0. ? 1 : (dp < 0. ? -1 : 0);
     }
+    double alpha = 1.;
+    if(plain && dmax < 0x1p300 && dmin > -0x1p300) {
+        alpha = sfx_limiter_min(a, b, dmax, dmin, first);
+    } else {
+        for(int j = end - 1; j >= beg; --j) {
+            const double dp = offset(j);
+            /* a face of zero area (NaN offset) is skipped; other NaNs never
+             * compare below alpha */
+            const double mx = sfx_limiter_ratio(a, b, dp);
+            alpha = (mx < alpha) ? mx : alpha;
+        }
+    }
+    double g[D];
 #pragma unroll
-    for(int l = 0; l < D; ++l) m.grad[((size_t)l * S + k) * n + i] = delta[l] * alpha;
+    for(int l = 0; l < D; ++l) g[l] = delta[l] * alpha;
+    /* dW/dt at the cell's state (time_derivative), one variable per lane */
+    const int base = slot * S;
+    double Wc[S], diag[D], gp[D];
+#pragma unroll
+    for(int q = 0; q < S; ++q) Wc[q] = __shfl_sync(0xffffffffu, W, base + q);
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        diag[l] = __shfl_sync(0xffffffffu, g[l], base + 1 + l);
+        gp[l] = __shfl_sync(0xffffffffu, g[l], base + S - 1);
+    }
+    if(!live) return;
+    double dW;
+    if(D == 3) {
+        const double div = diag[0] + diag[1] + diag[D - 1];
+        const double lead = k == 0 ? -Wc[0] * div : (k == S - 1 ? -gamma * Wc[S - 1] * div : 0.);
+        if(k == 0 || k == S - 1)
+            dW = lead - Wc[1] * g[0] - Wc[2] * g[1] - Wc[D] * g[D - 1];
+        else
+            dW = -Wc[1] * g[0] - Wc[2] * g[1] - Wc[D] * g[D - 1] -
+                 (k == 1 ? gp[0] : (k == 2 ? gp[1] : gp[D - 1])) / Wc[0];
+    } else {
+        const double div = diag[0] + diag[1];
+        if(k == 0)
+            dW = -Wc[1] * g[0] - Wc[2] * g[1] - Wc[0] * div;
+        else if(k == 1)
+            dW = -Wc[1] * g[0] - Wc[2] * g[1] - gp[0] / Wc[0];
+        else if(k == 2) /* d(vy)/dy in both terms (ExactRiemannSolver.cpp:920) */
+            dW = -Wc[1] * g[1] - Wc[2] * g[1] - gp[1] / Wc[0];
+        else
+            dW = -gamma * Wc[S - 1] * div - Wc[1] * g[0] - Wc[2] * g[1];
+    }
+    double* out = m.grec + (size_t)i * R::grec;
+#pragma unroll
+    for(int l = 0; l < D; ++l) out[l * S + k] = g[l];
+    out[D * S + k] = dW;
 }
 
 /* --------------------------- exact solver --------------------------- */
@@ -1058,22 +1302,21 @@ __device__ int hllc_flux(const sfx_solver_params& s, double* WL, double* WR,
 /* -------------------------------- faces -------------------------------- */
 
 /* MUSCL-Hancock prediction + reconstruction + pairwise limiter + positivity
- * fallbacks for one side (VorFace.cpp:715-759 right, 762-804 left) */
+ * fallbacks for one side (VorFace.cpp:715-759 right, 762-804 left); dW0 is
+ * dW/dt at Wt, w = |d| / |centroid difference| */
 template <int D>
-__device__ __forceinline__ void predict_side(double gamma, double dt, double* Wt,
-                                             const double* Wself, const double* Wother,
-                                             const double (*g)[D + 2], const double* d,
-                                             bool do_limit, double r) {
+__device__ __forceinline__ void predict_side(double dt, double* Wt, const double* Wself,
+                                             const double* Wother, const double (*g)[D + 2],
+                                             const double* dW0, const double* d, bool do_limit,
+                                             double w) {
     constexpr int S = D + 2;
-    double dW0[S], dW[S];
-    time_derivative<D>(gamma, Wt, g, dW0);
+    double dW[S];
 #pragma unroll
     for(int k = 0; k < S; ++k) dW[k] = 0.5 * dt * dW0[k];
     reconstruct<D>(Wt, g, d);
     if(do_limit) {
-        double dn = sqrt(dot<D>(d, d));
 #pragma unroll
-        for(int k = 0; k < S; ++k) Wt[k] = limit1<D>(Wt[k], Wself[k], Wother[k], dn, r);
+        for(int k = 0; k < S; ++k) Wt[k] = limit1<D>(Wt[k], Wself[k], Wother[k], w);
     }
     if(Wt[0] < 0. || Wt[D + 1] < 0.) {
 #pragma unroll
@@ -1087,35 +1330,126 @@ __device__ __forceinline__ void predict_side(double gamma, double dt, double* Wt
     }
 }
 
-template <int D, int SOLVER>
+/* what a face's flux needs of the mesh */
+template <int D>
+struct FaceGeom {
+    int iL, iR; /* iR = -1: mirror */
+    double A, facL, facR, wL, wR, dL[D], dR[D], n[D];
+};
+
+/* from positions, as the reference forms it (caller-owned arrays) */
+template <int D>
+__device__ __forceinline__ void face_geom(const sfx_dmesh& m, int f, FaceGeom<D>& q) {
+    const int n = m.n_cells, F = m.n_faces;
+    const int iL = q.iL, iR = q.iR < 0 ? 0 : q.iR;
+    const bool has_right = q.iR >= 0;
+    double dd[D], cd[D];
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        const double mid = m.mid[(size_t)l * F + f];
+        const double xL = m.pos[(size_t)l * n + iL];
+        const double xRi = m.rpos[(size_t)l * F + f];
+        const double cenL = m.cen[(size_t)l * n + iL];
+        q.dL[l] = mid - cenL + (xL - xL);
+        q.dR[l] = 0.;
+        cd[l] = 0.;
+        if(has_right) {
+            const double cenR = m.cen[(size_t)l * n + iR], xR = m.pos[(size_t)l * n + iR];
+            q.dR[l] = mid - cenR + (xR - xRi);
+            cd[l] = cenL - cenR;
+        }
+        dd[l] = xL - xRi;
+    }
+    const double r = norm<D>(cd);
+    q.wL = has_right ? sqrt(dot<D>(q.dL, q.dL)) / r : 0.;
+    q.wR = has_right ? sqrt(dot<D>(q.dR, q.dR)) / r : 0.;
+    q.facL = q.A / m.tarea[iL];
+    q.facR = has_right ? q.A / m.tarea[iR] : 0.;
+    /* VorFace::get_normal (VorFace.cpp:553-571) */
+    const double dn = norm<D>(dd);
+#pragma unroll
+    for(int l = 0; l < D; ++l) q.n[l] = -dd[l] / dn;
+}
+
+/* kFaceArrays: field-major caller-owned arrays.  kFaceRecords: a mesh's
+ * records, dW/dt from the cell's (a static mesh with one step).
+ * kFaceMoving: records, face velocities and local time steps, dW/dt formed
+ * here (at the boosted state; a cell in the middle of its step keeps its
+ * gradients).
+ * What a face needs of its two cells is one gather of 3 + 10 (2D: 3 + 6)
+ * 16-byte loads per side and its own geometry a coalesced record; from
+ * field-major arrays it was 28 (20) scattered doubles per side and the
+ * geometry's square roots and divisions on every step.  HLLC: 101 -> 67 us on
+ * 65,537 cells (500,000 faces) in 3D, 71 -> 51 us on 150,001 in 2D; bound by
+ * FP64 latency at 16 warps per SM (128 registers). */
+constexpr int kFaceArrays = 0, kFaceRecords = 1, kFaceMoving = 2;
+
+template <int D, int SOLVER, int MODE>
 __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp,
                                                double dt, int write_branch) {
+    using R = Rec<D>;
     constexpr int S = D + 2;
+    constexpr bool REC = MODE != kFaceArrays;
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if(f >= sfx_flux_faces(m) || failed(m.err)) return;
     const int n = m.n_cells, F = m.n_faces;
-    const double A = m.area[f];
-    if(A == 0.) {
+    auto store_dQ = [&](const double* v) {
+        if(REC) {
+            double t[R::dq];
 #pragma unroll
-        for(int k = 0; k < S; ++k) m.dQf[(size_t)k * F + f] = 0.;
+            for(int k = 0; k < R::dq; ++k) t[k] = k < S ? v[k] : 0.;
+            store_record<R::dq>(m.dQf + (size_t)f * R::dq, t);
+        } else {
+#pragma unroll
+            for(int k = 0; k < S; ++k) m.dQf[(size_t)k * F + f] = v[k];
+        }
+    };
+    auto skip = [&]() {
+        double z[S];
+#pragma unroll
+        for(int k = 0; k < S; ++k) z[k] = 0.;
+        store_dQ(z);
         if(write_branch) m.branch[f] = SFX_BRANCH_SKIPPED;
+    };
+    FaceGeom<D> q;
+    if(REC) {
+        double h[R::fgeo];
+        load_record<R::fgeo>(m.fgeo + (size_t)f * R::fgeo, h);
+        q.iL = __double2loint(h[0]);
+        q.iR = __double2hiint(h[0]);
+        q.A = h[1];
+        q.facL = h[2];
+        q.facR = h[3];
+        q.wL = h[4];
+        q.wR = h[5];
+#pragma unroll
+        for(int l = 0; l < D; ++l) {
+            q.dL[l] = h[6 + l];
+            q.dR[l] = h[6 + D + l];
+            q.n[l] = h[6 + 2 * D + l];
+        }
+    } else {
+        q.A = m.area[f];
+        q.iL = m.left[f];
+        q.iR = m.kind[f] == SFX_FACE_MIRROR ? -1 : m.right[f];
+    }
+    const double A = q.A;
+    if(A == 0.) {
+        skip();
         return;
     }
-    const int iL = m.left[f];
-    const int kind = m.kind[f];
-    const bool has_right = kind != SFX_FACE_MIRROR;
-    const int iR = has_right ? m.right[f] : 0;
+    const int iL = q.iL;
+    const bool has_right = q.iR >= 0;
+    const int iR = has_right ? q.iR : 0;
     /* local time steps (VorFace.cpp:672-697): a face is computed when its
      * left cell is active, or (with a right cell) either cell is; its time
      * step is the shorter of the two cells' steps */
     double dtmax = dt;
-    if(m.local) {
+    if(MODE == kFaceMoving && m.local) {
         const bool aL = m.tstart[iL] == m.t_now;
         const bool aR = has_right && m.tstart[iR] == m.t_now;
         if(!aL && !aR) {
-#pragma unroll
-            for(int k = 0; k < S; ++k) m.dQf[(size_t)k * F + f] = 0.;
-            if(write_branch) m.branch[f] = SFX_BRANCH_SKIPPED;
+            skip();
             return;
         }
         dt = sfx_realtime(m.t_total, m.tend[iL] - m.tstart[iL]);
@@ -1126,61 +1460,74 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
             dtmax = fmax(dtmax, dtR);
         }
     }
-    double v[D], mid[D], xL[D], xRi[D], cenL[D];
+    if(!REC) face_geom<D>(m, f, q);
+    double v[D];
 #pragma unroll
-    for(int l = 0; l < D; ++l) {
-        v[l] = m.vel ? m.vel[(size_t)l * F + f] : 0.;
-        mid[l] = m.mid[(size_t)l * F + f];
-        xL[l] = m.pos[(size_t)l * n + iL];
-        xRi[l] = m.rpos[(size_t)l * F + f];
-        cenL[l] = m.cen[(size_t)l * n + iL];
-    }
+    for(int l = 0; l < D; ++l)
+        v[l] = MODE == kFaceMoving && m.vel ? m.vel[(size_t)l * F + f] : 0.;
     double WL[S], WR[S], WRrec[S], Wt[S];
+    double QLm, QRm = 0.;
+    auto load_state = [&](int i, double* W, double& Qm) {
+        if(REC) {
+            double t[6];
+            load_record<6>(m.ws + (size_t)i * R::ws, t);
+#pragma unroll
+            for(int k = 0; k < S; ++k) W[k] = t[k];
+            Qm = t[S];
+        } else {
+#pragma unroll
+            for(int k = 0; k < S; ++k) W[k] = m.W[(size_t)k * n + i];
+            Qm = m.Q[i];
+        }
+    };
+    load_state(iL, WL, QLm);
 #pragma unroll
     for(int k = 0; k < S; ++k) {
-        WL[k] = m.W[(size_t)k * n + iL];
-        WR[k] = has_right ? m.W[(size_t)k * n + iR] : 0.;
+        WR[k] = 0.;
         WRrec[k] = 0.;
     }
-#pragma unroll
-    for(int l = 0; l < D; ++l) {
-        WL[1 + l] = WL[1 + l] - v[l];
-        WR[1 + l] = WR[1 + l] - v[l];
-    }
-    double r = 0.;
-    if(has_right) {
-        double cenR[D], xR[D], d[D], g[D][S];
+    if(has_right) load_state(iR, WR, QRm);
+    if(MODE == kFaceMoving) {
 #pragma unroll
         for(int l = 0; l < D; ++l) {
-            cenR[l] = m.cen[(size_t)l * n + iR];
-            xR[l] = m.pos[(size_t)l * n + iR];
-            d[l] = mid[l] - cenR[l] + (xR[l] - xRi[l]);
+            WL[1 + l] = WL[1 + l] - v[l];
+            WR[1 + l] = WR[1 + l] - v[l];
         }
+    }
+    /* gradients of cell i, and dW/dt at its (boosted) state W */
+    auto load_slopes = [&](int i, const double* W, double (*g)[S], double* dW0) {
+        if(REC) {
+            double t[R::grec];
+            load_record<R::grec>(m.grec + (size_t)i * R::grec, t);
 #pragma unroll
-        for(int l = 0; l < D; ++l)
+            for(int l = 0; l < D; ++l)
 #pragma unroll
-            for(int k = 0; k < S; ++k) g[l][k] = m.grad[((size_t)l * S + k) * n + iR];
-        double cd[D];
+                for(int k = 0; k < S; ++k) g[l][k] = t[l * S + k];
 #pragma unroll
-        for(int l = 0; l < D; ++l) cd[l] = cenL[l] - cenR[l];
-        r = norm<D>(cd);
+            for(int k = 0; k < S; ++k) dW0[k] = t[D * S + k];
+        } else {
+#pragma unroll
+            for(int l = 0; l < D; ++l)
+#pragma unroll
+                for(int k = 0; k < S; ++k) g[l][k] = m.grad[((size_t)l * S + k) * n + i];
+        }
+        if(MODE != kFaceRecords) time_derivative<D>(sp.gamma, W, g, dW0);
+    };
+    if(has_right) {
+        double g[D][S], dW0[S];
+        load_slopes(iR, WR, g, dW0);
 #pragma unroll
         for(int k = 0; k < S; ++k) Wt[k] = WR[k];
-        predict_side<D>(sp.gamma, dt, Wt, WR, WL, g, d, true, r);
+        predict_side<D>(dt, Wt, WR, WL, g, dW0, q.dR, true, q.wR);
 #pragma unroll
         for(int k = 0; k < S; ++k) WRrec[k] = Wt[k];
     }
     {
-        double d[D], g[D][S];
-#pragma unroll
-        for(int l = 0; l < D; ++l) d[l] = mid[l] - cenL[l] + (xL[l] - xL[l]);
-#pragma unroll
-        for(int l = 0; l < D; ++l)
-#pragma unroll
-            for(int k = 0; k < S; ++k) g[l][k] = m.grad[((size_t)l * S + k) * n + iL];
+        double g[D][S], dW0[S];
+        load_slopes(iL, WL, g, dW0);
 #pragma unroll
         for(int k = 0; k < S; ++k) Wt[k] = WL[k];
-        predict_side<D>(sp.gamma, dt, Wt, WL, WR, g, d, has_right, r);
+        predict_side<D>(dt, Wt, WL, WR, g, dW0, q.dL, has_right, q.wL);
     }
     if(WL[0] != 0.) {
 #pragma unroll
@@ -1190,28 +1537,18 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
 #pragma unroll
         for(int k = 0; k < S; ++k) WR[k] = WRrec[k];
     }
-    /* VorFace::get_normal (VorFace.cpp:553-571) */
-    double nrm[D];
-    {
-        double dd[D];
-#pragma unroll
-        for(int l = 0; l < D; ++l) dd[l] = xL[l] - xRi[l];
-        const double dn = norm<D>(dd);
-#pragma unroll
-        for(int l = 0; l < D; ++l) nrm[l] = -dd[l] / dn;
-    }
     double flux[S];
     int status = SFX_OK, code;
     if(SOLVER == SFX_SOLVER_EXACT) {
         double half[S];
-        ExactOut eo = exact_solve<D>(sp, WL, WR, nrm, !has_right, half);
+        ExactOut eo = exact_solve<D>(sp, WL, WR, q.n, !has_right, half);
         status = eo.status;
         code = eo.code;
 #pragma unroll
         for(int l = 0; l < D; ++l) half[1 + l] = half[1 + l] + v[l];
-        exact_flux_from_half<D>(sp.gamma, half, v, nrm, flux);
+        exact_flux_from_half<D>(sp.gamma, half, v, q.n, flux);
     } else {
-        code = hllc_flux<D>(sp, WL, WR, nrm, v, !has_right, flux);
+        code = hllc_flux<D>(sp, WL, WR, q.n, v, !has_right, flux);
     }
     double dQL[S], dQR[S];
 #pragma unroll
@@ -1222,10 +1559,8 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
     /* over-flux limiter (VorFace.cpp:837-866): timefac = dt / (the longer
      * of the two cells' steps); dt / dt with one global step */
     double timefac = 1.;
-    if(has_right) timefac = dt / dtmax;
-    double areafac = A / m.tarea[iL];
-    areafac = areafac * timefac;
-    const double QLm = m.Q[iL];
+    if(MODE == kFaceMoving && has_right) timefac = dt / dtmax;
+    const double areafac = q.facL * timefac;
     if(dQL[0] > areafac * QLm) {
         const double corfac = fabs(areafac * QLm / dQL[0]);
 #pragma unroll
@@ -1235,9 +1570,7 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
         code |= SFX_BRANCH_LIMIT_L;
     }
     if(has_right) {
-        double areafacR = A / m.tarea[iR];
-        areafacR = areafacR * timefac;
-        const double QRm = m.Q[iR];
+        const double areafacR = q.facR * timefac;
         if(dQR[0] > areafacR * QRm) {
             const double corfac = fabs(areafacR * QRm / dQR[0]);
 #pragma unroll
@@ -1247,8 +1580,7 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
             code |= SFX_BRANCH_LIMIT_R;
         }
     }
-#pragma unroll
-    for(int k = 0; k < S; ++k) m.dQf[(size_t)k * F + f] = dQL[k];
+    store_dQ(dQL);
     if(write_branch) m.branch[f] = code;
     if(status == SFX_OK && flux[0] != flux[0]) status = SFX_ERR_NAN_FLUX;
     if(status != SFX_OK) report_face(m.err, f, status);
@@ -1256,56 +1588,43 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
 
 /* ------------------------------ update ------------------------------ */
 
-/* get_W (ExactRiemannSolver.cpp:716-766 == HLLCRiemannSolver.cpp:495-535 on
- * the hydro fields); may rewrite Q[D+1] (pressure floor) */
-template <int D>
-__device__ __forceinline__ void get_W(double gamma, double V, double* Q, double* W) {
-    constexpr int S = D + 2;
-#pragma unroll
-    for(int k = 0; k < S; ++k) W[k] = 0.;
-    if(Q[0] == 0.) return;
-    W[0] = Q[0] / V;
-    W[1] = Q[1] / Q[0];
-    W[2] = Q[2] / Q[0];
-    double p2 = Q[1] * Q[1] + Q[2] * Q[2];
-    if(D == 3) {
-        W[3] = Q[3] / Q[0];
-        p2 = p2 + Q[3] * Q[3];
-    }
-    W[D + 1] = (gamma - 1.) * (Q[D + 1] - 0.5 * p2 / Q[0]) / V;
-    if(W[D + 1] < 1.e-30) {
-        W[D + 1] = 1.e-30;
-        Q[D + 1] = 0.5 * p2 / Q[0] + W[D + 1] * V / (gamma - 1.);
-    }
-    if(W[0] < 1.e-30) {
-#pragma unroll
-        for(int k = 0; k < S; ++k) W[k] = 0.;
-    }
-}
+/* One thread per cell: the cell's faces in ascending face order (aidx), the
+ * order in which the reference's face loop adds them (a face of zero area, or
+ * between two inactive cells, holds zeros, which change no sum), then Q and
+ * get_W.  Bound by the latency of the dQ gathers: a face's dQ is one record
+ * of 2 or 3 16-byte loads (field-major dQ touched a 32-byte sector per
+ * double), U faces' loads in flight.  65,537 cells 3D 33 -> 23 us, 150,001
+ * cells 2D 20.5 -> 19.1 us (event-timed); one lane per cell and variable took
+ * 23 and 24 us. */
+constexpr int kApplyBlock = 128;
 
 template <int D>
-__global__ void __launch_bounds__(128) k_apply(sfx_dmesh m, double gamma) {
-    constexpr int S = D + 2;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma) {
+    using R = Rec<D>;
+    constexpr int S = R::S;
+    const int i = blockIdx.x * kApplyBlock + threadIdx.x;
     if(i >= sfx_update_cells(m) || failed(m.err)) return;
-    const int n = m.n_cells, F = m.n_faces;
+    const int n = m.n_cells;
     double dQ[S];
 #pragma unroll
     for(int k = 0; k < S; ++k) dQ[k] = 0.;
     const int beg = m.off[i], end = m.off[i + 1];
-    /* the cell's faces in ascending face order (aidx), the order in which
-     * the reference's face loop adds them */
-    for(int j = beg; j < end; ++j) {
-        const unsigned e = (unsigned)m.aidx[j];
-        const int f = (int)(e & ~kRightBit);
-        if(m.area[f] == 0.) continue;
-        if(e & kRightBit) {
+    constexpr int U = 3; /* faces in flight */
+    for(int j = beg; j < end; j += U) {
+        unsigned e[U];
+        double v[U][R::dq];
 #pragma unroll
-            for(int k = 0; k < S; ++k) dQ[k] = dQ[k] + -1. * m.dQf[(size_t)k * F + f];
-        } else {
+        for(int t = 0; t < U; ++t) e[t] = (unsigned)__ldg(m.aidx + (j + t < end ? j + t : j));
 #pragma unroll
-            for(int k = 0; k < S; ++k) dQ[k] = dQ[k] + m.dQf[(size_t)k * F + f];
-        }
+        for(int t = 0; t < U; ++t)
+            load_record<R::dq>(m.dQf + (size_t)(e[t] & ~kRightBit) * R::dq, v[t]);
+#pragma unroll
+        for(int t = 0; t < U; ++t)
+            if(t == 0 || j + t < end) {
+#pragma unroll
+                for(int k = 0; k < S; ++k)
+                    dQ[k] = dQ[k] + (e[t] & kRightBit ? -1. * v[t][k] : v[t][k]);
+            }
     }
     double Q[S], W[S];
 #pragma unroll
@@ -1314,20 +1633,50 @@ __global__ void __launch_bounds__(128) k_apply(sfx_dmesh m, double gamma) {
         report_cell(m.err, i, SFX_ERR_NEG_STATE);
         return;
     }
+    double* ws = m.ws + (size_t)i * R::ws;
     if(m.local && m.tend[i] != m.t_next) {
         /* local time steps: a cell in the middle of its step takes the flux
          * of its active neighbours into Q; its W waits for the end of its
          * step (src/Simulation.cpp:791-836) */
 #pragma unroll
         for(int k = 0; k < S; ++k) m.Q[(size_t)k * n + i] = Q[k];
+        ws[S] = Q[0];
         return;
     }
-    get_W<D>(gamma, m.vol[i], Q, W);
+    /* get_W (ExactRiemannSolver.cpp:716-766 == HLLCRiemannSolver.cpp:495-535
+     * on the hydro fields); may rewrite Q[D+1] (pressure floor) */
+    const double V = m.vol[i];
+#pragma unroll
+    for(int k = 0; k < S; ++k) W[k] = 0.;
+    if(Q[0] != 0.) {
+        W[0] = Q[0] / V;
+        W[1] = Q[1] / Q[0];
+        W[2] = Q[2] / Q[0];
+        double p2 = Q[1] * Q[1] + Q[2] * Q[2];
+        if(D == 3) {
+            W[D] = Q[D] / Q[0];
+            p2 = p2 + Q[D] * Q[D];
+        }
+        W[D + 1] = (gamma - 1.) * (Q[D + 1] - 0.5 * p2 / Q[0]) / V;
+        if(W[D + 1] < 1.e-30) {
+            W[D + 1] = 1.e-30;
+            Q[D + 1] = 0.5 * p2 / Q[0] + W[D + 1] * V / (gamma - 1.);
+        }
+        if(W[0] < 1.e-30) {
+#pragma unroll
+            for(int k = 0; k < S; ++k) W[k] = 0.;
+        }
+    }
+    double t[6];
 #pragma unroll
     for(int k = 0; k < S; ++k) {
         m.Q[(size_t)k * n + i] = Q[k];
         m.W[(size_t)k * n + i] = W[k];
+        t[k] = W[k];
     }
+    t[S] = Q[0];
+    if(D == 2) t[5] = 0.;
+    store_record<6>(ws, t);
 }
 
 /* Q = get_Q(V, W): ExactRiemannSolver.cpp:776-804 / HLLCRiemannSolver.cpp:471-483 */
@@ -1357,6 +1706,12 @@ __global__ void k_init_Q(sfx_dmesh m, double gamma, int kind) {
     }
 #pragma unroll
     for(int k = 0; k < S; ++k) m.Q[(size_t)k * n + i] = Q[k];
+    if(m.ws) {
+        double* w = m.ws + (size_t)i * Rec<D>::ws;
+#pragma unroll
+        for(int k = 0; k < S; ++k) w[k] = W[k];
+        w[S] = Q[0];
+    }
 }
 
 /* deterministic totals: fixed 1024 blocks over fixed ranges, fixed tree */
@@ -1465,6 +1820,7 @@ __global__ void k_unpack_cells(sfx_dmesh m, const int32_t* idx, int count, const
         m.W[(size_t)q * m.n_cells + c] = in[t];
     else
         m.Q[c] = in[t];
+    m.ws[(size_t)c * Rec<3>::ws + q] = in[t]; /* W, then the mass: the same stride in 2D */
 }
 
 inline int grid_for(long long n, int block) {
@@ -1726,29 +2082,82 @@ void sfx_solver_params_init(sfx_solver_params* p, int kind, double g, double tol
     p->ginv = 1. / g;
 }
 
-int sfx_fp64_gradients(const sfx_dmesh* m, void* stream) {
-    const int nc = sfx_grad_cells(*m);
-    if(nc == 0) return SFX_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int B = 128;
-    if(m->gterm && m->gshare) {
-        const long long cs = (long long)nc * m->S;
-        if(m->dim == 3) {
-            if(m->n_faces) k_grad_terms<3><<<grid_for(m->n_faces, B), B, 0, s>>>(*m);
-            k_grad_sum<3><<<grid_for(cs, kGradBlock), kGradBlock, 0, s>>>(*m);
-        } else {
-            if(m->n_faces) k_grad_terms<2><<<grid_for(m->n_faces, B), B, 0, s>>>(*m);
-            k_grad_sum<2><<<grid_for(cs, kGradBlock), kGradBlock, 0, s>>>(*m);
-        }
-        sfx_count_launches(m->n_faces ? 2 : 1);
-        return cuda_status(cudaGetLastError());
-    }
-    if(m->dim == 3)
-        k_gradients<3><<<grid_for(nc, B), B, 0, s>>>(*m);
-    else
-        k_gradients<2><<<grid_for(nc, B), B, 0, s>>>(*m);
+/* threads for `cells` cells of the kernels with one lane per cell and variable */
+static int cell_lane_blocks(int dim, int cells, int block) {
+    const int per_warp = dim == 3 ? Rec<3>::cells : Rec<2>::cells;
+    return grid_for((cells + per_warp - 1) / per_warp * 32ll, block);
+}
+
+int sfx_fp64_record_bytes(int dim, int what) {
+    const int v3[5] = {Rec<3>::ws, Rec<3>::grec, Rec<3>::dq, Rec<3>::ggeo, Rec<3>::fgeo};
+    const int v2[5] = {Rec<2>::ws, Rec<2>::grec, Rec<2>::dq, Rec<2>::ggeo, Rec<2>::fgeo};
+    return (int)sizeof(double) * (dim == 3 ? v3 : v2)[what];
+}
+
+int sfx_fp64_csr_neighbours(const sfx_dmesh* m, void* stream) {
+    if(m->nnz == 0) return SFX_OK;
+    k_csr_neighbours<<<grid_for(m->nnz, 256), 256, 0, (cudaStream_t)stream>>>(*m);
     sfx_count_launches(1);
     return cuda_status(cudaGetLastError());
+}
+
+int sfx_fp64_face_records(const sfx_dmesh* m, void* stream) {
+    if(m->n_faces == 0) return SFX_OK;
+    cudaStream_t s = (cudaStream_t)stream;
+    if(m->dim == 3)
+        k_face_records<3><<<grid_for(m->n_faces, 128), 128, 0, s>>>(*m);
+    else
+        k_face_records<2><<<grid_for(m->n_faces, 128), 128, 0, s>>>(*m);
+    sfx_count_launches(1);
+    return cuda_status(cudaGetLastError());
+}
+
+int sfx_fp64_state_records(const sfx_dmesh* m, void* stream) {
+    cudaStream_t s = (cudaStream_t)stream;
+    if(m->dim == 3)
+        k_state_records<3><<<grid_for(m->n_cells, 128), 128, 0, s>>>(*m);
+    else
+        k_state_records<2><<<grid_for(m->n_cells, 128), 128, 0, s>>>(*m);
+    sfx_count_launches(1);
+    return cuda_status(cudaGetLastError());
+}
+
+/* k_grad_cells needs the records and face positions that are the cells' (see
+ * there); other meshes take k_gradients, caller-owned arrays its field-major
+ * form */
+template <int D>
+static void launch_gradients(const sfx_dmesh* m, double gamma, int nc, cudaStream_t s) {
+    const int B = 128;
+    if(m->ws && m->gshare)
+        k_grad_cells<D><<<cell_lane_blocks(D, nc, kGradBlock), kGradBlock, 0,
+                          s>>>(*m, gamma);
+    else if(m->ws)
+        k_gradients<D, true><<<grid_for(nc, B), B, 0, s>>>(*m, gamma);
+    else
+        k_gradients<D, false><<<grid_for(nc, B), B, 0, s>>>(*m, gamma);
+}
+
+int sfx_fp64_gradients(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream) {
+    const int nc = sfx_grad_cells(*m);
+    if(nc == 0) return SFX_OK;
+    if(m->dim == 3)
+        launch_gradients<3>(m, sp->gamma, nc, (cudaStream_t)stream);
+    else
+        launch_gradients<2>(m, sp->gamma, nc, (cudaStream_t)stream);
+    sfx_count_launches(1);
+    return cuda_status(cudaGetLastError());
+}
+
+template <int D, int SOLVER>
+static void launch_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
+                         int write_branch, int nf, cudaStream_t s) {
+    const int B = 128, G = grid_for(nf, B);
+    if(!m->ws)
+        k_faces<D, SOLVER, kFaceArrays><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+    else if(m->vel || m->local)
+        k_faces<D, SOLVER, kFaceMoving><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+    else
+        k_faces<D, SOLVER, kFaceRecords><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
 }
 
 int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
@@ -1756,18 +2165,16 @@ int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
     const int nf = sfx_flux_faces(*m);
     if(nf == 0) return SFX_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    const int B = 128;
-    const int G = grid_for(nf, B);
     if(m->dim == 3) {
         if(sp->kind == SFX_SOLVER_EXACT)
-            k_faces<3, SFX_SOLVER_EXACT><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+            launch_faces<3, SFX_SOLVER_EXACT>(m, sp, dt, write_branch, nf, s);
         else
-            k_faces<3, SFX_SOLVER_HLLC><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+            launch_faces<3, SFX_SOLVER_HLLC>(m, sp, dt, write_branch, nf, s);
     } else {
         if(sp->kind == SFX_SOLVER_EXACT)
-            k_faces<2, SFX_SOLVER_EXACT><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+            launch_faces<2, SFX_SOLVER_EXACT>(m, sp, dt, write_branch, nf, s);
         else
-            k_faces<2, SFX_SOLVER_HLLC><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+            launch_faces<2, SFX_SOLVER_HLLC>(m, sp, dt, write_branch, nf, s);
     }
     sfx_count_launches(1);
     return cuda_status(cudaGetLastError());
@@ -1777,7 +2184,7 @@ int sfx_fp64_apply(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream
     const int nc = sfx_update_cells(*m);
     if(nc == 0) return SFX_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    const int B = 128;
+    const int B = kApplyBlock;
     if(m->dim == 3)
         k_apply<3><<<grid_for(nc, B), B, 0, s>>>(*m, sp->gamma);
     else

@@ -42,7 +42,8 @@ struct sfx_dmesh {
                        cell lists its faces that way */
     double* W;      /* [S][n]    */
     double* Q;      /* [S][n]    */
-    double* grad;   /* [dim*S][n]: grad[(l*S + k)*n + i] = dW_k/dx_l       */
+    double* grad;   /* [dim*S][n]: grad[(l*S + k)*n + i] = dW_k/dx_l; caller-owned
+                       arrays only (meshes keep them in grec) */
     /* faces */
     double* area;   /* [F]       */
     double* mid;    /* [dim][F]  */
@@ -51,13 +52,15 @@ struct sfx_dmesh {
     int32_t* kind;  /* [F]       */
     double* rpos;   /* [dim][F]  */
     double* vel;    /* [dim][F] or NULL */
-    double* dQf;    /* [S][F] scratch: limited dQ received by the left cell */
-    /* plain-FP64 pass: the first gradient loop's terms as seen from each
-     * face's left cell, [F][sfx_grad_term_stride(dim)] (the right cell of a
-     * local face takes their negation).  NULL: one kernel computes the
-     * gradients without it.  The array is dead between the gradient and the
-     * face kernels, so dQf lives inside it. */
-    double* gterm;
+    double* dQf;    /* limited dQ received by the left cell: plain-FP64 meshes [F] records
+                       (sfx_fp64.cu), otherwise [S][F] */
+    /* plain-FP64 meshes: records of the cells' states and of their gradients
+     * and dW/dt, and of the faces' gradient and flux geometry (sfx_fp64.cu).
+     * ws == NULL: caller-owned field-major arrays */
+    double* ws;
+    double* grec;
+    double* ggeo;
+    double* fgeo;
     int32_t gshare; /* every local face's right position equals its right cell's */
     /* one part of a mesh split over several devices (plain FP64): gradients
      * of cells [0, r_grad), fluxes of faces [0, r_flux), update of cells
@@ -92,7 +95,8 @@ struct sfx_dmesh {
     float4* cg;
     float4* cdw;
     float4* cx;
-    int32_t* nbe; /* [nnz] neighbour cell of each CSR entry (-1 mirror) */
+    int2* ent;      /* [nnz] each CSR entry (idx) and its neighbour cell (-1 mirror), both
+                       precisions */
     /* moving generators (plain FP64, sfx_step_moving; allocated on first
      * use): generator velocities [dim][n], drifted positions [dim][n] */
     double* vgen;
@@ -177,8 +181,14 @@ void sfx_solver_params_init(sfx_solver_params* p, int kind, double gamma,
                             double tol, double cutoff);
 
 /* FP64 kernels (sfx_fp64.cu) */
-inline int64_t sfx_grad_term_stride(int dim) { return dim == 3 ? 16 : 8; }
-int sfx_fp64_gradients(const sfx_dmesh* m, void* stream);
+enum { SFX_REC_WS, SFX_REC_GREC, SFX_REC_DQ, SFX_REC_GGEO, SFX_REC_FGEO };
+int sfx_fp64_record_bytes(int dim, int what); /* bytes of one record */
+/* ent from idx and the face list */
+int sfx_fp64_csr_neighbours(const sfx_dmesh* m, void* stream);
+/* the face geometry records of an uploaded mesh; the state records from W, Q */
+int sfx_fp64_face_records(const sfx_dmesh* m, void* stream);
+int sfx_fp64_state_records(const sfx_dmesh* m, void* stream);
+int sfx_fp64_gradients(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream);
 int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
                    int write_branch, void* stream);
 int sfx_fp64_apply(const sfx_dmesh* m, const sfx_solver_params* sp,

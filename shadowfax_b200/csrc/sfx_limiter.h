@@ -48,3 +48,27 @@ SFX_LIM_HD double sfx_limiter_ratio(double a, double b, double dp) {
     }
     return sfx_limiter_ratio_ref(a, b, dp);
 }
+
+/*
+ * The minimum over a cell's faces of 1 and those quotients, with two
+ * divisions.  For dp > 0 the quotient is a / dp, smallest where dp is
+ * largest, and rounding is monotonic, so the minimum over those faces is
+ * a / dmax rounded; for dp < 0 it is b / dp, smallest at dmin.  dmax and dmin
+ * are the largest positive and smallest negative dp (0: none), `first` the sign
+ * of the first dp that is neither 0 nor NaN in the reference's face order
+ * (which of a +0 and a -0 quotient it keeps: the first).  For a, b, dmax and
+ * dmin finite and far from under- and overflow.
+ */
+SFX_LIM_HD double sfx_limiter_min(double a, double b, double dmax, double dmin, int first) {
+    double alpha = 1.;
+    if(dmax > 0.) {
+        const double q = a / dmax;
+        alpha = (q < alpha) ? q : alpha;
+    }
+    if(dmin < 0.) {
+        const double q = b / dmin;
+        alpha = (q < alpha) ? q : alpha;
+        if(b == 0. && (a != 0. || first < 0)) alpha = q; /* -0 */
+    }
+    return alpha;
+}

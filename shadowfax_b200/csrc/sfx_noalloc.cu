@@ -156,7 +156,7 @@ extern "C" int sfx_flux_pass_noalloc(const sfx_device_mesh* dm, const sfx_config
         cudaGetLastError();
         return SFX_ERR_CUDA;
     }
-    rc = sfx_fp64_gradients(&d, s);
+    rc = sfx_fp64_gradients(&d, &sp, s);
     if(rc == SFX_OK) rc = sfx_fp64_faces(&d, &sp, dt, 0, s);
     if(rc != SFX_OK) return rc;
     sfx_dev_error e;

@@ -390,15 +390,17 @@ __device__ __forceinline__ void sgrad_body(const sfx_dmesh& m, const float gamma
     unsigned e_next = 0u;
     int nb_next = -1;
     if(beg + lane < end) {
-        e_next = (unsigned)__ldg(m.idx + beg + lane);
-        nb_next = __ldg(m.nbe + beg + lane);
+        const int2 v = __ldg(m.ent + beg + lane);
+        e_next = (unsigned)v.x;
+        nb_next = v.y;
     }
     for(int j = beg + lane; j < end; j += LPC, ++k0) {
         const unsigned e = e_next;
         const int nb = nb_next;
         if(j + LPC < end) {
-            e_next = (unsigned)__ldg(m.idx + j + LPC);
-            nb_next = __ldg(m.nbe + j + LPC);
+            const int2 v = __ldg(m.ent + j + LPC);
+            e_next = (unsigned)v.x;
+            nb_next = v.y;
         }
         const int f = (int)(e & ~kRightBit);
         const bool right = e & kRightBit;

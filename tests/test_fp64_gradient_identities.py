@@ -144,3 +144,78 @@ def test_limiter_ratio_random_and_underflow(limlib):
     fast, ref = _run(limlib, a2, b2, dp2)
     assert _same(fast, ref)
     assert np.any(ref == 0)
+
+
+_MIN_SRC = r"""
+#include "sfx_limiter.h"
+extern "C" {
+/* the reference's running minimum against the two-division one, over n faces */
+int limiter_min_differs(double a, double b, const double* dp, int n) {
+    double alpha = 1., dmax = 0., dmin = 0.;
+    int first = 0;
+    for(int j = 0; j < n; ++j) {
+        const double mx = sfx_limiter_ratio_ref(a, b, dp[j]);
+        alpha = (mx < alpha) ? mx : alpha;
+        if(dp[j] > dmax) dmax = dp[j];
+        if(dp[j] < dmin) dmin = dp[j];
+        if(first == 0) first = dp[j] > 0. ? 1 : (dp[j] < 0. ? -1 : 0);
+    }
+    const double q = sfx_limiter_min(a, b, dmax, dmin, first);
+    return __builtin_memcmp(&q, &alpha, sizeof q) != 0;
+}
+/* div_by of the gradient kernel against the division */
+double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = __builtin_fma(__builtin_fma(-q, b, a), y, q);
+    return __builtin_fma(__builtin_fma(-q, b, a), y, q);
+}
+long div_differs(const double* a, const double* b, long n) {
+    long bad = 0;
+    for(long i = 0; i < n; ++i) bad += div_by(a[i], b[i], 1. / b[i]) != a[i] / b[i];
+    return bad;
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def identities(tmp_path_factory):
+    d = tmp_path_factory.mktemp("identities")
+    (d / "m.cpp").write_text(_MIN_SRC)
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-mfma", "-shared", "-fPIC", "-I", str(CSRC),
+                    str(d / "m.cpp"), "-o", str(d / "m.so"), "-lm"], check=True)
+    lib = C.CDLL(str(d / "m.so"))
+    lib.limiter_min_differs.argtypes = [C.c_double, C.c_double, C.POINTER(C.c_double), C.c_int]
+    lib.div_differs.argtypes = [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_long]
+    lib.div_differs.restype = C.c_long
+    return lib
+
+
+@pytest.mark.parametrize("a,b", [(0.0, 0.0), (0.0, -0.7), (0.3, 0.0), (0.3, -0.7), (1e-40, -1e30)])
+def test_limiter_minimum_with_two_divisions(identities, a, b):
+    rng = np.random.default_rng(8)
+    for n in (0, 1, 2, 3, 5, 16, 40):
+        for _ in range(300):
+            dp = np.ascontiguousarray(_values(rng, n))
+            dp[rng.random(n) < 0.1] = np.nan          # faces of zero area
+            if rng.random() < 0.3:
+                dp = np.abs(dp)
+            elif rng.random() < 0.3:
+                dp = -np.abs(dp)
+            p = dp.ctypes.data_as(C.POINTER(C.c_double))
+            assert not identities.limiter_min_differs(a, b, p, n)
+
+
+def test_division_by_a_stored_reciprocal(identities):
+    """correctly rounded for dividends and divisors over the sizes the kernel
+    admits, near-equal and short-mantissa operands included"""
+    rng = np.random.default_rng(9)
+    n = 2_000_000
+    b = np.abs(rng.standard_normal(n)) * 10.0 ** rng.integers(-50, 50, n)
+    a = rng.standard_normal(n) * 10.0 ** rng.integers(-140, 140, n)
+    a[::5] = b[::5] * (1 + rng.integers(-8, 9, a[::5].size) * 2.0**-52)
+    b[1::7] = np.ldexp(2.0 - 2.0**-52 * rng.integers(1, 5, b[1::7].size), rng.integers(-60, 60))
+    a[2::9] = np.round(a[2::9] * 64) / 64
+    a[3::11] = 0.0
+    p = C.POINTER(C.c_double)
+    assert identities.div_differs(a.ctypes.data_as(p), b.ctypes.data_as(p), n) == 0
