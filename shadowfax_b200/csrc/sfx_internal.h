@@ -114,6 +114,8 @@ struct sfx_dmesh {
     double* an;
     float2* dqm;
     double* dqv;
+    double* stage; /* [n][S] rows on their way between W or Q and the host; no kernel of a
+                      step touches it */
     /* exact solver, split pass: faces whose p* iteration falls back to
      * Brent's method are queued here by the face kernel (face ids; room for
      * every face; slowq_n counts them) and solved by a follow-up launch in
@@ -193,8 +195,13 @@ int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
                    int write_branch, void* stream);
 int sfx_fp64_apply(const sfx_dmesh* m, const sfx_solver_params* sp,
                    void* stream);
-int sfx_fp64_init_Q(const sfx_dmesh* m, const sfx_solver_params* sp,
+/* Q = get_Q(V, W); rows != NULL: W from these rows [n][S] first */
+int sfx_fp64_init_Q(const sfx_dmesh* m, const sfx_solver_params* sp, const double* rows,
                     void* stream);
+/* rows [n][w] <-> field-major [w][n], device arrays */
+int sfx_from_rows(const double* rows, int64_t n, int w, double* out, void* stream);
+int sfx_to_rows(const double* in, int64_t n, int w, double* rows, void* stream);
+/* totals of Q, and the error record after them: host_out[S + 2] (waits) */
 int sfx_fp64_totals(const sfx_dmesh* m, double* host_out, void* stream);
 /* halo records [count][S + 1] (W, then the mass Q[0]) of the listed cells */
 int sfx_fp64_pack_cells(const sfx_dmesh* m, const int32_t* idx, int count, double* out,
@@ -223,8 +230,10 @@ int sfx_fp64_riemann(int dim, const sfx_solver_params* sp, int n,
 /* FP32/FP64-split kernels (sfx_split.cu) */
 int sfx_split_prepare(const sfx_dmesh* m, void* stream);
 int sfx_split_load_state(const sfx_dmesh* m, void* stream);
-/* W (FP64 SoA) from the FP32 cell records, for downloads */
+/* W (FP64 SoA) from the FP32 cell records */
 int sfx_split_export_W(const sfx_dmesh* m, void* stream);
+/* the same as rows [n][S], for downloads */
+int sfx_split_W_rows(const sfx_dmesh* m, double* rows, void* stream);
 /* per-face dQ (FP32) widened into dQf (FP64 SoA), for parity checks */
 int sfx_split_export_dQ(const sfx_dmesh* m, void* stream);
 /* kernel launch counter behind sfx_launch_count (sfx_api.cu).  Launches made
@@ -246,15 +255,13 @@ const sfx_solver_params* sfx_ctx_params(sfx_ctx* c);
  * sfx_group_set_steps (sfx_group.cu) */
 int sfx_group_set_members(sfx_group* g, int32_t n, sfx_mesh* const* meshes, const double* dt,
                           const int32_t* steps);
-/* state transfers in the device's field-major layout [S][n] (sfx_api.cu):
- * upload W, derive Q (waits and returns the status, as sfx_state_upload_W);
- * the download enqueues the copies on `stream` and returns at once */
-int sfx_mesh_upload_W_fieldmajor(sfx_mesh* m, const double* W);
-int sfx_mesh_download_fieldmajor_async(sfx_mesh* m, double* W, double* Q, void* stream);
-/* the same without waiting, all device work on `stream` (W must stay valid
- * until the stream has run it); errors of the upload land in the mesh's
- * error record (sfx_mesh_last_status after the stream has finished) */
-int sfx_mesh_upload_W_fieldmajor_async(sfx_mesh* m, const double* W, void* stream);
+/* state transfers on `stream` that return at once (sfx_api.cu): host rows
+ * [n][S], as in sfx_state_upload_W and sfx_state_download; the host arrays
+ * must stay valid until the stream has run them.  Errors of the upload land in
+ * the mesh's error record (sfx_mesh_last_status after the stream has
+ * finished). */
+int sfx_mesh_upload_W_async(sfx_mesh* m, const double* W, void* stream);
+int sfx_mesh_download_async(sfx_mesh* m, double* W, double* Q, void* stream);
 /* sfx_mesh_clone with its device setup on `stream`, not waited for */
 int sfx_mesh_clone_async(sfx_ctx* ctx, sfx_mesh* base, void* stream, sfx_mesh** out);
 

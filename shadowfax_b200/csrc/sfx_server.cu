@@ -21,8 +21,8 @@
  * that arrive while a round runs join at the next round.
  *
  * The worker keeps the GPU busy between rounds: finished requests are copied
- * out on a separate stream into pinned buffers while the next round runs,
- * and their host-side transposes happen then too; instances of finished
+ * out on a separate stream into pinned buffers while the next round runs
+ * (transposed to the caller's layout on the device); instances of finished
  * requests are kept per (pool mesh, solver) and reused by later requests,
  * and launch groups keep their device tables, so a round in steady state
  * allocates and frees no device memory (cudaFree would wait for the whole
@@ -68,7 +68,7 @@ struct Request {
     int32_t admit_status = SFX_OK;
     int32_t mesh_id = 0, solver = 0, nsteps = 0;
     double dt = 0.;
-    std::vector<double> W0; /* field-major [S][n], transposed at submit */
+    std::vector<double> W0; /* rows [n][S], as submitted */
     std::vector<double> W, Q;
     double t_submit = 0., t_admit = 0., t_done = 0.;
     int32_t status = SFX_OK, steps_done = 0;
@@ -232,7 +232,7 @@ void leave(sfx_server* s, Request* r, int status) {
             r->stage = stage_take(s->down, 2 * n, &r->stage_own);
         }
         if(r->stage) {
-            const int rc = sfx_mesh_download_fieldmajor_async(r->inst, r->stage, r->stage + n,
+            const int rc = sfx_mesh_download_async(r->inst, r->stage, r->stage + n,
                                                               s->copy_stream);
             if(rc && r->status == SFX_OK) r->status = rc;
         } else if(r->status == SFX_OK) {
@@ -252,15 +252,9 @@ void finish_leaving(sfx_server* s) {
             const sfx_dmesh* d = sfx_mesh_dev(r->inst);
             const int64_t n = d->n_cells;
             const int S = d->S;
-            r->W.resize((size_t)n * S);
-            r->Q.resize((size_t)n * S);
-            const double* w = r->stage;
-            const double* q = r->stage + (size_t)n * S;
-            for(int64_t i = 0; i < n; ++i)
-                for(int k = 0; k < S; ++k) {
-                    r->W[(size_t)i * S + k] = w[(size_t)k * n + i];
-                    r->Q[(size_t)i * S + k] = q[(size_t)k * n + i];
-                }
+            const size_t count = (size_t)n * S;
+            r->W.assign(r->stage, r->stage + count);
+            r->Q.assign(r->stage + count, r->stage + 2 * count);
         }
         stage_release(r);
         release_instance(s, r);
@@ -341,7 +335,7 @@ void admit(sfx_server* s) {
         if(!rc) {
             if(r->stage) {
                 std::memcpy(r->stage, r->W0.data(), r->W0.size() * sizeof(double));
-                rc = sfx_mesh_upload_W_fieldmajor_async(r->inst, r->stage, s->up_stream);
+                rc = sfx_mesh_upload_W_async(r->inst, r->stage, s->up_stream);
             } else {
                 rc = SFX_ERR_NOMEM;
             }
@@ -690,10 +684,7 @@ extern "C" int sfx_server_submit(sfx_server* s, int32_t mesh_id, const double* W
         n = s->pool[mesh_id]->n_cells;
         S = s->pool[mesh_id]->S;
     }
-    /* the device layout, transposed here on the caller's thread */
-    r->W0.resize((size_t)n * S);
-    for(int64_t i = 0; i < n; ++i)
-        for(int k = 0; k < S; ++k) r->W0[(size_t)k * n + i] = W0[(size_t)i * S + k];
+    r->W0.assign(W0, W0 + (size_t)n * S);
     r->mesh_id = mesh_id;
     r->solver = solver;
     r->dt = dt;

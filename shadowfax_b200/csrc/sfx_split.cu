@@ -264,6 +264,15 @@ __global__ void k_export_W(sfx_dmesh m) {
     for(int k = 0; k < S; ++k) m.W[(size_t)k * n + i] = c.W[k];
 }
 
+template <int D>
+__global__ void k_W_rows(sfx_dmesh m, double* rows) {
+    constexpr int S = D + 2;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= m.n_cells) return;
+    const Cell<D> c = load_cell<D>(m.cw, i);
+    for(int k = 0; k < S; ++k) rows[(size_t)i * S + k] = c.W[k];
+}
+
 /* a part's ring exchange (split pass): per listed cell its FP32 state W (S
  * values) and its FP64 mass Q[0], as S + 1 doubles, the record layout of the
  * plain-FP64 pass; W goes through double and back exactly */
@@ -2339,6 +2348,15 @@ int sfx_split_export_W(const sfx_dmesh* m, void* stream) {
         k_export_W<3><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m);
     else
         k_export_W<2><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m);
+    return launched(1);
+}
+
+int sfx_split_W_rows(const sfx_dmesh* m, double* rows, void* stream) {
+    cudaStream_t s = (cudaStream_t)stream;
+    if(m->dim == 3)
+        k_W_rows<3><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m, rows);
+    else
+        k_W_rows<2><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m, rows);
     return launched(1);
 }
 
