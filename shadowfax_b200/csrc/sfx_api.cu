@@ -252,8 +252,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     d.err = nullptr;
     d.totals_scratch = nullptr;
     d.cw = d.cg = d.cdw = nullptr;
-    d.dqm = nullptr;
-    d.dqv = nullptr;
+    d.dq = nullptr;
     d.slowq = nullptr;
     d.slowq_n = nullptr;
     d.slowq_cap = 0;
@@ -268,8 +267,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
         A(&d.cw, 2 * n);
         A(&d.cg, (size_t)sfx_split_grad_vec4(dim) * n);
         A(&d.cdw, (size_t)sfx_split_dwdt_vec4(dim) * n);
-        A(&d.dqm, F);
-        A(&d.dqv, (size_t)dim * F);
+        A(&d.dq, 4 * F);
         d.slowq_cap = slowq_capacity(F);
         A(&d.slowq, (size_t)d.slowq_cap);
         A(&d.slowq_n, 1);
@@ -416,8 +414,8 @@ int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
         bytes += F * 8 * (dim + S); /* face velocities, dQf */
     }
     if(precision == SFX_PREC_SPLIT) {
-        /* fg, fi, fsh, an, dqm, dqv, queue; cw, cg, cx, self table */
-        bytes += F * (32 + 8 + 1 + 8 * dim + 8 + 8 * dim) + 4 * slowq_capacity(F) + 4;
+        /* fg, fr, an, dq, queue; cw, cg, cx, self table */
+        bytes += F * (32 + 4 * (dim == 3 ? 16 : 12) + 8 * dim + 32) + 4 * slowq_capacity(F) + 4;
         bytes += n * (32 + 16 * (sfx_split_grad_vec4((int)dim) + sfx_split_dwdt_vec4((int)dim)) +
                       16) + 256;
     }
@@ -667,15 +665,13 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
             return SFX_ERR_UNSUPPORTED; /* the split pass is for static meshes */
         }
         A(&d.fg, 2 * F);
-        A(&d.fi, F);
-        A(&d.fsh, F);
+        A(&d.fr, (size_t)(dim == 3 ? 16 : 12) * F);
         A(&d.cw, 2 * n);
         A(&d.cg, (size_t)sfx_split_grad_vec4(dim) * n);
         A(&d.cdw, (size_t)sfx_split_dwdt_vec4(dim) * n);
         A(&d.cx, n);
         A(&d.an, (size_t)dim * F);
-        A(&d.dqm, F);
-        A(&d.dqv, (size_t)dim * F);
+        A(&d.dq, 4 * F);
         d.slowq_cap = slowq_capacity(F);
         A(&d.slowq, (size_t)d.slowq_cap);
         A(&d.slowq_n, 1);
@@ -687,7 +683,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     }
     cudaStream_t s = ctx->stream;
     /* the dQ scratch holds dim doubles per face, the state staging per cell */
-    double* fstage = split ? d.dqv : d.dQf;
+    double* fstage = split ? d.dq : d.dQf;
     rc = rows_in(d.pos, desc->cell_pos, n, dim, d.stage, s);
     if(!rc) rc = rows_in(d.cen, desc->cell_centroid, n, dim, d.stage, s);
     if(!rc) rc = rows_in(d.mid, desc->face_midpoint, F, dim, fstage, s);
@@ -1080,7 +1076,7 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
     int64_t bytes = n * S * 24 + (S + 1) * 1024 * 8 + 64;
     if(precision == SFX_PREC_SPLIT)
         bytes += n * 32 + n * 16 * (sfx_split_grad_vec4((int)D) + sfx_split_dwdt_vec4((int)D)) +
-                 F * 8 + F * D * 8 +
+                 F * 32 +
                  4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 24;
     else
         bytes += n * (int64_t)(sfx_fp64_record_bytes((int)D, SFX_REC_WS) +

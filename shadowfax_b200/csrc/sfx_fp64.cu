@@ -28,6 +28,7 @@
 
 #include "sfx_internal.h"
 #include "sfx_limiter.h"
+#include "sfx_wide.h"
 
 /* sfx_pow for the arguments sfx_powq does not settle, out of line */
 __host__ __device__ __noinline__ double sfx_pow_rare64(double x, double y);
@@ -210,28 +211,37 @@ struct Rec {
     static constexpr int ws = 8;
     static constexpr int grec = D == 3 ? 20 : 12;
     static constexpr int dq = D == 3 ? 6 : 4;
-    static constexpr int ggeo = D == 3 ? 12 : 10;
+    static constexpr int ggeo = 12;
     static constexpr int fgeo = D == 3 ? 16 : 12;
     /* cells per warp of the kernels with one lane per cell and variable */
     static constexpr int cells = 32 / S;
 };
 
+/* N doubles of a record on a 32-byte (N % 4 == 0) or 16-byte boundary */
 template <int N>
 __device__ __forceinline__ void load_record(const double* p, double* out) {
-    const double2* q = reinterpret_cast<const double2*>(p);
+    static_assert(N % 2 == 0, "whole 16-byte units");
 #pragma unroll
-    for(int i = 0; i < N / 2; ++i) {
-        const double2 v = __ldg(q + i);
-        out[2 * i] = v.x;
-        out[2 * i + 1] = v.y;
+    for(int i = 0; i < N; i += N % 4 ? 2 : 4) {
+        if constexpr(N % 4 == 0) {
+            sfx_load32(p + i, out + i);
+        } else {
+            const double2 v = __ldg(reinterpret_cast<const double2*>(p + i));
+            out[i] = v.x;
+            out[i + 1] = v.y;
+        }
     }
 }
 
 template <int N>
 __device__ __forceinline__ void store_record(double* p, const double* v) {
-    double2* q = reinterpret_cast<double2*>(p);
 #pragma unroll
-    for(int i = 0; i < N / 2; ++i) q[i] = make_double2(v[2 * i], v[2 * i + 1]);
+    for(int i = 0; i < N; i += N % 4 ? 2 : 4) {
+        if constexpr(N % 4 == 0)
+            sfx_store32(p + i, v + i);
+        else
+            *reinterpret_cast<double2*>(p + i) = make_double2(v[i], v[i + 1]);
+    }
 }
 
 /* a length, or a difference of positions, for which sfx_div_by's products and
@@ -283,7 +293,12 @@ __global__ void __launch_bounds__(128) k_face_records(sfx_dmesh m) {
         /* a NaN offset takes no part in the slope limiter */
         g[3 + 2 * D + l] = A == 0. ? __longlong_as_double(0x7ff8000000000000ll) : mid[l];
     }
-    if(D == 2) g[R::ggeo - 1] = 0.;
+    if(D == 2) {
+        /* the midpoint to the record's third 32 bytes */
+        g[8] = g[7];
+        g[9] = A == 0. ? g[7] : mid[1];
+        g[7] = g[10] = g[11] = 0.;
+    }
     store_record<R::ggeo>(m.ggeo + (size_t)f * R::ggeo, g);
     const double cn = norm<D>(cd);
     const double dn = norm<D>(dd);
@@ -302,7 +317,9 @@ __global__ void __launch_bounds__(128) k_face_records(sfx_dmesh m) {
         h[6 + 2 * D + l] = -dd[l] / dn;
     }
     if(D == 3) h[R::fgeo - 1] = 0.;
-    store_record<R::fgeo>(m.fgeo + (size_t)f * R::fgeo, h);
+    /* planes of 32 bytes per face: consecutive threads read consecutive faces */
+#pragma unroll
+    for(int q = 0; q < R::fgeo; q += 4) store_record<4>(m.fgeo + (size_t)q * F + 4 * (size_t)f, h + q);
 }
 
 /* each CSR entry with its neighbour cell, so that the gradient kernels load
@@ -502,7 +519,7 @@ constexpr int kGradBlock = 128, kGradStages = 4;
 template <int D>
 struct GradSlot {
     static constexpr int S = D + 2;
-    double2 geo[S];  /* A, 1/|r|, |r|, c, r (and, 2D, the midpoint's x) */
+    double2 geo[S];  /* A, 1/|r|, |r|, c, r */
     double W[S];     /* the neighbour's state */
     int2 ent;        /* CSR entry, neighbour (-1: mirror) */
     /* to 144 bytes (3D) and 112 (2D): a warp's cells on different banks */
@@ -618,8 +635,9 @@ __global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double g
 #pragma unroll
             for(int l = 0; l < D; ++l) d[l] = t[(l + 1) & 3] - cen[l];
         } else {
-            d[0] = __ldg(p + 7) - cen[0];
-            d[1] = __ldg(p + 8) - cen[1];
+            const double2 t = __ldg(reinterpret_cast<const double2*>(p + 8));
+            d[0] = t.x - cen[0];
+            d[1] = t.y - cen[1];
         }
         double dp = delta[0] * d[0] + delta[1] * d[1];
         if(D == 3) dp = dp + delta[D - 1] * d[D - 1];
@@ -1414,7 +1432,9 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
     FaceGeom<D> q;
     if(REC) {
         double h[R::fgeo];
-        load_record<R::fgeo>(m.fgeo + (size_t)f * R::fgeo, h);
+#pragma unroll
+        for(int k = 0; k < R::fgeo; k += 4)
+            load_record<4>(m.fgeo + (size_t)k * F + 4 * (size_t)f, h + k);
         q.iL = __double2loint(h[0]);
         q.iR = __double2hiint(h[0]);
         q.A = h[1];
@@ -1469,8 +1489,8 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
     double QLm, QRm = 0.;
     auto load_state = [&](int i, double* W, double& Qm) {
         if(REC) {
-            double t[6];
-            load_record<6>(m.ws + (size_t)i * R::ws, t);
+            double t[8];
+            load_record<8>(m.ws + (size_t)i * R::ws, t);
 #pragma unroll
             for(int k = 0; k < S; ++k) W[k] = t[k];
             Qm = t[S];
@@ -1667,7 +1687,9 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma
             for(int k = 0; k < S; ++k) W[k] = 0.;
         }
     }
-    double t[6];
+    double t[8];
+#pragma unroll
+    for(int k = 0; k < 8; ++k) t[k] = 0.;
 #pragma unroll
     for(int k = 0; k < S; ++k) {
         m.Q[(size_t)k * n + i] = Q[k];
@@ -1675,8 +1697,7 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma
         t[k] = W[k];
     }
     t[S] = Q[0];
-    if(D == 2) t[5] = 0.;
-    store_record<6>(ws, t);
+    store_record<8>(ws, t);
 }
 
 /* Host arrays are rows of one cell or face, device arrays field-major: the

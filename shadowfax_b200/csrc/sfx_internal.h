@@ -74,8 +74,8 @@ struct sfx_dmesh {
      *     {r1, |r|, 0, 0}) with c = midpoint - (x_L + x_R)/2 and
      *     r = x_L - x_R (right generator at its image/mirror position),
      *     computed in FP64 and rounded once;
-     * fi [F] int2: {L, R}; R = -1 mirror, R | 1<<30 periodic image;
-     * fsh [F]: periodic image shift, 2 bits per axis (0, +1, -1 box);
+     * fr [12 F] (2D) or [16 F] (3D): the face's cells and flux geometry (FaceRec,
+     *     sfx_split.cu), formed in FP64 and rounded once;
      * cw [2n] float4 cell record {rho, v.., p | Q.m, total area ..};
      * cg [G*n] float4 gradients (G = 4 in 3D, 2 in 2D: 64 / 32 bytes, so a
      *     record never straddles more 32-byte sectors than it fills);
@@ -86,11 +86,10 @@ struct sfx_dmesh {
      * an [dim][F] FP64 area vector A n (n from x_L to x_R), for the pressure
      *     force, so that the forces on a cell cancel to FP64 round-off in a
      *     uniform region;
-     * dqm [F] float2 {mass, energy} and dqv [dim][F] FP64 momentum: the
-     *     limited dQ received by the left cell. */
+     * dq [4 F]: the limited dQ received by the left cell, 32 bytes per face
+     *     (store_dq, sfx_split.cu). */
     float4* fg;
-    int2* fi;
-    uint8_t* fsh;
+    float* fr;
     float4* cw;
     float4* cg;
     float4* cdw;
@@ -112,8 +111,7 @@ struct sfx_dmesh {
     uint64_t t_now, t_next;
     double t_total;
     double* an;
-    float2* dqm;
-    double* dqv;
+    double* dq;
     double* stage; /* [n][S] rows on their way between W or Q and the host; no kernel of a
                       step touches it */
     /* exact solver, split pass: faces whose p* iteration falls back to
