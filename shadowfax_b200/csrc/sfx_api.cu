@@ -131,15 +131,16 @@ int32_t slowq_capacity(int64_t n_faces) {
     return (int32_t)(n_faces > 0 ? n_faces : 1);
 }
 
+/* a one-member group's prefix sums and the word behind them */
+constexpr int kSelfPre = 7;
+
 /* device table of a split mesh as a one-member launch group */
 int setup_self(sfx_mesh* m, cudaStream_t s) {
-    if(!m->self_tab) SFX_TRY(dalloc(m, &m->self_tab, 1));
-    if(!m->self_pre) SFX_TRY(dalloc(m, &m->self_pre, 6));
     sfx_group_entry e;
     std::memset(&e, 0, sizeof e);
     e.m = m->d;
     m->self_dt = 0.f;
-    SFX_TRY(cuda_ok(cudaMemsetAsync(m->self_pre, 0, 6 * sizeof(int32_t), s)));
+    SFX_TRY(cuda_ok(cudaMemsetAsync(m->self_pre, 0, kSelfPre * sizeof(int32_t), s)));
     /* pageable source: staged before the call returns */
     return h2d(m->self_tab, &e, 1, s);
 }
@@ -272,7 +273,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
         A(&d.slowq, (size_t)d.slowq_cap);
         A(&d.slowq_n, 1);
         A(&m->self_tab, 1);
-        A(&m->self_pre, 6);
+        A(&m->self_pre, kSelfPre);
     } else {
         A(&d.ws, n * rec_doubles(dim, SFX_REC_WS));
         A(&d.grec, n * rec_doubles(dim, SFX_REC_GREC));
@@ -675,6 +676,8 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         d.slowq_cap = slowq_capacity(F);
         A(&d.slowq, (size_t)d.slowq_cap);
         A(&d.slowq_n, 1);
+        A(&m->self_tab, 1);
+        A(&m->self_pre, kSelfPre);
     }
     int rc = arrays.allocate(m);
     if(rc != SFX_OK) {
@@ -1077,7 +1080,7 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
     if(precision == SFX_PREC_SPLIT)
         bytes += n * 32 + n * 16 * (sfx_split_grad_vec4((int)D) + sfx_split_dwdt_vec4((int)D)) +
                  F * 32 +
-                 4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 24;
+                 4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 28;
     else
         bytes += n * (int64_t)(sfx_fp64_record_bytes((int)D, SFX_REC_WS) +
                                sfx_fp64_record_bytes((int)D, SFX_REC_GREC)) +

@@ -98,7 +98,7 @@ int reserve(sfx_group* g, int n) {
     g->d_steps = nullptr;
     g->cap = 0;
     int rc = cuda_ok(cudaMalloc((void**)&g->dev.tab, sizeof(sfx_group_entry) * cap));
-    if(!rc) rc = cuda_ok(cudaMalloc((void**)&g->dev.pre, sizeof(int32_t) * 3 * (cap + 1)));
+    if(!rc) rc = cuda_ok(cudaMalloc((void**)&g->dev.pre, sizeof(int32_t) * (3 * (cap + 1) + 1)));
     if(!rc) rc = cuda_ok(cudaMalloc((void**)&g->d_err_out, sizeof(sfx_dev_error) * cap));
     if(!rc) g->cap = cap;
     return rc;

@@ -159,7 +159,8 @@ struct sfx_group_entry {
 };
 
 /* device view of a launch group: table of meshes and, per phase, the prefix
- * sum of blocks over the meshes (3 arrays of n_meshes + 1) */
+ * sum of blocks over the meshes (3 arrays of n_meshes + 1, then one word: whether a face
+ * was queued in this step) */
 struct sfx_group_dev {
     sfx_group_entry* tab;
     int32_t* pre;

@@ -1093,10 +1093,9 @@ __device__ __forceinline__ void side64(const sfx_solver_params& s, double p, dou
  * step to first order (error of the order of the step squared).  Two FP64
  * powers at most instead of one per FP64 iteration plus two per face.
  * Returns false, and the FP64 iteration runs from the start, outside the
- * range where FP32 is safe, when the FP32 iteration does not converge or
- * takes a Newton step to (nearly) zero pressure (where the reference's
- * iteration can stop at p = 0), when the FP64 step is not small, or when it
- * moves a side between shock and rarefaction. */
+ * range where FP32 is safe, when the FP32 iteration takes a Newton step to
+ * (nearly) zero pressure where the reference's can stop at p = 0, or when four
+ * FP64 steps leave no small step that keeps each side's wave. */
 template <bool G53 = false>
 __device__ __forceinline__ bool fast_root(const sfx_solver_params& s, double rL, double pL,
                                           double rR, double pR, double aL, double aR, double vL,
@@ -1142,30 +1141,50 @@ __device__ __forceinline__ bool fast_root(const sfx_solver_params& s, double rL,
     }
     pg = fmaxf(floorp, pg);
     if(!(pg > 0.f && pg < 3e38f)) return false;
+    /* A Newton step below (nearly) zero pressure: where f(0) lies under the
+     * cutoff the reference stops at p = 0 (left to the queue, and so is an f(0)
+     * too near the cutoff for FP32 to tell); elsewhere it brackets the root in
+     * [0, p], and a step to p / 100 does the same: f is concave, so iterates
+     * that land left of the root rise to it. */
+    const bool bracket = dv - tdgm1 * (faL + faR) > (float)s.cutoff + 1e-4f * fabsf((float)s.cutoff);
     for(int it = 0;; ++it) {
         float f1, g1, f2, g2;
         side(pg, fpL, AL, BL, faL, frL, f1, g1);
         side(pg, fpR, AR, BR, faR, frR, f2, g2);
-        const float pn = pg - (f1 + f2 + dv) * rcp32(g1 + g2);
-        if(!(pn > 1e-3f * pg && pn < 3e38f) || it >= 16) return false;
-        const bool conv = fabsf(pn - pg) <= 1e-6f * pg;
+        float pn = pg - (f1 + f2 + dv) * rcp32(g1 + g2);
+        if(!(pn < 3e38f)) return false;
+        if(!(pn > 1e-3f * pg)) {
+            if(!bracket) return false;
+            pn = 1e-2f * pg;
+        }
+        /* near vacuum f's round-off exceeds that step: the FP64 steps decide */
+        const bool conv = fabsf(pn - pg) <= 1e-6f * pg || it >= 10;
         pg = pn;
         if(conv) break;
     }
-    const double p0 = (double)pg;
-    double fpl, fpr;
-    side64<G53>(s, p0, rL, pL, aL, fL, fpl, zL);
-    side64<G53>(s, p0, rR, pR, aR, fR, fpr, zR);
-    const double dp = -(fL + fR + (vR - vL)) / (fpl + fpr);
-    const double p1 = p0 + dp;
-    if(!(fabs(dp) <= 1e-5 * p0) || (p0 > pL) != (p1 > pL) || (p0 > pR) != (p1 > pR))
-        return false;
-    fL += fpl * dp;
-    fR += fpr * dp;
-    zL *= 1. + s.gm1d2g * dp / p0;
-    zR *= 1. + s.gm1d2g * dp / p0;
-    p = p1;
-    return true;
+    /* One FP64 step is enough from most FP32 roots.  From the others (a root
+     * near zero pressure, where the two-rarefaction guess cancels, or at a
+     * side's pressure, where its branch changes) two or three are: far cheaper
+     * here than the queue's full iteration in a launch of its own, whose few
+     * faces are one long dependent chain. */
+    double p0 = (double)pg;
+    for(int it = 0;; ++it) {
+        double fpl, fpr;
+        side64<G53>(s, p0, rL, pL, aL, fL, fpl, zL);
+        side64<G53>(s, p0, rR, pR, aR, fR, fpr, zR);
+        const double dp = -(fL + fR + (vR - vL)) / (fpl + fpr);
+        const double p1 = p0 + dp;
+        if(fabs(dp) <= 1e-5 * p0 && (p0 > pL) == (p1 > pL) && (p0 > pR) == (p1 > pR)) {
+            fL += fpl * dp;
+            fR += fpr * dp;
+            zL *= 1. + s.gm1d2g * dp / p0;
+            zR *= 1. + s.gm1d2g * dp / p0;
+            p = p1;
+            return true;
+        }
+        if(it >= 3 || !(p1 > 1e-3 * p0)) return false;
+        p0 = p1;
+    }
 }
 
 template <int D, int MODE>
@@ -1801,8 +1820,9 @@ __device__ __forceinline__ int wave_class(const sfx_solver_params& s, const Face
     const float g = (float)s.gamma, tdgm1 = (float)s.tdgm1, e = (float)s.gm1d2g;
     const float aL = sqrt32(g * pL * rcp32(rL)), aR = sqrt32(g * pR * rcp32(rR));
     const float dv = vR - vL;
-    /* vacuum generation (and states near it, FP32 being coarse): the queue */
-    if(!(tdgm1 * (aL + aR) > 1.0001f * dv)) return kClassQueue;
+    /* vacuum generation, and states near it (FP32 being coarse): phase 3
+     * decides in FP64; beside the two rarefactions it is or nearly is */
+    if(!(tdgm1 * (aL + aR) > 1.0001f * dv)) return kClassRR;
     const bool lowL = pL <= pR;
     const float pmin = lowL ? pL : pR, pmax = lowL ? pR : pL;
     /* f(p_min): the lower side contributes 0, the other one rarefies */
@@ -1857,57 +1877,58 @@ __device__ __forceinline__ int exact_fast(const sfx_solver_params& s,
     const double g = s.gamma;
     const double aL = sqrt(g * pL / rL);
     const double aR = sqrt(g * pR / rR);
-    if(s.tdgm1 * (aL + aR) <= vR - vL) return kDefer;
-    double p, fL, fR, zL, zR;
-    if(!fast_root<G53>(s, rL, pL, rR, pR, aL, aR, vL, vR, p, fL, fR, zL, zR)) return kDefer;
-    /* sampling at x/t = 0 (ExactRiemannSolver.cpp:178-265): the side, the
-     * half state's density and pressure, and its velocity shift along n */
-    const double u = 0.5 * (vL + vR) + 0.5 * (fR - fL);
-    const bool right = u < 0.;
-    double srho = right ? rR : rL, spr = right ? pR : pL, vhalf = 0.;
-    if(right) {
-        const double r = p / pR;
-        if(p > pR) {
-            if(vR + aR * sqrt(s.gp1d2g * r + s.gm1d2g) > 0.) {
-                srho = rR * (r + s.gm1dgp1) / (s.gm1dgp1 * r + 1.);
-                spr = p;
-                vhalf = u - vR;
-            }
-        } else if(vR + aR > 0.) {
-            if(u + aR * zR <= 0.) {
-                const double base = s.tdgp1 - s.gm1dgp1 / aR * vR;
-                const double b3 = base * base * base;
-                srho = rR * (G53 ? b3 : xpow(base, s.tdgm1));
-                vhalf = s.tdgp1 * (-aR + s.gm1d2 * vR) - vR;
-                spr = pR * (G53 ? b3 * base * base : xpow(base, s.tgdgm1));
-            } else {
-                srho = rR * (G53 ? zR * zR * zR : xpow(r, s.ginv));
-                spr = p;
-                vhalf = u - vR;
-            }
-        }
+    /* vacuum opens between the sides (ExactRiemannSolver.cpp:376-446) */
+    const bool vac = s.tdgm1 * (aL + aR) <= vR - vL;
+    double p = 0., u = 0., fL, fR, zL = 0., zR = 0.;
+    bool right, empty = false;
+    if(vac) {
+        right = vL + s.tdgm1 * aL < 0.;
+        empty = right && vR - s.tdgm1 * aR > 0.;
     } else {
-        const double r = p / pL;
-        if(p > pL) {
-            if(vL - aL * sqrt(s.gp1d2g * r + s.gm1d2g) < 0.) {
-                srho = rL * (r + s.gm1dgp1) / (s.gm1dgp1 * r + 1.);
-                spr = p;
-                vhalf = u - vL;
-            }
-        } else if(vL - aL < 0.) {
-            if(u - aL * zL > 0.) {
-                const double base = s.tdgp1 + s.gm1dgp1 / aL * vL;
-                const double b3 = base * base * base;
-                srho = rL * (G53 ? b3 : xpow(base, s.tdgm1));
-                vhalf = s.tdgp1 * (aL + s.gm1d2 * vL) - vL;
-                spr = pL * (G53 ? b3 * base * base : xpow(base, s.tgdgm1));
-            } else {
-                srho = rL * (G53 ? zL * zL * zL : xpow(r, s.ginv));
-                spr = p;
-                vhalf = u - vL;
-            }
+        if(!fast_root<G53>(s, rL, pL, rR, pR, aL, aR, vL, vR, p, fL, fR, zL, zR)) return kDefer;
+        u = 0.5 * (vL + vR) + 0.5 * (fR - fL);
+        right = u < 0.;
+    }
+    /* sampling at x/t = 0 (ExactRiemannSolver.cpp:178-265) on the side the
+     * interface lies in, the right one mirrored onto the left: the half
+     * state's density and pressure, and its velocity shift along n */
+    const double rK = right ? rR : rL, pK = right ? pR : pL, aK = right ? aR : aL;
+    const double zK = right ? zR : zL;
+    const double vK = right ? -vR : vL, uK = right ? -u : u;
+    double srho = rK, spr = pK, vhalf = 0.;
+    bool fan = vac && vK < aK;
+    if(!vac) {
+        const double r = p / pK;
+        bool star;
+        double rho = 0.;
+        if(p > pK) {
+            star = vK - aK * sqrt(s.gp1d2g * r + s.gm1d2g) < 0.;
+            if(star) rho = rK * (r + s.gm1dgp1) / (s.gm1dgp1 * r + 1.);
+        } else {
+            const double tail = uK - aK * zK;
+            const bool inside = vK - aK < 0.;
+            fan = inside && (right ? tail >= 0. : tail > 0.);
+            star = inside && !fan;
+            if(star) rho = rK * (G53 ? zK * zK * zK : xpow(r, s.ginv));
+        }
+        if(star) {
+            srho = rho;
+            spr = p;
+            vhalf = uK - vK;
         }
     }
+    if(fan) {
+        const double base = s.tdgp1 + s.gm1dgp1 / aK * vK;
+        const double b3 = base * base * base;
+        srho = rK * (G53 ? b3 : xpow(base, s.tdgm1));
+        spr = pK * (G53 ? b3 * base * base : xpow(base, s.tgdgm1));
+        vhalf = s.tdgp1 * (aK + s.gm1d2 * vK) - vK;
+    }
+    if(empty) {
+        srho = 0.;
+        spr = 0.;
+    }
+    if(right) vhalf = -vhalf;
     /* the half state's velocity (in the face's frame; + v in the lab frame)
      * and its flux (ExactRiemannSolver::get_flux contracted with n,
      * :815-880) */
@@ -1942,13 +1963,16 @@ __device__ __forceinline__ int exact_fast(const sfx_solver_params& s,
 
 /* queue face f of the block's mesh for the lanes with `push` set: one
  * atomic per warp (all 32 lanes call this) */
-__device__ __forceinline__ void queue_faces(const sfx_dmesh& m, bool push, int f) {
+__device__ __forceinline__ void queue_faces(const sfx_dmesh& m, bool push, int f, int* any) {
     const unsigned q = __ballot_sync(0xffffffffu, push);
     if(!q) return;
     const int lane = threadIdx.x & 31;
     const int leader = __ffs(q) - 1;
     int base = 0;
-    if(lane == leader) base = atomicAdd(m.slowq_n, __popc(q));
+    if(lane == leader) {
+        base = atomicAdd(m.slowq_n, __popc(q));
+        *(volatile int*)any = 1;
+    }
     base = __shfl_sync(0xffffffffu, base, leader);
     const int at = base + __popc(q & ((1u << lane) - 1u));
     /* the queue has room for every face and each face is queued at most once
@@ -2069,6 +2093,14 @@ __device__ __forceinline__ int group_mesh_of_block(const int* __restrict__ pre, 
     return s_mesh;
 }
 
+/* whether any member queued a face in this step: one word behind the group's
+ * three prefix arrays, cleared by the gradient launch, so that the queued-face
+ * launch of a step that queued none (the usual one) ends at once instead of
+ * scanning the members */
+__device__ __forceinline__ int* group_queued(const int* pre, int nm) {
+    return const_cast<int*>(pre) + 3 * (nm + 1);
+}
+
 /* a member whose step counter reached 0 is done: all its blocks return */
 __device__ __forceinline__ bool member_done(const sfx_group_entry* tab, int mi) {
     const int32_t* sl = tab[mi].steps_left;
@@ -2090,6 +2122,7 @@ __global__ void __launch_bounds__(kExactBlock, MINB)
     __shared__ int sf[kExactBlock];
     __shared__ int sbase[kNClass][NW];
     __shared__ int stotal;
+    int* any = group_queued(pre - (nm + 1), nm); /* pre: the second prefix array */
     const int mi = group_mesh_of_block(pre, nm);
     if(member_done(tab, mi)) return; /* the same for every thread of the block */
     const sfx_dmesh& m = tab[mi].m;
@@ -2112,7 +2145,7 @@ __global__ void __launch_bounds__(kExactBlock, MINB)
     if(f < sfx_flux_faces(m) && !failed(m.err) &&
        face_work<D, true, MOVING, TILE>(m, (float)sp.gamma, dt, f, w, tile))
         cls = wave_class<D>(sp, w);
-    queue_faces(m, cls == kClassQueue, f);
+    queue_faces(m, cls == kClassQueue, f, any);
     if(TILE && !tile_ok) mbar_wait(tile_bar, kTileWaitLimit); /* copies still in flight */
     /* phase 2: counting sort by class */
     unsigned mine = 0; /* the ballot of this thread's class */
@@ -2181,12 +2214,13 @@ __global__ void __launch_bounds__(kExactBlock, MINB)
             face_dq<D>(m, fq, v, F, st);
         }
     }
-    queue_faces(m, push, fq);
+    queue_faces(m, push, fq, any);
 }
 
 template <int D, int LPC>
 __global__ void __launch_bounds__(256, 4) k_group_sgrad(const sfx_group_entry* tab, const int* pre,
                                                      int nm, float gamma) {
+    if(blockIdx.x == 0 && threadIdx.x == 0) *group_queued(pre, nm) = 0;
     const int mi = group_mesh_of_block(pre, nm);
     if(member_done(tab, mi)) return;
     sgrad_body<D, LPC>(tab[mi].m, gamma,
@@ -2199,6 +2233,7 @@ __global__ void __launch_bounds__(256, MINB)
         k_group_sfaces(const sfx_group_entry* tab, const int* pre, int nm,
                        sfx_solver_params sp) {
     static_assert(SOLVER == SFX_SOLVER_HLLC, "the exact solver has k_group_sfaces_exact");
+    int* any = group_queued(pre - (nm + 1), nm); /* pre: the second prefix array */
     const int mi = group_mesh_of_block(pre, nm);
     if(member_done(tab, mi)) return; /* the same for every thread of the block */
     const sfx_dmesh& m = tab[mi].m;
@@ -2211,12 +2246,12 @@ __global__ void __launch_bounds__(256, MINB)
         if(!ok && threadIdx.x == 0) report_face(m.err, f, SFX_ERR_CUDA);
         const bool push = sfaces_body<D, SOLVER, kSolveDefer, STORED_DW, MOVING, true>(
                 m, sp, tab[mi].dt, f, tile);
-        queue_faces(m, push, f);
+        queue_faces(m, push, f, any);
         if(!ok) mbar_wait(&ts.mbar, kTileWaitLimit); /* copies still in flight */
     } else {
         const bool push =
                 sfaces_body<D, SOLVER, kSolveDefer, STORED_DW, MOVING>(m, sp, tab[mi].dt, f);
-        queue_faces(m, push, f);
+        queue_faces(m, push, f, any);
     }
 }
 
@@ -2232,8 +2267,10 @@ constexpr int kSlowBlock = 128, kSlowChunk = 2048, kSlowPer = kSlowChunk / kSlow
 
 template <int D, bool MOVING = false, int SOLVER = SFX_SOLVER_EXACT,
           bool STORED_DW = SOLVER == SFX_SOLVER_EXACT>
-__global__ void __launch_bounds__(kSlowBlock) k_group_sfaces_slow(const sfx_group_entry* tab,
-                                                                 int nm, sfx_solver_params sp) {
+__global__ void __launch_bounds__(kSlowBlock)
+        k_group_sfaces_slow(const sfx_group_entry* tab, const int* pre, int nm,
+                            sfx_solver_params sp) {
+    if(*(volatile const int*)group_queued(pre, nm) == 0) return;
     __shared__ int spre[kSlowChunk + 1];
     __shared__ int swarp[kSlowBlock / 32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -2336,15 +2373,19 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
             if(g->moving) {
                 /* a moving mesh stepped alone: the face kernels with the boost */
                 if(sp->kind == SFX_SOLVER_EXACT) {
-                    k_group_sfaces_exact<D, 4, true><<<g->blocks[1], kExactBlock, 0, s>>>(
-                            g->tab, pre1, nm, *sp);
+                    if(sp->gamma == 5. / 3.)
+                        k_group_sfaces_exact<D, 4, true, true>
+                                <<<g->blocks[1], kExactBlock, 0, s>>>(g->tab, pre1, nm, *sp);
+                    else
+                        k_group_sfaces_exact<D, 4, true><<<g->blocks[1], kExactBlock, 0, s>>>(
+                                g->tab, pre1, nm, *sp);
                     k_group_sfaces_slow<D, true><<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(
-                            g->tab, nm, *sp);
+                            g->tab, g->pre, nm, *sp);
                 } else {
                     k_group_sfaces<D, SFX_SOLVER_HLLC, 4, false, true>
                             <<<g->blocks[1], 256, 0, s>>>(g->tab, pre1, nm, *sp);
                     k_group_sfaces_slow<D, true, SFX_SOLVER_HLLC>
-                            <<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, nm, *sp);
+                            <<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, g->pre, nm, *sp);
                 }
                 sfx_count_launches(1);
             } else if(sp->kind == SFX_SOLVER_EXACT) {
@@ -2367,7 +2408,7 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
                 else
                     k_group_sfaces_exact<D, 4><<<g->blocks[1], kExactBlock, 0, s>>>(
                             g->tab, pre1, nm, *sp);
-                k_group_sfaces_slow<D><<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, nm, *sp);
+                k_group_sfaces_slow<D><<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, g->pre, nm, *sp);
                 sfx_count_launches(1);
             } else {
                 /* HLLC; then the faces whose FP32 flux was not finite, in FP64 */
@@ -2376,7 +2417,7 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
                     k_group_sfaces<D, SFX_SOLVER_HLLC, 4, true><<<g->blocks[1], 256, 0, s>>>(
                             g->tab, pre1, nm, *sp);
                     k_group_sfaces_slow<D, false, SFX_SOLVER_HLLC, true>
-                            <<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, nm, *sp);
+                            <<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, g->pre, nm, *sp);
                 } else {
                     if(v == 4)
                         k_group_sfaces<D, SFX_SOLVER_HLLC, 5, false, false, true>
@@ -2391,7 +2432,7 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
                         k_group_sfaces<D, SFX_SOLVER_HLLC, 4><<<g->blocks[1], 256, 0, s>>>(
                                 g->tab, pre1, nm, *sp);
                     k_group_sfaces_slow<D, false, SFX_SOLVER_HLLC>
-                            <<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, nm, *sp);
+                            <<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, g->pre, nm, *sp);
                 }
                 sfx_count_launches(1);
             }
@@ -2471,11 +2512,12 @@ int sfx_split_export_dQ(const sfx_dmesh* m, void* stream) {
 int sfx_split_face_variant_kernel(const sfx_solver_params* sp, int variant) {
     if(variant < 0 || variant >= SFX_FACE_VARIANTS) return 0;
     if(sp->kind == SFX_SOLVER_EXACT) {
-        /* the gamma = 5/3 forms (2: 64 registers, 3: 80) exist for that gamma
-         * only; 4 (left cells staged) is the gamma = 5/3 form at that gamma
-         * and the generic one at others */
-        if(sp->gamma != 5. / 3. && (variant == 2 || variant == 3)) return variant - 2;
-        return variant;
+        /* kernels 2 (64 registers) and 3 (80) are the gamma = 5/3 forms of 0 and
+         * 1: the fifth root and integer powers take 98 us where the general
+         * powers take 124 (1.29 million faces in 3D), so variants 0 and 1 run
+         * them at that gamma; 4 (left cells staged) likewise */
+        if(variant >= 4) return variant;
+        return (variant & 1) + (sp->gamma == 5. / 3. ? 2 : 0);
     }
     return variant; /* HLLC: 3 is the 48-register kernel, 4 that with staged left cells */
 }

@@ -279,8 +279,8 @@ class FluxPass:
 
     def set_face_variant(self, variant: int):
         """split pass: face-kernel variant (SFX_FACE_VARIANTS: 0 and 1 the
-        64- and 80-register kernels; 2 and 3 the exact solver's gamma = 5/3
-        forms, HLLC's stored dW/dt; include/sfxflux.h)"""
+        64- and 80-register kernels; 2 HLLC's stored dW/dt, 3 its
+        48-register kernel; include/sfxflux.h)"""
         L.check(L.lib().sfx_mesh_set_face_variant(self.h, variant), "sfx_mesh_set_face_variant")
 
     def tune_faces(self, dt: float, reps: int = 3) -> int:
