@@ -286,8 +286,9 @@ int sfx_mesh_clone(sfx_ctx* ctx, sfx_mesh* base, sfx_mesh** out);
 /* device bytes a clone of `base` at `precision` allocates */
 int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision);
 
-/* split pass: lanes of a warp that share one cell in the gradient and update
- * kernels (1, 2, 4, 8 or 16; default 1 in 2D, 4 in 3D).  Changes the summation
+/* split pass: lanes of a warp that share one cell in the gradient kernel (1, 2,
+ * 4, 8 or 16; default 2 in 2D, 4 in 3D; the update kernel takes a quarter of
+ * them, at least 1).  Changes the summation
  * tree of the per-cell sums, not the algorithm. */
 int sfx_mesh_set_lanes(sfx_mesh* mesh, int32_t lanes);
 /* split pass: face-kernel variant: 0 (64 registers, four 256-thread blocks

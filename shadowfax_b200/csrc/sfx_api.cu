@@ -176,7 +176,7 @@ int run_phase(sfx_mesh* m, int phase, double dt, int write_branch, cudaStream_t 
             g.blocks[0] = b[0];
             g.blocks[1] = b[1];
             sfx_split_blocks(m->d.dim, m->d.lanes, sfx_update_cells(m->d), 0, b);
-            g.blocks[2] = b[0];
+            g.blocks[2] = b[2];
         }
         return sfx_split_group_phase(&g, phase, &c->sp, s);
     }

@@ -264,10 +264,6 @@ int sfx_mesh_download_async(sfx_mesh* m, double* W, double* Q, void* stream);
 /* sfx_mesh_clone with its device setup on `stream`, not waited for */
 int sfx_mesh_clone_async(sfx_ctx* ctx, sfx_mesh* base, void* stream, sfx_mesh** out);
 
-/* lanes per cell of the split gradient and update kernels before any
- * tuning, the same for a mesh alone and in a group: one in 2D (about six
- * faces per cell), four in 3D (about sixteen); measured fastest on 300,000-cell
- * meshes */
 /* float4s of the split pass's per-cell gradient record (cg) and of its
  * per-cell dW/dt record (cdw) */
 inline int sfx_split_grad_vec4(int dim) {
@@ -278,8 +274,18 @@ inline int sfx_split_dwdt_vec4(int dim) {
     return (dim + 2 + 3) / 4;
 }
 
+/* Lanes per cell of the split gradient kernel before any tuning, the same for
+ * a mesh alone and in a group.  Gradients of 464,159 cells in 2D (six faces a
+ * cell): 64 us at 1 lane, 57 at 2, 73 at 4; of 262,144 cells in 3D (fifteen):
+ * 116, 91, 88 at 4, 115 at 8. */
 inline int sfx_default_lanes(int dim) {
-    return dim == 2 ? 1 : 4;
+    return dim == 2 ? 2 : 4;
+}
+/* and of the update kernel, whose lanes keep three faces in flight each and
+ * share the cell's get_W: 34 us at 1 lane, 42 at 2 (2D); 48, 49, 56 at 4, 85 at
+ * 8 (3D) */
+SFX_RANGE_HD constexpr int sfx_update_lanes(int lanes) {
+    return lanes >= 4 ? lanes / 4 : 1;
 }
 
 /* grouped launches (sfx_split.cu) */

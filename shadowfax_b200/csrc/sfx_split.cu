@@ -2439,8 +2439,8 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
         }
     } else {
         if(g->blocks[2])
-            k_group_sapply<D, LPC><<<g->blocks[2], 256, 0, s>>>(g->tab, g->pre + 2 * (nm + 1),
-                                                                 nm, sp->gamma);
+            k_group_sapply<D, sfx_update_lanes(LPC)><<<g->blocks[2], 256, 0, s>>>(
+                    g->tab, g->pre + 2 * (nm + 1), nm, sp->gamma);
     }
     if(g->blocks[phase]) sfx_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? SFX_OK : SFX_ERR_CUDA;
@@ -2549,7 +2549,7 @@ int sfx_split_blocks(int dim, int lanes, int n_cells, int n_faces, int32_t* out)
     (void)dim;
     out[0] = grid_for((long long)n_cells * lanes, 256);
     out[1] = grid_for(n_faces, 256);
-    out[2] = out[0];
+    out[2] = grid_for((long long)n_cells * sfx_update_lanes(lanes), 256);
     return SFX_OK;
 }
 
