@@ -249,6 +249,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     const int64_t n = d.n_cells, F = d.n_faces;
     const int S = d.S, dim = d.dim;
     d.W = d.Q = d.stage = d.dQf = d.ws = d.grec = nullptr;
+    d.listed = d.listed_n = nullptr;
     d.branch = nullptr;
     d.err = nullptr;
     d.totals_scratch = nullptr;
@@ -278,6 +279,8 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
         A(&d.ws, n * rec_doubles(dim, SFX_REC_WS));
         A(&d.grec, n * rec_doubles(dim, SFX_REC_GREC));
         A(&d.dQf, F * rec_doubles(dim, SFX_REC_DQ));
+        A(&d.listed, F);
+        A(&d.listed_n, 1);
         A(&d.branch, F);
     }
     int rc = arrays.allocate(m);
@@ -409,7 +412,7 @@ int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
          * order); face velocities */
         auto rec = [&](int what) { return (int64_t)sfx_fp64_record_bytes(dim, what); };
         bytes += n * (rec(SFX_REC_WS) + rec(SFX_REC_GREC)) +
-                 F * (rec(SFX_REC_DQ) + rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO) + 8 * dim) +
+                 F * (rec(SFX_REC_DQ) + rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO) + 8 * dim + 4) +
                  nnz * 4;
     } else {
         bytes += F * 8 * (dim + S); /* face velocities, dQf */
@@ -651,6 +654,8 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         A(&d.ws, n * rec_doubles(dim, SFX_REC_WS));
         A(&d.grec, n * rec_doubles(dim, SFX_REC_GREC));
         A(&d.dQf, F * rec_doubles(dim, SFX_REC_DQ));
+        A(&d.listed, F);
+        A(&d.listed_n, 1);
         A(&d.ggeo, F * rec_doubles(dim, SFX_REC_GGEO));
         A(&d.fgeo, F * rec_doubles(dim, SFX_REC_FGEO));
     } else {
@@ -1084,7 +1089,7 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
     else
         bytes += n * (int64_t)(sfx_fp64_record_bytes((int)D, SFX_REC_WS) +
                                sfx_fp64_record_bytes((int)D, SFX_REC_GREC)) +
-                 F * (4 + (int64_t)sfx_fp64_record_bytes((int)D, SFX_REC_DQ)) + 512;
+                 F * (8 + (int64_t)sfx_fp64_record_bytes((int)D, SFX_REC_DQ)) + 512;
     return bytes;
 }
 

@@ -351,6 +351,7 @@ template <int D, bool REC>
 __global__ void __launch_bounds__(128) k_gradients(sfx_dmesh m, double gamma) {
     constexpr int S = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(REC && i == 0) *m.listed_n = 0; /* a new step's list */
     if(i >= sfx_grad_cells(m) || failed(m.err)) return;
     /* local time steps: an inactive cell keeps its gradients (src/Simulation.cpp:414-420) */
     if(m.local && m.tstart[i] != m.t_now) return;
@@ -532,6 +533,7 @@ __global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double g
     constexpr int S = R::S;
     static_assert(sizeof(GradSlot<D>) == (D == 3 ? 144 : 112), "slot layout");
     __shared__ __align__(16) GradSlot<D> ring[kGradBlock / 32][kGradStages][R::cells];
+    if(blockIdx.x == 0 && threadIdx.x == 0) *m.listed_n = 0; /* a new step's list */
     const int lane = threadIdx.x & 31;
     const int slot = lane / S, k = lane - slot * S;
     const int i = ((blockIdx.x * kGradBlock + threadIdx.x) >> 5) * R::cells + slot;
@@ -720,7 +722,7 @@ __device__ __forceinline__ double sound(const sfx_solver_params& s, const double
  * ratio p / p_K (f, f', the sampling), which share the logarithm.  Out of line
  * because the solver has some twenty power sites: inlined, its code overran
  * the instruction cache (21.5 of 27 stall cycles per issue were instruction
- * fetch; 807,000 random-field faces took 6.1 ms, now 0.82 ms). */
+ * fetch; 807,000 random-field faces took 6.1 ms, then 0.82 ms). */
 struct LogPair {
     double x, h, l; /* h is NaN where x is not a positive normal number */
 };
@@ -728,7 +730,6 @@ struct LogPair {
 __device__ __noinline__ LogPair xlog(double x) {
     LogPair p;
     p.x = x;
-    p.l = 0.;
     if(!sfx_powq_log(x, &p.h, &p.l)) p.h = __longlong_as_double(0x7ff8000000000000ll);
     return p;
 }
@@ -737,8 +738,7 @@ __device__ __noinline__ double xexp(LogPair p, double y) {
     const double th = y * p.h;
     const double tl = sfx_fma(y, p.h, -th) + y * p.l;
     double r;
-    if(fabs(th) < 22. && sfx_powq_exp(th, tl, &r)) return r;
-    return sfx_pow_rare64(p.x, y);
+    return sfx_powq_exp(th, tl, &r) ? r : sfx_pow_rare64(p.x, y);
 }
 
 __device__ __forceinline__ double xpow(double x, double y) {
@@ -1054,25 +1054,26 @@ __device__ ExactOut exact_solve(const sfx_solver_params& s, double* WL, double* 
     const double fp = WL[D + 1] > 0. && WR[D + 1] > 0.
                               ? s.tdgm1 * aL * (0. - 1.) + s.tdgm1 * aR * (0. - 1.) + (vR - vL)
                               : ffl<D>(s, p, WL, WR, vL, vR, aL, aR, last);
-    double fpguess = ffl<D>(s, pguess, WL, WR, vL, vR, aL, aR, last);
+    double fpguess;
     int newton = 0, brent_it = 0, mode;
     bool errexit = false, noconv = false;
     /* The reference has one Newton loop per mode: below the cutoff it runs to
      * the tolerance with p kept non-negative; above it, only while f < 0 (and
-     * not at all when f(0) and f(guess) differ in sign).  One loop here. */
+     * not at all when f(0) and f(guess) differ in sign).  One loop here, and one
+     * evaluation site. */
     const bool only_newton = fp < s.cutoff;
-    if(only_newton || fp * fpguess >= 0.) {
-        while(fabs(p - pguess) > tol * 0.5 * (p + pguess) && (only_newton || fpguess < 0.)) {
-            if(newton >= SFX_MAX_ITER) {
-                noconv = true;
-                break;
-            }
-            ++newton;
-            p = pguess;
-            pguess = pguess - fpguess / fprime<D>(s, WL, WR, aL, aR, last);
-            if(only_newton && pguess < 0.) pguess = 0.;
-            fpguess = ffl<D>(s, pguess, WL, WR, vL, vR, aL, aR, last);
+    for(;;) {
+        fpguess = ffl<D>(s, pguess, WL, WR, vL, vR, aL, aR, last);
+        if(newton == 0 && !(only_newton || fp * fpguess >= 0.)) break;
+        if(!(fabs(p - pguess) > tol * 0.5 * (p + pguess) && (only_newton || fpguess < 0.))) break;
+        if(newton >= SFX_MAX_ITER) {
+            noconv = true;
+            break;
         }
+        ++newton;
+        p = pguess;
+        pguess = pguess - fpguess / fprime<D>(s, WL, WR, aL, aR, last);
+        if(only_newton && pguess < 0.) pguess = 0.;
     }
     if(only_newton) {
         mode = 1 << 3;
@@ -1402,75 +1403,88 @@ __device__ __forceinline__ void face_geom(const sfx_dmesh& m, int f, FaceGeom<D>
  * FP64 latency at 16 warps per SM (128 registers). */
 constexpr int kFaceArrays = 0, kFaceRecords = 1, kFaceMoving = 2;
 
-template <int D, int SOLVER, int MODE>
-__global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp,
-                                               double dt, int write_branch) {
+/* a face's Riemann problem and what its dQ needs: predicted states, normal,
+ * face velocity, dt A, and the over-flux limits (VorFace.cpp:837-866) */
+template <int D>
+struct FaceProblem {
+    double WL[D + 2], WR[D + 2], n[D], v[D];
+    double dtA, limL, limR;
+    bool has_right;
+};
+
+template <int D, bool REC>
+__device__ __forceinline__ void store_dQ(const sfx_dmesh& m, int f, const double* v) {
+    constexpr int S = D + 2;
+    if(REC) {
+        double t[Rec<D>::dq];
+#pragma unroll
+        for(int k = 0; k < Rec<D>::dq; ++k) t[k] = k < S ? v[k < S ? k : 0] : 0.;
+        store_record<Rec<D>::dq>(m.dQf + (size_t)f * Rec<D>::dq, t);
+    } else {
+#pragma unroll
+        for(int k = 0; k < S; ++k) m.dQf[(size_t)k * m.n_faces + f] = v[k];
+    }
+}
+
+/* The MUSCL-Hancock half of calculate_flux (VorFace.cpp:670-838); false:
+ * nothing to solve (zero area, no active cell), dQ is zero */
+template <int D, int MODE>
+__device__ __forceinline__ bool face_problem(const sfx_dmesh& m, const sfx_solver_params& sp,
+                                             double dt, int f, int write_branch,
+                                             FaceProblem<D>& q) {
     using R = Rec<D>;
     constexpr int S = D + 2;
     constexpr bool REC = MODE != kFaceArrays;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if(f >= sfx_flux_faces(m) || failed(m.err)) return;
     const int n = m.n_cells, F = m.n_faces;
-    auto store_dQ = [&](const double* v) {
-        if(REC) {
-            double t[R::dq];
-#pragma unroll
-            for(int k = 0; k < R::dq; ++k) t[k] = k < S ? v[k] : 0.;
-            store_record<R::dq>(m.dQf + (size_t)f * R::dq, t);
-        } else {
-#pragma unroll
-            for(int k = 0; k < S; ++k) m.dQf[(size_t)k * F + f] = v[k];
-        }
-    };
     auto skip = [&]() {
         double z[S];
 #pragma unroll
         for(int k = 0; k < S; ++k) z[k] = 0.;
-        store_dQ(z);
+        store_dQ<D, REC>(m, f, z);
         if(write_branch) m.branch[f] = SFX_BRANCH_SKIPPED;
     };
-    FaceGeom<D> q;
+    FaceGeom<D> g;
     if(REC) {
         double h[R::fgeo];
 #pragma unroll
         for(int k = 0; k < R::fgeo; k += 4)
             load_record<4>(m.fgeo + (size_t)k * F + 4 * (size_t)f, h + k);
-        q.iL = __double2loint(h[0]);
-        q.iR = __double2hiint(h[0]);
-        q.A = h[1];
-        q.facL = h[2];
-        q.facR = h[3];
-        q.wL = h[4];
-        q.wR = h[5];
+        g.iL = __double2loint(h[0]);
+        g.iR = __double2hiint(h[0]);
+        g.A = h[1];
+        g.facL = h[2];
+        g.facR = h[3];
+        g.wL = h[4];
+        g.wR = h[5];
 #pragma unroll
         for(int l = 0; l < D; ++l) {
-            q.dL[l] = h[6 + l];
-            q.dR[l] = h[6 + D + l];
-            q.n[l] = h[6 + 2 * D + l];
+            g.dL[l] = h[6 + l];
+            g.dR[l] = h[6 + D + l];
+            g.n[l] = h[6 + 2 * D + l];
         }
     } else {
-        q.A = m.area[f];
-        q.iL = m.left[f];
-        q.iR = m.kind[f] == SFX_FACE_MIRROR ? -1 : m.right[f];
+        g.A = m.area[f];
+        g.iL = m.left[f];
+        g.iR = m.kind[f] == SFX_FACE_MIRROR ? -1 : m.right[f];
     }
-    const double A = q.A;
-    if(A == 0.) {
+    if(g.A == 0.) {
         skip();
-        return;
+        return false;
     }
-    const int iL = q.iL;
-    const bool has_right = q.iR >= 0;
-    const int iR = has_right ? q.iR : 0;
+    const int iL = g.iL;
+    const bool has_right = g.iR >= 0;
+    const int iR = has_right ? g.iR : 0;
     /* local time steps (VorFace.cpp:672-697): a face is computed when its
      * left cell is active, or (with a right cell) either cell is; its time
-     * step is the shorter of the two cells' steps */
+     * step is the shorter of the two cells' steps; the limits' timefac is that
+     * over the longer one (dt / dt with one global step) */
     double dtmax = dt;
-    if(MODE == kFaceMoving && m.local) {
+    if(MODE != kFaceRecords && m.local) {
         const bool aL = m.tstart[iL] == m.t_now;
         const bool aR = has_right && m.tstart[iR] == m.t_now;
         if(!aL && !aR) {
             skip();
-            return;
+            return false;
         }
         dt = sfx_realtime(m.t_total, m.tend[iL] - m.tstart[iL]);
         dtmax = dt;
@@ -1480,12 +1494,14 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
             dtmax = fmax(dtmax, dtR);
         }
     }
-    if(!REC) face_geom<D>(m, f, q);
-    double v[D];
+    if(!REC) face_geom<D>(m, f, g);
+    q.has_right = has_right;
 #pragma unroll
-    for(int l = 0; l < D; ++l)
-        v[l] = MODE == kFaceMoving && m.vel ? m.vel[(size_t)l * F + f] : 0.;
-    double WL[S], WR[S], WRrec[S], Wt[S];
+    for(int l = 0; l < D; ++l) {
+        q.n[l] = g.n[l];
+        q.v[l] = MODE != kFaceRecords && m.vel ? m.vel[(size_t)l * F + f] : 0.;
+    }
+    double WRrec[S], Wt[S];
     double QLm, QRm = 0.;
     auto load_state = [&](int i, double* W, double& Qm) {
         if(REC) {
@@ -1500,6 +1516,8 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
             Qm = m.Q[i];
         }
     };
+    double* WL = q.WL;
+    double* WR = q.WR;
     load_state(iL, WL, QLm);
 #pragma unroll
     for(int k = 0; k < S; ++k) {
@@ -1507,47 +1525,47 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
         WRrec[k] = 0.;
     }
     if(has_right) load_state(iR, WR, QRm);
-    if(MODE == kFaceMoving) {
+    if(MODE != kFaceRecords) {
 #pragma unroll
         for(int l = 0; l < D; ++l) {
-            WL[1 + l] = WL[1 + l] - v[l];
-            WR[1 + l] = WR[1 + l] - v[l];
+            WL[1 + l] = WL[1 + l] - q.v[l];
+            WR[1 + l] = WR[1 + l] - q.v[l];
         }
     }
     /* gradients of cell i, and dW/dt at its (boosted) state W */
-    auto load_slopes = [&](int i, const double* W, double (*g)[S], double* dW0) {
+    auto load_slopes = [&](int i, const double* W, double (*gr)[S], double* dW0) {
         if(REC) {
             double t[R::grec];
             load_record<R::grec>(m.grec + (size_t)i * R::grec, t);
 #pragma unroll
             for(int l = 0; l < D; ++l)
 #pragma unroll
-                for(int k = 0; k < S; ++k) g[l][k] = t[l * S + k];
+                for(int k = 0; k < S; ++k) gr[l][k] = t[l * S + k];
 #pragma unroll
             for(int k = 0; k < S; ++k) dW0[k] = t[D * S + k];
         } else {
 #pragma unroll
             for(int l = 0; l < D; ++l)
 #pragma unroll
-                for(int k = 0; k < S; ++k) g[l][k] = m.grad[((size_t)l * S + k) * n + i];
+                for(int k = 0; k < S; ++k) gr[l][k] = m.grad[((size_t)l * S + k) * n + i];
         }
-        if(MODE != kFaceRecords) time_derivative<D>(sp.gamma, W, g, dW0);
+        if(MODE != kFaceRecords) time_derivative<D>(sp.gamma, W, gr, dW0);
     };
     if(has_right) {
-        double g[D][S], dW0[S];
-        load_slopes(iR, WR, g, dW0);
+        double gr[D][S], dW0[S];
+        load_slopes(iR, WR, gr, dW0);
 #pragma unroll
         for(int k = 0; k < S; ++k) Wt[k] = WR[k];
-        predict_side<D>(dt, Wt, WR, WL, g, dW0, q.dR, true, q.wR);
+        predict_side<D>(dt, Wt, WR, WL, gr, dW0, g.dR, true, g.wR);
 #pragma unroll
         for(int k = 0; k < S; ++k) WRrec[k] = Wt[k];
     }
     {
-        double g[D][S], dW0[S];
-        load_slopes(iL, WL, g, dW0);
+        double gr[D][S], dW0[S];
+        load_slopes(iL, WL, gr, dW0);
 #pragma unroll
         for(int k = 0; k < S; ++k) Wt[k] = WL[k];
-        predict_side<D>(dt, Wt, WL, WR, g, dW0, q.dL, has_right, q.wL);
+        predict_side<D>(dt, Wt, WL, WR, gr, dW0, g.dL, has_right, g.wL);
     }
     if(WL[0] != 0.) {
 #pragma unroll
@@ -1557,32 +1575,29 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
 #pragma unroll
         for(int k = 0; k < S; ++k) WR[k] = WRrec[k];
     }
-    double flux[S];
-    int status = SFX_OK, code;
-    if(SOLVER == SFX_SOLVER_EXACT) {
-        double half[S];
-        ExactOut eo = exact_solve<D>(sp, WL, WR, q.n, !has_right, half);
-        status = eo.status;
-        code = eo.code;
-#pragma unroll
-        for(int l = 0; l < D; ++l) half[1 + l] = half[1 + l] + v[l];
-        exact_flux_from_half<D>(sp.gamma, half, v, q.n, flux);
-    } else {
-        code = hllc_flux<D>(sp, WL, WR, q.n, v, !has_right, flux);
-    }
+    double timefac = 1.;
+    if(MODE != kFaceRecords && has_right) timefac = dt / dtmax;
+    q.dtA = dt * g.A;
+    q.limL = g.facL * timefac * QLm;
+    q.limR = g.facR * timefac * QRm;
+    return true;
+}
+
+/* dt A flux with the over-flux limiter into the face's dQ; its branch code and
+ * status */
+template <int D, bool REC>
+__device__ __forceinline__ void face_dQ(const sfx_dmesh& m, int f, const double* flux,
+                                        double dtA, double limL, double limR, bool has_right,
+                                        int code, int status, int write_branch) {
+    constexpr int S = D + 2;
     double dQL[S], dQR[S];
 #pragma unroll
     for(int k = 0; k < S; ++k) {
-        dQL[k] = dt * A * flux[k];
-        dQR[k] = -dt * A * flux[k];
+        dQL[k] = dtA * flux[k];
+        dQR[k] = -dtA * flux[k];
     }
-    /* over-flux limiter (VorFace.cpp:837-866): timefac = dt / (the longer
-     * of the two cells' steps); dt / dt with one global step */
-    double timefac = 1.;
-    if(MODE == kFaceMoving && has_right) timefac = dt / dtmax;
-    const double areafac = q.facL * timefac;
-    if(dQL[0] > areafac * QLm) {
-        const double corfac = fabs(areafac * QLm / dQL[0]);
+    if(dQL[0] > limL) {
+        const double corfac = fabs(limL / dQL[0]);
 #pragma unroll
         for(int k = 0; k < S; ++k) dQL[k] = dQL[k] * corfac;
 #pragma unroll
@@ -1590,9 +1605,8 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
         code |= SFX_BRANCH_LIMIT_L;
     }
     if(has_right) {
-        const double areafacR = q.facR * timefac;
-        if(dQR[0] > areafacR * QRm) {
-            const double corfac = fabs(areafacR * QRm / dQR[0]);
+        if(dQR[0] > limR) {
+            const double corfac = fabs(limR / dQR[0]);
 #pragma unroll
             for(int k = 0; k < S; ++k) dQR[k] = dQR[k] * corfac;
 #pragma unroll
@@ -1600,10 +1614,205 @@ __global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp
             code |= SFX_BRANCH_LIMIT_R;
         }
     }
-    store_dQ(dQL);
+    store_dQ<D, REC>(m, f, dQL);
     if(write_branch) m.branch[f] = code;
     if(status == SFX_OK && flux[0] != flux[0]) status = SFX_ERR_NAN_FLUX;
     if(status != SFX_OK) report_face(m.err, f, status);
+}
+
+/* the exact solver's half state and flux in a face's frame */
+template <int D>
+__device__ __forceinline__ ExactOut exact_face(const sfx_solver_params& sp, double* WL,
+                                               double* WR, const double* n, const double* v,
+                                               bool has_right, double* flux) {
+    double half[D + 2];
+    const ExactOut eo = exact_solve<D>(sp, WL, WR, n, !has_right, half);
+#pragma unroll
+    for(int l = 0; l < D; ++l) half[1 + l] = half[1 + l] + v[l];
+    exact_flux_from_half<D>(sp.gamma, half, v, n, flux);
+    return eo;
+}
+
+/* one thread per face: HLLC, and both solvers on caller-owned arrays */
+template <int D, int SOLVER, int MODE>
+__global__ void __launch_bounds__(128) k_faces(sfx_dmesh m, sfx_solver_params sp,
+                                               double dt, int write_branch) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if(f >= sfx_flux_faces(m) || failed(m.err)) return;
+    FaceProblem<D> q;
+    if(!face_problem<D, MODE>(m, sp, dt, f, write_branch, q)) return;
+    double flux[D + 2];
+    int status = SFX_OK, code;
+    if(SOLVER == SFX_SOLVER_EXACT) {
+        const ExactOut eo = exact_face<D>(sp, q.WL, q.WR, q.n, q.v, q.has_right, flux);
+        status = eo.status;
+        code = eo.code;
+    } else {
+        code = hllc_flux<D>(sp, q.WL, q.WR, q.n, q.v, !q.has_right, flux);
+    }
+    face_dQ<D, MODE != kFaceArrays>(m, f, flux, q.dtA, q.limL, q.limR, q.has_right, code,
+                                    status, write_branch);
+}
+
+/* ------------------- exact solver: faces sorted by wave pattern -------------------
+ * The iteration's cost depends on the face: which side is a shock and which a
+ * rarefaction (different code on each side, and powers on a rarefaction), and
+ * whether f(0) lies under the cutoff (Newton alone, a few steps) or not (5% of
+ * a random field's faces; 2% then take Brent's method, about 30 evaluations).
+ * One thread per face ran 9.5 of 32 lanes.  So a block sorts its faces by
+ * wave pattern through shared memory and its threads solve them in that order;
+ * faces with f(0) above the cutoff go to a list that k_faces_listed solves,
+ * full warps of them (they would leave every block a warp of six running ten
+ * times as long as the others).  The keys are formed in FP32: they decide
+ * which thread solves a face and nothing else.  807,000 random-field faces in
+ * 3D: 735 -> 254 us and 86 us for the list's 5%; bound by FP64 latency (16 warps
+ * per SM at 128 registers).  The two rarefactions' powers interleaved, inline,
+ * for more independent operations: 297 us (registers and code). */
+constexpr int kExactBlock = 256, kKeys = 8, kKeyListed = 8, kKeyNone = 9;
+
+template <int D>
+__device__ __forceinline__ int wave_key(const sfx_solver_params& s, const FaceProblem<D>& q) {
+    const float rL = (float)q.WL[0], pL = (float)q.WL[D + 1];
+    const float rR = q.has_right ? (float)q.WR[0] : rL;
+    const float pR = q.has_right ? (float)q.WR[D + 1] : pL;
+    float vL = 0.f, vR = 0.f;
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        vL += (float)q.WL[1 + l] * (float)q.n[l];
+        vR += (float)q.WR[1 + l] * (float)q.n[l];
+    }
+    if(!q.has_right) vR = -vL;
+    const float g = (float)s.gamma, tdgm1 = (float)s.tdgm1, e = (float)s.gm1d2g;
+    const float aL = sqrtf(__fdividef(g * pL, rL)), aR = sqrtf(__fdividef(g * pR, rR));
+    const float dv = vR - vL;
+    const float f0 = dv - tdgm1 * (aL + aR);
+    if(!(f0 < 0.f)) return kKeys - 1; /* vacuum (or no number): no iteration */
+    if(f0 >= (float)s.cutoff) return kKeyListed;
+    const bool lowL = pL <= pR;
+    const float pmin = lowL ? pL : pR, pmax = lowL ? pR : pL;
+    /* f(p_min): the lower side contributes 0, the other one rarefies;
+     * f(p_max): the lower side is a shock, the other one contributes 0 */
+    const float fmin = tdgm1 * (lowL ? aR : aL) *
+                               (exp2f(e * __log2f(__fdividef(pmin, pmax))) - 1.f) +
+                       dv;
+    const float A = __fdividef((float)s.tdgp1, lowL ? rL : rR);
+    const float fmax = (pmax - pmin) * sqrtf(__fdividef(A, pmax + (float)s.gm1dgp1 * pmin)) + dv;
+    /* the guess: a linear one for similar pressures, otherwise with powers or
+     * square roots (ExactRiemannSolver.cpp:644-673) */
+    const float ppv = 0.5f * (pL + pR) - 0.125f * dv * (rL + rR) * (aL + aR);
+    const int linear = pmax <= 2.f * pmin && pmin <= ppv && ppv <= pmax;
+    if(fmin >= 0.f) return 0 + linear;
+    if(fmax <= 0.f) return 2 + linear;
+    return (lowL ? 4 : 5);
+}
+
+template <int D, int MODE>
+__global__ void __launch_bounds__(kExactBlock, 2)
+        k_faces_exact(sfx_dmesh m, sfx_solver_params sp, double dt, int write_branch, int list) {
+    constexpr int S = D + 2, NW = kExactBlock / 32;
+    constexpr bool MOVING = MODE == kFaceMoving;
+    __shared__ double sW[2 * S][kExactBlock], sn[D][kExactBlock];
+    __shared__ double sv[MOVING ? D : 1][kExactBlock]; /* one unused row when static */
+    __shared__ double sA[kExactBlock], sL[kExactBlock], sR[kExactBlock];
+    __shared__ int sf[kExactBlock]; /* face, bit 31: no right cell */
+    __shared__ int sbase[kKeys][NW];
+    __shared__ int stotal;
+    const int f = blockIdx.x * kExactBlock + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    FaceProblem<D> q;
+    int key = kKeyNone;
+    if(f < sfx_flux_faces(m) && !failed(m.err) &&
+       face_problem<D, MODE>(m, sp, dt, f, write_branch, q))
+        key = wave_key<D>(sp, q);
+    if(!list && key == kKeyListed) key = kKeys - 2;
+    /* the list: one atomic per warp; each face enters it at most once a step */
+    const unsigned listed = __ballot_sync(0xffffffffu, key == kKeyListed);
+    if(listed) {
+        int at = 0;
+        if(lane == 0) at = atomicAdd(m.listed_n, __popc(listed));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(listed & ((1u << lane) - 1u));
+        if(key == kKeyListed) m.listed[at] = f;
+    }
+    /* counting sort by key */
+    unsigned mine = 0;
+#pragma unroll
+    for(int c = 0; c < kKeys; ++c) {
+        const unsigned b = __ballot_sync(0xffffffffu, key == c);
+        if(lane == c) sbase[c][warp] = __popc(b);
+        if(key == c) mine = b;
+    }
+    __syncthreads();
+    if(warp == 0) {
+        /* exclusive scan in (key, warp) order, two entries per lane */
+        static_assert(kKeys * NW == 64, "two counts per lane");
+        int* t = &sbase[0][0];
+        const int a = t[2 * lane], b = t[2 * lane + 1];
+        int x = a + b;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if(lane >= o) x += y;
+        }
+        t[2 * lane] = x - a - b;
+        t[2 * lane + 1] = x - b;
+        if(lane == 31) stotal = x;
+    }
+    __syncthreads();
+    if(key < kKeys) {
+        const int at = sbase[key][warp] + __popc(mine & ((1u << lane) - 1u));
+#pragma unroll
+        for(int k = 0; k < S; ++k) {
+            sW[k][at] = q.WL[k];
+            sW[S + k][at] = q.WR[k];
+        }
+#pragma unroll
+        for(int l = 0; l < D; ++l) {
+            sn[l][at] = q.n[l];
+            if(MOVING) sv[MOVING ? l : 0][at] = q.v[l];
+        }
+        sA[at] = q.dtA;
+        sL[at] = q.limL;
+        sR[at] = q.limR;
+        sf[at] = f | (q.has_right ? 0 : (int)kRightBit);
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if(t >= stotal) return;
+    const bool has_right = sf[t] >= 0;
+    double WL[S], WR[S], n[D], v[D], flux[S];
+#pragma unroll
+    for(int k = 0; k < S; ++k) {
+        WL[k] = sW[k][t];
+        WR[k] = sW[S + k][t];
+    }
+#pragma unroll
+    for(int l = 0; l < D; ++l) {
+        n[l] = sn[l][t];
+        v[l] = MOVING ? sv[MOVING ? l : 0][t] : 0.;
+    }
+    const ExactOut eo = exact_face<D>(sp, WL, WR, n, v, has_right, flux);
+    face_dQ<D, true>(m, (int)((unsigned)sf[t] & ~kRightBit), flux, sA[t], sL[t], sR[t], has_right,
+                     eo.code, eo.status, write_branch);
+}
+
+/* the listed faces, one per thread; nothing to do when there are none */
+constexpr int kListedBlock = 128, kListedBlocks = 4 * 148;
+
+template <int D, int MODE>
+__global__ void __launch_bounds__(kListedBlock)
+        k_faces_listed(sfx_dmesh m, sfx_solver_params sp, double dt, int write_branch) {
+    const int count = *(volatile const int*)m.listed_n;
+    for(int j = blockIdx.x * kListedBlock + threadIdx.x; j < count;
+        j += kListedBlocks * kListedBlock) {
+        if(failed(m.err)) return;
+        const int f = m.listed[j];
+        FaceProblem<D> q;
+        if(!face_problem<D, MODE>(m, sp, dt, f, write_branch, q)) continue;
+        double flux[D + 2];
+        const ExactOut eo = exact_face<D>(sp, q.WL, q.WR, q.n, q.v, q.has_right, flux);
+        face_dQ<D, true>(m, f, flux, q.dtA, q.limL, q.limR, q.has_right, eo.code, eo.status,
+                         write_branch);
+    }
 }
 
 /* ------------------------------ update ------------------------------ */
@@ -1761,40 +1970,38 @@ __global__ void k_init_Q(sfx_dmesh m, double gamma, int kind, const double* rows
 constexpr int kTotBlocks = 1024;
 constexpr int kTotThreads = 256;
 
-/* sums of the fields over cells [0, count) of Q [S][n] */
-__global__ void k_totals_partial(const double* Q, int n, int count, int S, double* part) {
+/* sum of field blockIdx.y over this block's cells of [0, count) of Q [S][n] */
+__global__ void k_totals_partial(const double* Q, int n, int count, double* part) {
     __shared__ double sh[kTotThreads];
     const int per = (count + kTotBlocks - 1) / kTotBlocks;
     const int b0 = blockIdx.x * per;
     const int b1 = min(count, b0 + per);
-    for(int k = 0; k < S; ++k) {
-        double acc = 0.;
-        for(int i = b0 + threadIdx.x; i < b1; i += kTotThreads) acc = acc + Q[(size_t)k * n + i];
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for(int w = kTotThreads / 2; w > 0; w >>= 1) {
-            if(threadIdx.x < w) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + w];
-            __syncthreads();
-        }
-        if(threadIdx.x == 0) part[k * kTotBlocks + blockIdx.x] = sh[0];
+    const int k = blockIdx.y;
+    double acc = 0.;
+    for(int i = b0 + threadIdx.x; i < b1; i += kTotThreads) acc = acc + Q[(size_t)k * n + i];
+    sh[threadIdx.x] = acc;
+    __syncthreads();
+    for(int w = kTotThreads / 2; w > 0; w >>= 1) {
+        if(threadIdx.x < w) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + w];
         __syncthreads();
     }
+    if(threadIdx.x == 0) part[k * kTotBlocks + blockIdx.x] = sh[0];
 }
 
+/* one block per field */
 __global__ void k_totals_final(double* part, int S, const sfx_dev_error* err) {
     __shared__ double sh[kTotBlocks];
-    for(int k = 0; k < S; ++k) {
-        for(int t = threadIdx.x; t < kTotBlocks; t += blockDim.x) sh[t] = part[k * kTotBlocks + t];
-        __syncthreads();
-        for(int w = kTotBlocks / 2; w > 0; w >>= 1) {
-            for(int t = threadIdx.x; t < w; t += blockDim.x) sh[t] = sh[t] + sh[t + w];
-            __syncthreads();
-        }
-        if(threadIdx.x == 0) part[S * kTotBlocks + k] = sh[0];
+    const int k = blockIdx.x;
+    for(int t = threadIdx.x; t < kTotBlocks; t += blockDim.x) sh[t] = part[k * kTotBlocks + t];
+    __syncthreads();
+    for(int w = kTotBlocks / 2; w > 0; w >>= 1) {
+        for(int t = threadIdx.x; t < w; t += blockDim.x) sh[t] = sh[t] + sh[t + w];
         __syncthreads();
     }
+    if(threadIdx.x != 0) return;
+    part[S * kTotBlocks + k] = sh[0];
     /* the error record beside them: one copy to the host for both */
-    if(threadIdx.x == 0) {
+    if(k == 0) {
         part[S * kTotBlocks + S] = __longlong_as_double((long long)err->face_key);
         part[S * kTotBlocks + S + 1] = __longlong_as_double((long long)err->cell_key);
     }
@@ -2210,16 +2417,37 @@ int sfx_fp64_gradients(const sfx_dmesh* m, const sfx_solver_params* sp, void* st
     return cuda_status(cudaGetLastError());
 }
 
-template <int D, int SOLVER>
-static void launch_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
-                         int write_branch, int nf, cudaStream_t s) {
+template <int D, int MODE>
+static int launch_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
+                        int write_branch, int nf, cudaStream_t s) {
     const int B = 128, G = grid_for(nf, B);
-    if(!m->ws)
-        k_faces<D, SOLVER, kFaceArrays><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
-    else if(m->vel || m->local)
-        k_faces<D, SOLVER, kFaceMoving><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
-    else
-        k_faces<D, SOLVER, kFaceRecords><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+    if(sp->kind != SFX_SOLVER_EXACT) {
+        k_faces<D, SFX_SOLVER_HLLC, MODE><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+        return 1;
+    }
+    if constexpr(MODE == kFaceArrays) {
+        k_faces<D, SFX_SOLVER_EXACT, MODE><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
+        return 1;
+    } else {
+        /* one wave of blocks waits for its longest face whichever way it is
+         * sorted, and a second launch would add to that: the list from two
+         * blocks on every SM */
+        const int list = nf > 2 * 148 * kExactBlock;
+        k_faces_exact<D, MODE><<<grid_for(nf, kExactBlock), kExactBlock, 0, s>>>(
+                *m, *sp, dt, write_branch, list);
+        if(!list) return 1;
+        k_faces_listed<D, MODE>
+                <<<kListedBlocks, kListedBlock, 0, s>>>(*m, *sp, dt, write_branch);
+        return 2;
+    }
+}
+
+template <int D>
+static int launch_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
+                        int write_branch, int nf, cudaStream_t s) {
+    if(!m->ws) return launch_faces<D, kFaceArrays>(m, sp, dt, write_branch, nf, s);
+    if(m->vel || m->local) return launch_faces<D, kFaceMoving>(m, sp, dt, write_branch, nf, s);
+    return launch_faces<D, kFaceRecords>(m, sp, dt, write_branch, nf, s);
 }
 
 int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
@@ -2227,18 +2455,8 @@ int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
     const int nf = sfx_flux_faces(*m);
     if(nf == 0) return SFX_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if(m->dim == 3) {
-        if(sp->kind == SFX_SOLVER_EXACT)
-            launch_faces<3, SFX_SOLVER_EXACT>(m, sp, dt, write_branch, nf, s);
-        else
-            launch_faces<3, SFX_SOLVER_HLLC>(m, sp, dt, write_branch, nf, s);
-    } else {
-        if(sp->kind == SFX_SOLVER_EXACT)
-            launch_faces<2, SFX_SOLVER_EXACT>(m, sp, dt, write_branch, nf, s);
-        else
-            launch_faces<2, SFX_SOLVER_HLLC>(m, sp, dt, write_branch, nf, s);
-    }
-    sfx_count_launches(1);
+    sfx_count_launches(m->dim == 3 ? launch_faces<3>(m, sp, dt, write_branch, nf, s)
+                                   : launch_faces<2>(m, sp, dt, write_branch, nf, s));
     return cuda_status(cudaGetLastError());
 }
 
@@ -2270,9 +2488,10 @@ int sfx_fp64_init_Q(const sfx_dmesh* m, const sfx_solver_params* sp, const doubl
 
 int sfx_fp64_totals(const sfx_dmesh* m, double* host_out, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    k_totals_partial<<<kTotBlocks, kTotThreads, 0, s>>>(m->Q, m->n_cells, sfx_update_cells(*m),
-                                                         m->S, m->totals_scratch);
-    k_totals_final<<<1, 256, 0, s>>>(m->totals_scratch, m->S, m->err);
+    const dim3 grid(kTotBlocks, m->S);
+    k_totals_partial<<<grid, kTotThreads, 0, s>>>(m->Q, m->n_cells, sfx_update_cells(*m),
+                                                  m->totals_scratch);
+    k_totals_final<<<m->S, 256, 0, s>>>(m->totals_scratch, m->S, m->err);
     sfx_count_launches(2);
     cudaError_t e = cudaMemcpyAsync(host_out, m->totals_scratch + (size_t)m->S * kTotBlocks,
                                     sizeof(double) * (m->S + 2), cudaMemcpyDeviceToHost, s);

@@ -61,6 +61,10 @@ struct sfx_dmesh {
     double* grec;
     double* ggeo;
     double* fgeo;
+    /* plain-FP64 exact solver: the faces solved by the second launch of a step
+     * (room for every face) and their number */
+    int32_t* listed;
+    int32_t* listed_n;
     int32_t gshare; /* every local face's right position equals its right cell's */
     /* one part of a mesh split over several devices (plain FP64): gradients
      * of cells [0, r_grad), fluxes of faces [0, r_flux), update of cells

@@ -157,11 +157,11 @@ SFX_HD double sfx_powq_exp_tab(int i) {
 }
 
 /* ln x as a pair, absolute error below 2^-72 + 2^-100 |ln x|; 0: x is not a
- * positive normal number */
+ * positive normal number (the pair is then of no use).  No branches, here and
+ * in sfx_powq_exp, so that two calls side by side overlap. */
 SFX_HD int sfx_powq_log(double x, double* rh, double* rl) {
     const uint64_t u = sfx_d2u(x);
     const uint64_t ex = u >> 52; /* includes the sign bit */
-    if(ex - 1 >= 0x7fe) return 0;
     const double e = (double)((int)ex - 1023);
     const double m = sfx_u2d((u & 0x000fffffffffffffull) | 0x3ff0000000000000ull);
     const int j = 3 * (int)((u >> 46) & 63);
@@ -193,13 +193,15 @@ SFX_HD int sfx_powq_log(double x, double* rh, double* rl) {
                       sfx_fma(e, 0x1.ef35793c76730p-45, sfx_powq_log_tab(j + 2)) +
                       ((e1 + e2) + e3);
     sfx_two_sum(h, lo, rh, rl);
-    return 1;
+    return ex - 1 < 0x7fe;
 }
 
-/* exp(th + tl), |th| < 22, rounded; 0: a rounding boundary lies too near */
+/* exp(th + tl), rounded; 0: |th| >= 22 or NaN, or a rounding boundary lies too
+ * near */
 SFX_HD int sfx_powq_exp(double th, double tl, double* out) {
     const double kd = (th * 0x1.71547652b82fep+5 + 0x1.8p52) - 0x1.8p52;
-    const int k = (int)kd;
+    const int in_range = (th < 0.0 ? -th : th) < 22.0; /* 0 for a NaN */
+    const int k = in_range ? (int)kd : 0;
     const double a = th - kd * 0x1.62e42fefa3800p-6; /* exact */
     const double mh = kd * 0x1.ef35793c76730p-50;
     const double me = sfx_fma(kd, 0x1.ef35793c76730p-50, -mh);
@@ -228,7 +230,7 @@ SFX_HD int sfx_powq_exp(double th, double tl, double* out) {
     const double err = h * 0x1p-68;
     const double up = h + (l + err), dn = h + (l - err);
     *out = up * sfx_u2d((uint64_t)((k >> 5) + 1023) << 52);
-    return up == dn;
+    return in_range & (up == dn);
 }
 
 SFX_HD double sfx_powq(double x, double y) {
@@ -236,8 +238,7 @@ SFX_HD double sfx_powq(double x, double y) {
     if(sfx_powq_log(x, &lh, &ll)) {
         const double th = y * lh;
         const double tl = sfx_fma(y, lh, -th) + y * ll;
-        /* false for a NaN too */
-        if((th < 0.0 ? -th : th) < 22.0 && sfx_powq_exp(th, tl, &r)) return r;
+        if(sfx_powq_exp(th, tl, &r)) return r;
     }
     return SFX_POWQ_RARE(x, y);
 }
