@@ -511,8 +511,10 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src) {
  * kGradStages faces ahead (lane k of a cell copies 16 bytes of the geometry
  * and one variable): no registers hold loads in flight.  Both loops divided
  * per face before, the first one in a kernel of its own that wrote 128 bytes
- * per face: 220 -> 88 us on 65,537 cells in 3D, 104 -> 66 us on 150,001 in 2D
- * (109 and 68 us without the ring).  Cells sorted by face count so that a
+ * per face: 220 -> 83 us on 65,537 cells in 3D, 104 -> 63 us on 150,001 in 2D
+ * (109 and 68 us without the ring; 88 and 66 without the kept midpoints).  96
+ * registers in 3D: 102 left four blocks per SM instead of five (87 us), 80 spill
+ * (86).  Two faces per ring stage: 85.  Cells sorted by face count so that a
  * warp's lanes run equally long: 83 us, but the update in that order lost
  * more than that to a lower L1 hit rate. */
 constexpr int kGradBlock = 128, kGradStages = 4;
@@ -528,11 +530,15 @@ struct GradSlot {
 };
 
 template <int D>
-__global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double gamma) {
+__global__ void __launch_bounds__(kGradBlock, D == 3 ? 5 : 6) k_grad_cells(sfx_dmesh m, double gamma) {
     using R = Rec<D>;
     constexpr int S = R::S;
     static_assert(sizeof(GradSlot<D>) == (D == 3 ? 144 : 112), "slot layout");
     __shared__ __align__(16) GradSlot<D> ring[kGradBlock / 32][kGradStages][R::cells];
+    /* the first kKept faces' midpoints, for the limiter's loop (one double of
+     * padding: a warp's cells on different banks) */
+    constexpr int kKept = D == 3 ? 24 : 12;
+    __shared__ double kept[kGradBlock / 32][R::cells][kKept * D + 1];
     if(blockIdx.x == 0 && threadIdx.x == 0) *m.listed_n = 0; /* a new step's list */
     const int lane = threadIdx.x & 31;
     const int slot = lane / S, k = lane - slot * S;
@@ -557,13 +563,15 @@ __global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double g
     int2 next = make_int2(0, -1);
     if(count > 0) next = __ldg(m.ent + end - 1);
     GradSlot<D>(*mine)[R::cells] = ring[threadIdx.x >> 5];
+    double* mids = kept[threadIdx.x >> 5][slot < R::cells ? slot : 0];
     auto fetch = [&](int it) {
         if(it < count) {
             const int2 v = next;
             if(it + 1 < count) next = __ldg(m.ent + end - 2 - it);
             GradSlot<D>& q = mine[it % kGradStages][slot];
-            copy_async<16>(&q.geo[k],
-                           m.ggeo + (size_t)((unsigned)v.x & ~kRightBit) * R::ggeo + 2 * k);
+            const double* rec = m.ggeo + (size_t)((unsigned)v.x & ~kRightBit) * R::ggeo;
+            copy_async<16>(&q.geo[k], rec + 2 * k);
+            if(k < D && it < kKept) copy_async<8>(mids + it * D + k, rec + (D == 3 ? 9 : 8) + k);
             copy_async<8>(&q.W[k], m.ws + (size_t)(v.y < 0 ? ic : v.y) * R::ws + k);
             if(k == 0) q.ent = v;
         }
@@ -627,29 +635,28 @@ __global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double g
     }
     const double a = Wmax - W, b = Wmin - W;
     /* the offsets' projections on the gradient: the extremes decide the limiter */
-    auto offset = [&](int j) {
-        const unsigned f = (unsigned)__ldg(m.idx + j) & ~kRightBit;
-        const double* p = m.ggeo + (size_t)f * R::ggeo;
+    auto offset = [&](int it) {
         double d[D];
-        if(D == 3) {
-            double t[4];
-            load_record<4>(p + 8, t);
+        if(it < kKept) {
 #pragma unroll
-            for(int l = 0; l < D; ++l) d[l] = t[(l + 1) & 3] - cen[l];
+            for(int l = 0; l < D; ++l) d[l] = mids[it * D + l] - cen[l];
         } else {
-            const double2 t = __ldg(reinterpret_cast<const double2*>(p + 8));
-            d[0] = t.x - cen[0];
-            d[1] = t.y - cen[1];
+            const unsigned f = (unsigned)__ldg(m.idx + end - 1 - it) & ~kRightBit;
+            const double* rec = m.ggeo + (size_t)f * R::ggeo + (D == 3 ? 9 : 8);
+#pragma unroll
+            for(int l = 0; l < D; ++l) d[l] = __ldg(rec + l) - cen[l];
         }
         double dp = delta[0] * d[0] + delta[1] * d[1];
         if(D == 3) dp = dp + delta[D - 1] * d[D - 1];
         return dp;
     };
+    /* every lane's copies have landed */
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
     double dmax = 0., dmin = 0.;
     int first = 0;
-#pragma unroll 4
-    for(int j = end - 1; j >= beg; --j) {
-        const double dp = offset(j);
+    for(int it = 0; it < count; ++it) {
+        const double dp = offset(it);
         if(dp > dmax) dmax = dp;
         if(dp < dmin) dmin = dp;
         if(first == 0) first = dp > 0. ? 1 : (dp < 0. ? -1 : 0);
@@ -658,8 +665,8 @@ __global__ void __launch_bounds__(kGradBlock) k_grad_cells(sfx_dmesh m, double g
     if(plain && dmax < 0x1p300 && dmin > -0x1p300) {
         alpha = sfx_limiter_min(a, b, dmax, dmin, first);
     } else {
-        for(int j = end - 1; j >= beg; --j) {
-            const double dp = offset(j);
+        for(int it = 0; it < count; ++it) {
+            const double dp = offset(it);
             /* a face of zero area (NaN offset) is skipped; other NaNs never
              * compare below alpha */
             const double mx = sfx_limiter_ratio(a, b, dp);

@@ -621,10 +621,9 @@ __device__ __forceinline__ void sgrad_body(const sfx_dmesh& m, const float gamma
     float alpha[S];
 #pragma unroll
     for(int k = 0; k < S; ++k) {
-        const float up = (Wmax[k] - W[k]) / pmax[k], dn = (Wmin[k] - W[k]) / pmin[k];
         alpha[k] = 1.f;
-        if(pmax[k] > 0.f) alpha[k] = fminf(alpha[k], up);
-        if(pmin[k] < 0.f) alpha[k] = fminf(alpha[k], dn);
+        if(pmax[k] > 0.f) alpha[k] = fminf(alpha[k], (Wmax[k] - W[k]) * rcp32(pmax[k]));
+        if(pmin[k] < 0.f) alpha[k] = fminf(alpha[k], (Wmin[k] - W[k]) * rcp32(pmin[k]));
         alpha[k] = seg_min<LPC>(alpha[k]);
     }
     if(!live) return;
