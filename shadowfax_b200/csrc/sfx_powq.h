@@ -169,30 +169,26 @@ SFX_HD int sfx_powq_log(double x, double* rh, double* rl) {
     const double ph = m * c;
     const double pl = sfx_fma(m, c, -ph);
     double r, s; /* r + s = m c - 1 (ph - 1 is exact) */
-    sfx_two_sum(ph - 1.0, pl, &r, &s);
-    /* r^3/3 - ... + r^11/11 */
-    double q = 1.0 / 11.0;
-    q = sfx_fma(q, r, -1.0 / 10.0);
-    q = sfx_fma(q, r, 1.0 / 9.0);
-    q = sfx_fma(q, r, -1.0 / 8.0);
-    q = sfx_fma(q, r, 1.0 / 7.0);
-    q = sfx_fma(q, r, -1.0 / 6.0);
-    q = sfx_fma(q, r, 1.0 / 5.0);
-    q = sfx_fma(q, r, -1.0 / 4.0);
-    q = sfx_fma(q, r, 1.0 / 3.0);
+    sfx_fast_two_sum(ph - 1.0, pl, &r, &s);
+    /* (r^3/3 - ... + r^11/11) / r^3 by pairs (Estrin): a chain of four */
+    const double r2 = r * r, r4 = r2 * r2;
+    const double q0 = sfx_fma(r, -1.0 / 4.0, 1.0 / 3.0), q2 = sfx_fma(r, -1.0 / 6.0, 1.0 / 5.0);
+    const double q4 = sfx_fma(r, -1.0 / 8.0, 1.0 / 7.0), q6 = sfx_fma(r, -1.0 / 10.0, 1.0 / 9.0);
+    const double q = sfx_fma(r4 * r4, 1.0 / 11.0,
+                             sfx_fma(r4, sfx_fma(r2, q6, q4), sfx_fma(r2, q2, q0)));
     const double hr = -0.5 * r;
     const double qh = hr * r;
     const double ql = sfx_fma(hr, r, -qh);
-    const double r3 = r * (r * r);
+    const double r3 = r * r2;
     /* the large parts exactly: e ln2_hi (42 significant bits) - ln c + r - r^2/2 */
     double h, e1, e2, e3;
-    sfx_two_sum(e * 0x1.62e42fefa3800p-1, sfx_powq_log_tab(j + 1), &h, &e1);
+    sfx_fast_two_sum(e * 0x1.62e42fefa3800p-1, sfx_powq_log_tab(j + 1), &h, &e1);
     sfx_two_sum(h, r, &h, &e2);
     sfx_two_sum(h, qh, &h, &e3);
     const double lo = sfx_fma(q, r3, ql) + sfx_fma(-r, s, s) +
                       sfx_fma(e, 0x1.ef35793c76730p-45, sfx_powq_log_tab(j + 2)) +
                       ((e1 + e2) + e3);
-    sfx_two_sum(h, lo, rh, rl);
+    sfx_fast_two_sum(h, lo, rh, rl); /* |lo| < 2^-21: off by 2^-75 where |h| is smaller */
     return ex - 1 < 0x7fe;
 }
 
@@ -206,15 +202,12 @@ SFX_HD int sfx_powq_exp(double th, double tl, double* out) {
     const double mh = kd * 0x1.ef35793c76730p-50;
     const double me = sfx_fma(kd, 0x1.ef35793c76730p-50, -mh);
     double r, s;
-    sfx_two_sum(a, -mh, &r, &s);
-    sfx_two_sum(r, s + (tl - me), &r, &s); /* tl is up to an ulp of th, not of r */
-    double q = 1.0 / 40320.0;
-    q = sfx_fma(q, r, 1.0 / 5040.0);
-    q = sfx_fma(q, r, 1.0 / 720.0);
-    q = sfx_fma(q, r, 1.0 / 120.0);
-    q = sfx_fma(q, r, 1.0 / 24.0);
-    q = sfx_fma(q, r, 1.0 / 6.0);
+    sfx_fast_two_sum(a, -mh, &r, &s); /* |mh| < 2^-39: off by 2^-92 where |a| is smaller */
+    sfx_fast_two_sum(r, s + (tl - me), &r, &s); /* tl is up to an ulp of th, not of r */
     const double r2 = r * r;
+    const double q = sfx_fma(r2 * r2, sfx_fma(r, 1.0 / 40320.0, 1.0 / 5040.0),
+                             sfx_fma(r2, sfx_fma(r, 1.0 / 720.0, 1.0 / 120.0),
+                                     sfx_fma(r, 1.0 / 24.0, 1.0 / 6.0)));
     const double r2l = sfx_fma(r, r, -r2);
     /* exp(r + s) - 1 */
     double eh, el;
