@@ -419,7 +419,7 @@ int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
     }
     if(precision == SFX_PREC_SPLIT) {
         /* fg, fr, an, dq, queue; cw, cg, cx, self table */
-        bytes += F * (32 + 4 * (dim == 3 ? 16 : 12) + 8 * dim + 32) + 4 * slowq_capacity(F) + 4;
+        bytes += F * (32 + 4 * 12 + 8 * dim + 32) + 4 * slowq_capacity(F) + 4;
         bytes += n * (32 + 16 * (sfx_split_grad_vec4((int)dim) + sfx_split_dwdt_vec4((int)dim)) +
                       16) + 256;
     }
@@ -671,7 +671,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
             return SFX_ERR_UNSUPPORTED; /* the split pass is for static meshes */
         }
         A(&d.fg, 2 * F);
-        A(&d.fr, (size_t)(dim == 3 ? 16 : 12) * F);
+        A(&d.fr, 12 * F);
         A(&d.cw, 2 * n);
         A(&d.cg, (size_t)sfx_split_grad_vec4(dim) * n);
         A(&d.cdw, (size_t)sfx_split_dwdt_vec4(dim) * n);

@@ -78,7 +78,7 @@ struct sfx_dmesh {
      *     {r1, |r|, 0, 0}) with c = midpoint - (x_L + x_R)/2 and
      *     r = x_L - x_R (right generator at its image/mirror position),
      *     computed in FP64 and rounded once;
-     * fr [12 F] (2D) or [16 F] (3D): the face's cells and flux geometry (FaceRec,
+     * fr [12 F]: the face's cells and flux geometry (FaceRec,
      *     sfx_split.cu), formed in FP64 and rounded once;
      * cw [2n] float4 cell record {rho, v.., p | Q.m, total area ..};
      * cg [G*n] float4 gradients (G = 4 in 3D, 2 in 2D: 64 / 32 bytes, so a

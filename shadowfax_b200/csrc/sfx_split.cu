@@ -16,8 +16,8 @@
  * no FP32 subtraction of nearby absolute positions happens per step.
  *
  * Memory layout: a 32-byte cell record, a 64-byte (2D 32) gradient record, a
- * 32-byte gradient-geometry record and a 64-byte (2D 48) flux record per face,
- * each gather one or two 32-byte loads (sfx_wide.h).  No floating-point atomics: each cell sums its own
+ * 32-byte gradient-geometry record and a 48-byte flux record per face, each
+ * gather one or two 32-byte loads (sfx_wide.h).  No floating-point atomics: each cell sums its own
  * faces in ascending face order in FP64, so reruns are bitwise identical and
  * the face flux leaving one cell enters the other exactly.
  */
@@ -202,45 +202,48 @@ __device__ __forceinline__ void geom(const float4* __restrict__ fg, int f, float
 }
 
 /* What a face's flux needs of the mesh, formed in FP64 at upload: {left,
- * right or -1, A, |d_L| / |c_LR|, |d_R| / |c_LR|, d_L, d_R, n} (d = midpoint -
- * centroid, c_LR the centroids' difference) and, in 3D, A over each cell's
- * total area.  Consecutive threads read consecutive faces, so the record lies
- * in planes: [F] 8 floats, then [F] 8 floats (3D) or 4 (2D). */
+ * right or -1, A, |d_L| / |c_LR|, |d_R| / |c_LR|, d_L, d_R} (d = midpoint -
+ * centroid, c_LR the centroids' difference) and in 2D the normal; in 3D the
+ * normal comes from the FP64 area vector, which the pressure force reads
+ * anyway (a record with it and with A over each cell's total area is 16 bytes
+ * longer).  Consecutive threads read consecutive faces, so the record lies in
+ * planes: [F] 8 floats, then [F] 4 floats. */
 template <int D>
 struct FaceRec {
-    static constexpr int words = D == 3 ? 16 : 12;
+    static constexpr int words = 12;
     int L, R;
-    float A, wL, wR, dL[D], dR[D], n[D], facL, facR;
+    float A, wL, wR, dL[D], dR[D];
+    float n[D];
     /* float k of face f */
     static __device__ __forceinline__ size_t at(int F, int f, int k) {
-        return k < 8 ? (size_t)8 * f + k : (size_t)8 * F + (size_t)(words - 8) * f + (k - 8);
+        return k < 8 ? (size_t)8 * f + k : (size_t)8 * F + (size_t)4 * f + (k - 8);
     }
     __device__ __forceinline__ void load(const sfx_dmesh& m, int f) {
-        float v[16];
+        float v[words];
+        double an[D];
         sfx_load32(m.fr + at(m.n_faces, f, 0), v);
-        if constexpr(D == 3) {
-            sfx_load32(m.fr + at(m.n_faces, f, 8), v + 8);
-        } else {
-            const float4 t = __ldg((const float4*)(m.fr + at(m.n_faces, f, 8)));
-            v[8] = t.x;
-            v[9] = t.y;
-            v[10] = t.z;
-            v[11] = t.w;
+        const float4 t = __ldg((const float4*)(m.fr + at(m.n_faces, f, 8)));
+        if(D == 3) {
+#pragma unroll
+            for(int l = 0; l < D; ++l) an[l] = __ldg(m.an + (size_t)l * m.n_faces + f);
         }
+        v[8] = t.x;
+        v[9] = t.y;
+        v[10] = t.z;
+        v[11] = t.w;
         L = __float_as_int(v[0]);
         R = __float_as_int(v[1]);
         A = v[2];
         wL = v[3];
         wR = v[4];
+        /* one Newton step: the normal's length takes the reciprocal's error */
+        float iA = D == 3 ? rcp32(A) : 0.f;
+        iA = fmaf(fmaf(-A, iA, 1.f), iA, iA);
 #pragma unroll
         for(int l = 0; l < D; ++l) {
             dL[l] = v[5 + l];
             dR[l] = v[5 + D + l];
-            n[l] = v[5 + 2 * D + l];
-        }
-        if(D == 3) {
-            facL = v[14];
-            facR = v[15];
+            n[l] = D == 3 ? (float)an[l] * iA : v[5 + 2 * D + l < words ? 5 + 2 * D + l : 0];
         }
     }
 };
@@ -296,14 +299,9 @@ __global__ void k_prep_faces(sfx_dmesh m) {
     for(int l = 0; l < D; ++l) {
         v[5 + l] = (float)dL[l];
         v[5 + D + l] = (float)dR[l];
-        v[5 + 2 * D + l] = (float)(-r[l] / rn64);
+        if(D == 2) v[5 + 2 * D + l < FaceRec<D>::words ? 5 + 2 * D + l : 0] = (float)(-r[l] / rn64);
     }
-    if(D == 3) {
-        v[FaceRec<D>::words - 2] = (float)(m.area[f] / m.tarea[L]);
-        v[FaceRec<D>::words - 1] = R >= 0 ? (float)(m.area[f] / m.tarea[R]) : 0.f;
-    } else {
-        v[11] = 0.f;
-    }
+    v[FaceRec<D>::words - 1] = 0.f;
     for(int k = 0; k < FaceRec<D>::words; ++k) m.fr[FaceRec<D>::at(F, f, k)] = v[k];
 }
 
@@ -1539,7 +1537,7 @@ __device__ __forceinline__ bool face_work(const sfx_dmesh& m, const float gamma,
         w.v[l] = MOVING ? (float)__ldg(m.vel + (size_t)l * m.n_faces + f) : 0.f;
         if(MOVING) w.WL[1 + l] -= w.v[l];
     }
-    w.limL = (D == 3 ? q.facL : w.A * rcp32(cL.tarea)) * timefac * cL.Qm;
+    w.limL = w.A * rcp32(cL.tarea) * timefac * cL.Qm;
     w.limR = 0.f;
     if(!w.mirror) {
         const Cell<D> cR = load_cell<D>(m.cw, iR);
@@ -1549,7 +1547,7 @@ __device__ __forceinline__ bool face_work(const sfx_dmesh& m, const float gamma,
 #pragma unroll
             for(int l = 0; l < D; ++l) w.WR[1 + l] -= w.v[l];
         }
-        w.limR = (D == 3 ? q.facR : w.A * rcp32(cR.tarea)) * timefac * cR.Qm;
+        w.limR = w.A * rcp32(cR.tarea) * timefac * cR.Qm;
         float gR[D][S], dWR[S];
         load_grad<D, STORED>(m.cg, m.cdw, iR, gamma, w.WR, gR, dWR, moving);
 #pragma unroll
