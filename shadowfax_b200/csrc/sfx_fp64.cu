@@ -9,7 +9,7 @@
  * glibc's and CUDA's pow differ in the last bit; it is evaluated by sfx_powq
  * (sfx_powq.h).
  *
- * Kernels (one step = three launches):
+ * Kernels (one step = three launches, four with the exact solver's face list):
  *   k_grad_cells one thread per cell and variable: VorCell::estimate_gradient
  *                (src/VorCell.cpp:464-530); k_gradients, one thread per
  *                cell, for meshes whose faces do not sit between their
@@ -1402,12 +1402,14 @@ __device__ __forceinline__ void face_geom(const sfx_dmesh& m, int f, FaceGeom<D>
  * kFaceMoving: records, face velocities and local time steps, dW/dt formed
  * here (at the boosted state; a cell in the middle of its step keeps its
  * gradients).
- * What a face needs of its two cells is one gather of 3 + 10 (2D: 3 + 6)
- * 16-byte loads per side and its own geometry a coalesced record; from
- * field-major arrays it was 28 (20) scattered doubles per side and the
- * geometry's square roots and divisions on every step.  HLLC: 101 -> 67 us on
- * 65,537 cells (500,000 faces) in 3D, 71 -> 51 us on 150,001 in 2D; bound by
- * FP64 latency at 16 warps per SM (128 registers). */
+ * What a face needs of its two cells is one gather of 2 + 5 (2D: 2 + 3)
+ * 32-byte loads per side and its own geometry planes of 32 bytes that
+ * consecutive threads read consecutively; from field-major arrays it was 28
+ * (20) scattered doubles per side and the geometry's square roots and
+ * divisions on every step.  HLLC: 101 -> 55 us on 65,537 cells (500,000 faces)
+ * in 3D, 71 -> 44 us on 150,001 in 2D (67 and 51 with 16-byte loads); bound by
+ * FP64 latency at 16 warps per SM (118 registers; 5 or 6 blocks of 128 per SM
+ * took the same time). */
 constexpr int kFaceArrays = 0, kFaceRecords = 1, kFaceMoving = 2;
 
 /* a face's Riemann problem and what its dQ needs: predicted states, normal,
@@ -1738,7 +1740,12 @@ __global__ void __launch_bounds__(kExactBlock, 2)
         int at = 0;
         if(lane == 0) at = atomicAdd(m.listed_n, __popc(listed));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(listed & ((1u << lane) - 1u));
-        if(key == kKeyListed) m.listed[at] = f;
+        if(key == kKeyListed) {
+            if(at < m.n_faces)
+                m.listed[at] = f;
+            else
+                report_face(m.err, f, SFX_ERR_INVALID);
+        }
     }
     /* counting sort by key */
     unsigned mine = 0;
@@ -1808,7 +1815,7 @@ constexpr int kListedBlock = 128, kListedBlocks = 4 * 148;
 template <int D, int MODE>
 __global__ void __launch_bounds__(kListedBlock)
         k_faces_listed(sfx_dmesh m, sfx_solver_params sp, double dt, int write_branch) {
-    const int count = *(volatile const int*)m.listed_n;
+    const int count = min(*(volatile const int*)m.listed_n, m.n_faces);
     for(int j = blockIdx.x * kListedBlock + threadIdx.x; j < count;
         j += kListedBlocks * kListedBlock) {
         if(failed(m.err)) return;
@@ -2415,7 +2422,12 @@ static void launch_gradients(const sfx_dmesh* m, double gamma, int nc, cudaStrea
 
 int sfx_fp64_gradients(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream) {
     const int nc = sfx_grad_cells(*m);
-    if(nc == 0) return SFX_OK;
+    if(nc == 0) {
+        /* no gradient launch to empty the face list (a part without cells) */
+        if(!m->listed_n) return SFX_OK;
+        return cuda_status(
+                cudaMemsetAsync(m->listed_n, 0, sizeof(int32_t), (cudaStream_t)stream));
+    }
     if(m->dim == 3)
         launch_gradients<3>(m, sp->gamma, nc, (cudaStream_t)stream);
     else

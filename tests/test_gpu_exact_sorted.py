@@ -36,3 +36,22 @@ def test_sorted_faces_equal_the_oracle(oracle, dim, n, cutoff):
         assert np.array_equal(dq, odq)
     fp.close()
     ctx.close()
+
+
+def test_face_list_is_emptied_without_a_gradient_launch():
+    """a part with faces and no cells of its own: the list of each step starts empty"""
+    mesh = build_voronoi(random_generators(25_600, 2, 17), periodic=True)
+    assert mesh.n_faces > LIST_FROM
+    W = wl.random_field_state(mesh, 23)
+    ctx = Context(2, RiemannSolverFactory.generate("Exact", cutoff=-1e3), 0)   # every face listed
+    fp = FluxPass(ctx, mesh)
+    fp.set_primitive(W)
+    fp.step(0.1 * wl.cfl_dt(mesh, W), 1)
+    before = fp.state()
+    fp.set_ranges(0, mesh.n_faces, 0)
+    st = fp.step(0.1 * wl.cfl_dt(mesh, W), 3)
+    assert st.status == 0
+    after = fp.state()
+    assert np.array_equal(before[0], after[0]) and np.array_equal(before[1], after[1])
+    fp.close()
+    ctx.close()
