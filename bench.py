@@ -221,37 +221,40 @@ def peaks():
 
 
 def algorithmic_bytes(dim: int, n_cells: int, n_faces: int, nnz: int, precision: str):
-    """bytes each kernel of one step must move at least once (FP64 plain):
-    gradients: read W, pos, centroid, volume, CSR (offsets + entries) per
-    cell; per face area, midpoint, left, right, kind, right generator
-    position; write the gradient (dim*S) per cell.
-    faces: read the face record, per cell W, gradient, centroid, pos, Q.m,
-    total area; write dQ (S) per face.
-    update: read Q, volume, CSR, dQ per face; write Q and W per cell."""
+    """bytes each kernel of one step must move at least once (plain FP64), in
+    its device layout (sfx_fp64.cu's records).
+    gradients: per cell the state record (S + 1 doubles), centroid, volume,
+    offset; per face the gradient geometry (12 doubles); 8 bytes per CSR
+    entry; write gradients and dW/dt ((dim + 1) S) per cell.
+    faces: per face the flux geometry (16 doubles in 3D, 12 in 2D) and the
+    dQ record (6 / 4); per cell state record, gradients and dW/dt.
+    update: read Q, volume, CSR, dQ per face; write Q, W and the state
+    record per cell."""
     S = dim + 2
-    face_rec = 8 + 8 * dim + 4 + 4 + 4 + 8 * dim
-    cell_grad_in = 8 * S + 8 * dim + 8 * dim + 8 + 4
-    grad = n_cells * (cell_grad_in + 8 * dim * S) + nnz * 4 + n_faces * face_rec
-    faces = n_faces * (face_rec + 8 * S) + n_cells * (8 * S + 8 * dim * S + 8 * dim + 8 * dim + 8 + 8)
-    update = n_cells * (8 * S + 8 + 4 + 8 * S * 2) + nnz * 4 + n_faces * (8 * S + 8)
+    dq = 8 * (6 if dim == 3 else 4)
+    slopes = 8 * (dim + 1) * S
+    grad = n_cells * (8 * (S + 1) + 8 * dim + 8 + 4 + slopes) + nnz * 8 + n_faces * 96
+    faces = n_faces * (8 * (16 if dim == 3 else 12) + dq) + n_cells * (8 * (S + 1) + slopes)
+    update = n_cells * (8 * S + 8 + 4 + 8 * S * 2 + 8 * (S + 1)) + nnz * 4 + n_faces * dq
     return {"gradients": grad, "faces": faces, "update": update}
 
 
 def split_kernel_bytes(dim: int, n_cells: int, n_faces: int, nnz: int):
     """bytes each split-pass kernel must move at least once per launch, in
-    its device layout: face record fg (2 float4) + fi (int2) + shift code
-    (1 B) + FP64 area vector (8 dim); cell record cw (2 float4), cx
-    (float4), gradients cg (G float4, G = 4 in 3D, 2 in 2D); per-face dQ
-    {mass, energy} float2 + FP64 momentum (8 dim); Q FP64 (8 S).
-    gradients: cw, cx, offset, CSR entry, face fg + fi; write cg.
-    faces: face record, dQ write, and per cell cw, cx, cg.
-    update: offset, CSR entry, per-face dQ, Q read+write, volume, total
-    area (FP64), write cw."""
+    its device layout: gradient geometry fg (32 per face), flux record fr
+    (48 per face), FP64 area vector (8 dim), cell record cw (32), cx (16),
+    gradients cg (G = 64 in 3D, 32 in 2D) and dW/dt (G / 2), dQ record (32 in
+    3D, 24 in 2D); Q FP64 (8 S).
+    gradients: cw, cx, offset, CSR entries (8), fg; write cg and dW/dt.
+    faces: fr, area vector, dQ write, and per cell cw and cg.
+    update: offset, CSR entry, dQ, Q read+write, volume, total area (FP64),
+    write cw."""
     S = dim + 2
-    G = 16 * (4 if dim == 3 else 2)
-    grad = n_cells * (32 + 16 + 4 + G) + n_faces * (32 + 8) + nnz * 4
-    faces = n_faces * (32 + 8 + 1 + 8 * dim + 8 + 8 * dim) + n_cells * (32 + 16 + G)
-    update = n_cells * (4 + 16 * S + 8 + 8 + 32) + nnz * 4 + n_faces * (8 + 8 * dim)
+    G = 64 if dim == 3 else 32
+    dq = 32 if dim == 3 else 24
+    grad = n_cells * (32 + 16 + 4 + G + G // 2) + n_faces * 32 + nnz * 8
+    faces = n_faces * (48 + 8 * dim + dq) + n_cells * (32 + G)
+    update = n_cells * (4 + 16 * S + 8 + 8 + 32) + nnz * 4 + n_faces * dq
     return {"gradients": grad, "faces": faces, "update": update}
 
 
@@ -469,7 +472,7 @@ def bench_batch(args, rank, world, local, torch):
                        "parallelism": f"replicas x{world}", "mesh_build_s": round(t_build, 1)},
             "clocks": clk.summary(),
             "fp64_per_mesh": {"value": fp64_value, "unit": UNIT, "steps": base_steps,
-                              "launch": "4 launches per mesh per step, plain FP64"},
+                              "launch": "3 launches per mesh per step, plain FP64"},
             "speedup_vs_fp64_per_mesh": value / fp64_value,
             "split_vs_fp64_max_rel_l1_mass_energy": max(acc) if acc else None,
             "roofline": {"bound": "hbm", "peak": peak, "unit": "GB/s",
@@ -790,10 +793,10 @@ def run_resident(pool, reqs, nseg, warmup, chunk, torch, local):
 # (2,396,113 faces) and a 700,000-cell one in 2D; the gathers and the per-face
 # records scale with the faces, so a launch over F faces moves about F times
 # these
-TRAFFIC_B_PER_FACE = {("faces", 3, "Exact"): 106.8, ("faces", 3, "HLLC"): 102.0,
-                      ("gradients", 3): 61.4, ("update", 3): 52.8,
-                      ("faces", 2, "Exact"): 104.8, ("faces", 2, "HLLC"): 98.6,
-                      ("gradients", 2): 73.3, ("update", 2): 54.2}
+TRAFFIC_B_PER_FACE = {("faces", 3, "Exact"): 114.1, ("faces", 3, "HLLC"): 107.3,
+                      ("gradients", 3): 61.7, ("update", 3): 49.2,
+                      ("faces", 2, "Exact"): 107.8, ("faces", 2, "HLLC"): 101.3,
+                      ("gradients", 2): 74.2, ("update", 2): 55.6}
 
 
 def split_kernel_name(role: str, solver: str) -> str:
@@ -1276,7 +1279,8 @@ def main():
         traffic = split_traffic(names[top], D, pr.solver, mesh.n_active_faces)
     else:
         alg = algorithmic_bytes(D, mesh.n_cells, mesh.n_faces, mesh.nnz, args.precision)
-        kname = {"gradients": "k_grad_terms + k_grad_sum", "faces": "k_faces",
+        kname = {"gradients": "k_grad_cells",
+                 "faces": "k_faces" if pr.solver == "HLLC" else "k_faces_exact + k_faces_listed",
                  "update": "k_apply"}[names[top]]
         traffic = None
     peak, peak_kind = peaks()
