@@ -292,7 +292,7 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision);
  * tree of the per-cell sums, not the algorithm. */
 int sfx_mesh_set_lanes(sfx_mesh* mesh, int32_t lanes);
 /* split pass: face-kernel variant: 0 (64 registers, four 256-thread blocks
- * per SM; the default), 1 (80 registers, three blocks), 2 (HLLC: the
+ * per SM, in 2D HLLC as 3 where that is more than one wave; the default), 1 (80 registers, three blocks), 2 (HLLC: the
  * half-step prediction's dW/dt read from the per-cell record instead of
  * formed per face; exact solver: as 0), 3 (exact solver: as 1; HLLC: 48
  * registers, five blocks), 4 (the left cells of each 256-face block staged in

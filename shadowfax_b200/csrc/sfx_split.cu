@@ -49,6 +49,13 @@ constexpr int kSolveInline = 0, kSolveDefer = 1;
 /* blocks of the group's queued-face launch (two waves of 128-thread blocks
  * on 148 SMs; the launch strides over each member's queue) */
 constexpr int kSlowGroupBlocks = 296;
+/* 2D HLLC face kernel: above one wave of 64-register blocks (four per SM on
+ * 148 SMs) variant 0 takes the 48-register kernel, five blocks per SM, whose
+ * gathers have more warps to hide in: 12.0 us against 12.5 at 300,000 faces,
+ * 36.6 against 39.8 at 1.2 million, 123 against 138 at 4.8 million; below a
+ * wave (60,000 faces) 5.6 against 5.4.  In 3D it is slower at every size (35
+ * against 31.5 us at 800,000 faces). */
+constexpr int kOneWaveHllc2d = 4 * 148;
 
 __device__ __forceinline__ void report_face(sfx_dev_error* e, int f, int st) {
     atomicMin(&e->face_key, ((unsigned long long)(unsigned)f << 8) | (unsigned)st);
@@ -2419,7 +2426,7 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
                     if(v == 4)
                         k_group_sfaces<D, SFX_SOLVER_HLLC, 5, false, false, true>
                                 <<<g->blocks[1], 256, 0, s>>>(g->tab, pre1, nm, *sp);
-                    else if(v == 3)
+                    else if(v == 3 || (v == 0 && D == 2 && g->blocks[1] > kOneWaveHllc2d))
                         k_group_sfaces<D, SFX_SOLVER_HLLC, 5><<<g->blocks[1], 256, 0, s>>>(
                                 g->tab, pre1, nm, *sp);
                     else if(v == 1)

@@ -79,3 +79,22 @@ def test_small_and_ragged_meshes_at_every_lane_count(dim, n, solver):
     scale = (W64[:, 0] * mesh.cell_volume * np.sqrt(wl.GAMMA * W64[:, -1] / W64[:, 0])).sum()
     for lanes in (1, 2, 4, 16):
         _close(_run(mesh, W, solver, 1, dt, 3, lanes)[1], Q64, scale)
+
+
+@pytest.mark.parametrize("n", [50_000, 51_500])
+def test_2d_hllc_kernels_on_both_sides_of_one_wave(n):
+    """the default face variant, 64 registers below 151,552 faces and 48 above, has the bits of
+    the 80-register variant 1"""
+    mesh = build_voronoi(random_generators(n, 2, 5), periodic=True)
+    assert (mesh.n_faces > 4 * 148 * 256) == (n == 51_500)
+    W = wl.random_field_state(mesh, 5)
+    ctx = Context(2, RiemannSolverFactory.generate("HLLC"), 1)
+    fp = FluxPass(ctx, mesh)
+    out = []
+    for variant in (0, 1):
+        fp.set_face_variant(variant)
+        fp.set_primitive(W)
+        out.append(fp.flux_pass(0.1 * wl.cfl_dt(mesh, W))[1])
+    assert np.array_equal(out[0], out[1])
+    fp.close()
+    ctx.close()
