@@ -788,10 +788,12 @@ int sfx_step_moving(sfx_mesh* m, double dt, int32_t periodic, double* positions,
     sfx_dmesh& d = m->d;
     const int64_t n = d.n_cells, F = d.n_faces;
     const int D = d.dim;
-    if(!d.vgen) SFX_TRY(dalloc(m, &d.vgen, (size_t)D * n));
-    if(!d.newpos) SFX_TRY(dalloc(m, &d.newpos, (size_t)D * n));
     const bool fresh = d.vel == nullptr;
-    if(fresh) SFX_TRY(dalloc(m, &d.vel, (size_t)D * (F > 0 ? F : 1)));
+    Carver first; /* one allocation: a moving mesh takes one step per tessellation */
+    if(!d.vgen) first.add(&d.vgen, (size_t)D * n);
+    if(!d.newpos) first.add(&d.newpos, (size_t)D * n);
+    if(fresh) first.add(&d.vel, (size_t)D * F);
+    if(!first.slots.empty()) SFX_TRY(first.allocate(m));
     d.has_velocity = 1;
     SFX_TRY(reset_err(m));
     /* the split pass keeps the state in FP32 cell records: the FP64 W the
