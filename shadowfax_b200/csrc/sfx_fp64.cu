@@ -745,7 +745,7 @@ __device__ __noinline__ double xexp(LogPair p, double y) {
     const double th = y * p.h;
     const double tl = sfx_fma(y, p.h, -th) + y * p.l;
     double r;
-    return sfx_powq_exp(th, tl, &r) ? r : sfx_pow_rare64(p.x, y);
+    return sfx_powq_exp(th, tl, y, &r) ? r : sfx_pow_rare64(p.x, y);
 }
 
 __device__ __forceinline__ double xpow(double x, double y) {

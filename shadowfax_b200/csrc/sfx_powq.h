@@ -3,14 +3,15 @@
  * the plain-FP64 exact solver (host and device code).
  *
  * sfx_pow (sfx_pow.h) returns the correctly rounded power except within 2^-90
- * of a rounding boundary.  sfx_powq evaluates the power to about 2^-70 with
- * table-driven reductions and rounds it once, but only where no rounding
- * boundary lies within 2^-68 of the value (Ziv's rounding test: A. Ziv, "Fast
+ * of a rounding boundary.  sfx_powq evaluates the power with table-driven
+ * reductions, to about 2^-71 (1 + |y|): the logarithm's error is multiplied by
+ * the exponent.  It rounds the value once, but only where no rounding boundary
+ * lies within a margin of 2^-68 + |y| 2^-70 (Ziv's rounding test: A. Ziv, "Fast
  * evaluation of elementary mathematical functions with correctly rounded last
  * bit", ACM TOMS 17, 1991); there both routines return the same double.
- * Elsewhere (about 1 argument in 10^4), outside x > 0 normal, and for
- * |y ln x| >= 22, it calls SFX_POWQ_RARE (sfx_pow, or the includer's
- * out-of-line copy of it).
+ * Elsewhere (about 1 argument in 10^4 for |y| <= 5, 1 in 440 at |y| = 202 and
+ * all above |y| = 2^17), outside x > 0 normal, and for |y ln x| >= 22, it calls
+ * SFX_POWQ_RARE (sfx_pow, or the includer's out-of-line copy of it).
  *
  * Method (P. T. P. Tang, "Table-driven implementation of the logarithm
  * function", ACM TOMS 16, 1990, and "... of the exponential function", ACM
@@ -156,8 +157,9 @@ SFX_HD double sfx_powq_exp_tab(int i) {
 #endif
 }
 
-/* ln x as a pair, absolute error below 2^-72 + 2^-100 |ln x|; 0: x is not a
- * positive normal number (the pair is then of no use).  No branches, here and
+/* ln x as a pair, absolute error below 2^-71 + 2^-100 |ln x| (the cubic term's
+ * roundings, r^3 2^-52 and less, and the last sum's); 0: x is not a positive
+ * normal number (the pair is then of no use).  No branches, here and
  * in sfx_powq_exp, so that two calls side by side overlap. */
 SFX_HD int sfx_powq_log(double x, double* rh, double* rl) {
     const uint64_t u = sfx_d2u(x);
@@ -192,9 +194,9 @@ SFX_HD int sfx_powq_log(double x, double* rh, double* rl) {
     return ex - 1 < 0x7fe;
 }
 
-/* exp(th + tl), rounded; 0: |th| >= 22 or NaN, or a rounding boundary lies too
- * near */
-SFX_HD int sfx_powq_exp(double th, double tl, double* out) {
+/* exp(th + tl) with th + tl = y ln x, rounded; 0: |th| >= 22 or NaN, or a
+ * rounding boundary lies too near */
+SFX_HD int sfx_powq_exp(double th, double tl, double y, double* out) {
     const double kd = (th * 0x1.71547652b82fep+5 + 0x1.8p52) - 0x1.8p52;
     const int in_range = (th < 0.0 ? -th : th) < 22.0; /* 0 for a NaN */
     const int k = in_range ? (int)kd : 0;
@@ -220,7 +222,8 @@ SFX_HD int sfx_powq_exp(double th, double tl, double* out) {
     double h, l;
     sfx_fast_two_sum(Th, p, &h, &l);
     l = l + (pl + sfx_fma(Th, el, sfx_fma(Tl, eh, Tl)));
-    const double err = h * 0x1p-68;
+    /* this function's error (below 2^-71) and |y| times the logarithm's */
+    const double err = h * sfx_fma(y < 0.0 ? -y : y, 0x1p-70, 0x1p-68);
     const double up = h + (l + err), dn = h + (l - err);
     *out = up * sfx_u2d((uint64_t)((k >> 5) + 1023) << 52);
     return in_range & (up == dn);
@@ -231,7 +234,7 @@ SFX_HD double sfx_powq(double x, double y) {
     if(sfx_powq_log(x, &lh, &ll)) {
         const double th = y * lh;
         const double tl = sfx_fma(y, lh, -th) + y * ll;
-        if(sfx_powq_exp(th, tl, &r)) return r;
+        if(sfx_powq_exp(th, tl, y, &r)) return r;
     }
     return SFX_POWQ_RARE(x, y);
 }
