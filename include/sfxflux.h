@@ -281,7 +281,8 @@ int sfx_mesh_totals(sfx_mesh* mesh, double* totals);
  * only a state (W, Q and the per-step scratch of ctx's precision): several
  * integrations of one tessellation without copying it again.  `base` must
  * outlive the clone and have been uploaded with the split arrays if ctx is
- * SFX_PREC_SPLIT.  sfx_flux_pass is not available on split clones. */
+ * SFX_PREC_SPLIT.  A plain-FP64 clone of a split mesh forms the FP64 pass's face
+ * records and lists of faces for itself.  sfx_flux_pass is not available on split clones. */
 int sfx_mesh_clone(sfx_ctx* ctx, sfx_mesh* base, sfx_mesh** out);
 /* device bytes a clone of `base` at `precision` allocates */
 int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision);

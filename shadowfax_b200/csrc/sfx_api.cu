@@ -10,8 +10,10 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "sfx_internal.h"
@@ -39,6 +41,13 @@ struct sfx_mesh {
     int32_t* self_pre = nullptr;
     float self_dt = 0.f; /* time step held in self_tab (0: none yet) */
     bool clone = false;  /* geometry shared with the base mesh */
+    /* split meshes: the CSR entries that name the other copy of a periodic face
+     * pair (sfx_mesh_upload), as {position, the cell's own face} */
+    std::shared_ptr<const std::vector<std::pair<int64_t, int32_t>>> merged;
+    /* a plain-FP64 clone of a split mesh has a CSR of its own; the split one, for
+     * split clones of it in turn */
+    int32_t* split_idx = nullptr;
+    int2* split_ent = nullptr;
     unsigned long long* d_smin = nullptr; /* local time steps: smallest new step */
 };
 
@@ -226,6 +235,49 @@ struct Carver {
     }
 };
 
+/* The CSR with each cell's faces in ascending order, when `idx` does not list
+ * them so (empty otherwise): the reference adds each face's dQ to its cells in
+ * its face loop (src/VorTessManager.cpp:198-212), while a cell's gradient walks
+ * the cell's own face list (src/VorCell.cpp:464-530) */
+std::vector<int32_t> ascending_csr(const int32_t* off, const std::vector<int32_t>& idx,
+                                   int64_t n) {
+    std::vector<int32_t> out;
+    bool ascending = true;
+    for(int64_t i = 0; i < n && ascending; ++i)
+        for(int64_t j = off[i] + 1; j < off[i + 1]; ++j)
+            if((idx[j] & 0x7fffffff) < (idx[j - 1] & 0x7fffffff)) {
+                ascending = false;
+                break;
+            }
+    if(ascending) return out;
+    out = idx;
+    for(int64_t i = 0; i < n; ++i)
+        std::sort(out.begin() + off[i], out.begin() + off[i + 1],
+                  [](int32_t a, int32_t b) { return (a & 0x7fffffff) < (b & 0x7fffffff); });
+    return out;
+}
+
+/* What a plain-FP64 clone of a split mesh cannot share: the pass's face records
+ * (formed here from the base's geometry) and a CSR in which every cell names
+ * its own copy of a periodic face, in the FP64 update's order */
+int fill_fp64_geometry(sfx_mesh* m, cudaStream_t s) {
+    sfx_dmesh& d = m->d;
+    std::vector<int32_t> off((size_t)d.n_cells + 1), idx((size_t)d.nnz);
+    SFX_TRY(cuda_ok(cudaMemcpyAsync(off.data(), d.off, off.size() * sizeof(int32_t),
+                                    cudaMemcpyDeviceToHost, s)));
+    SFX_TRY(cuda_ok(cudaMemcpyAsync(idx.data(), m->split_idx, idx.size() * sizeof(int32_t),
+                                    cudaMemcpyDeviceToHost, s)));
+    SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
+    if(m->merged)
+        for(const auto& e : *m->merged) idx[(size_t)e.first] = e.second;
+    const std::vector<int32_t> aidx = ascending_csr(off.data(), idx, d.n_cells);
+    SFX_TRY(h2d(d.idx, idx.data(), idx.size(), s));
+    SFX_TRY(h2d(d.aidx, (aidx.empty() ? idx : aidx).data(), idx.size(), s));
+    SFX_TRY(sfx_fp64_csr_neighbours(&d, s));
+    SFX_TRY(sfx_fp64_face_records(&d, s));
+    return cuda_ok(cudaStreamSynchronize(s)); /* the host vectors end here */
+}
+
 /* a state on base's geometry: one device block carved into the arrays,
  * set up on stream s (waited for when `wait`) */
 int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh** out) {
@@ -242,6 +294,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     ctx->live_meshes++;
     m->d = b; /* geometry pointers shared with the base */
     m->clone = true;
+    m->merged = base->merged;
     m->d.vgen = m->d.newpos = nullptr;
     m->d.tstart = m->d.tend = nullptr;
     m->d_smin = nullptr;
@@ -258,6 +311,14 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     d.slowq = nullptr;
     d.slowq_n = nullptr;
     d.slowq_cap = 0;
+    if(split) {
+        /* of an FP64 clone of a split mesh: that mesh's CSR again */
+        d.ggeo = d.fgeo = nullptr;
+        if(base->split_idx) {
+            d.idx = base->split_idx;
+            d.ent = base->split_ent;
+        }
+    }
     Carver arrays;
     auto A = [&](auto** p, size_t c) { arrays.add(p, c); };
     A(&d.W, n * S);
@@ -265,6 +326,19 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     A(&d.stage, n * S);
     A(&d.err, 1);
     A(&d.totals_scratch, (size_t)(S + 1) * 1024);
+    const bool geometry = !split && !b.ggeo; /* the base is split */
+    if(geometry) {
+        m->split_idx = d.idx;
+        m->split_ent = d.ent;
+        A(&d.ggeo, F * rec_doubles(dim, SFX_REC_GGEO));
+        A(&d.fgeo, F * rec_doubles(dim, SFX_REC_FGEO));
+        A(&d.idx, d.nnz);
+        A(&d.aidx, d.nnz);
+        A(&d.ent, d.nnz);
+    } else if(!split) {
+        m->split_idx = base->split_idx;
+        m->split_ent = base->split_ent;
+    }
     if(split) {
         A(&d.cw, 2 * n);
         A(&d.cg, (size_t)sfx_split_grad_vec4(dim) * n);
@@ -287,6 +361,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     if(!rc) rc = reset_err_on(m, s);
     if(!rc && split) rc = cuda_ok(cudaMemsetAsync(d.slowq_n, 0, sizeof(int32_t), s));
     if(!rc && split) rc = setup_self(m, s);
+    if(!rc && geometry) rc = fill_fp64_geometry(m, s);
     if(!rc && wait) rc = cuda_ok(cudaStreamSynchronize(s));
     if(rc) {
         sfx_mesh_free(m);
@@ -512,28 +587,11 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
             }
         }
     }
-    /* The reference adds each face's dQ to its cells in its face loop, in
-     * ascending face order (src/VorTessManager.cpp:198-212), while a cell's
-     * gradient walks the cell's own face list (src/VorCell.cpp:464-530).  A
-     * face list whose cells list their faces in ascending order (the
-     * builder's) serves both; otherwise the plain-FP64 update gets a copy of
-     * the CSR sorted per cell, so that its sums round as the reference's. */
+    /* The builder's cells list their faces in ascending order and one CSR serves
+     * both passes; otherwise the plain-FP64 update gets a sorted copy, so that
+     * its sums round as the reference's. */
     std::vector<int32_t> aidx;
-    if(ctx->cfg.precision == SFX_PREC_FP64) {
-        bool ascending = true;
-        for(int64_t i = 0; i < n && ascending; ++i)
-            for(int64_t j = off[i] + 1; j < off[i + 1]; ++j)
-                if((idx[j] & 0x7fffffff) < (idx[j - 1] & 0x7fffffff)) {
-                    ascending = false;
-                    break;
-                }
-        if(!ascending) {
-            aidx = idx;
-            for(int64_t i = 0; i < n; ++i)
-                std::sort(aidx.begin() + off[i], aidx.begin() + off[i + 1],
-                          [](int32_t a, int32_t b) { return (a & 0x7fffffff) < (b & 0x7fffffff); });
-        }
-    }
+    if(ctx->cfg.precision == SFX_PREC_FP64) aidx = ascending_csr(off, idx, n);
     /* Split pass only: a face across a periodic boundary is listed twice, once
      * owned by each cell (the reference computes it twice and lets each copy
      * update only its owner, src/VorFace.cpp:913-955).  The split pass
@@ -548,6 +606,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
      * copy with the same rounding. */
     std::vector<uint8_t> skip;
     std::vector<int32_t> idx_split;
+    std::vector<std::pair<int64_t, int32_t>> merged;
     if(ctx->cfg.precision == SFX_PREC_SPLIT) {
         skip.assign(F, 0);
         idx_split = idx;
@@ -601,7 +660,10 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         for(int64_t i = 0; i < n; ++i)
             for(int64_t j = off[i]; j < off[i + 1]; ++j) {
                 const int32_t g = desc->cell_face_index[j];
-                if(skip[g]) idx_split[j] = (int32_t)((uint32_t)twin[g] | 0x80000000u);
+                if(skip[g]) {
+                    idx_split[j] = (int32_t)((uint32_t)twin[g] | 0x80000000u);
+                    merged.emplace_back(j, idx[j]);
+                }
             }
     }
     SFX_TRY(cuda_ok(cudaSetDevice(ctx->cfg.device)));
@@ -610,6 +672,9 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!m) return SFX_ERR_NOMEM;
     m->ctx = ctx;
     ctx->live_meshes++;
+    if(!merged.empty())
+        m->merged = std::make_shared<const std::vector<std::pair<int64_t, int32_t>>>(
+                std::move(merged));
     sfx_dmesh& d = m->d;
     std::memset(&d, 0, sizeof d);
     d.dim = dim;
@@ -1088,10 +1153,12 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
         bytes += n * 32 + n * 16 * (sfx_split_grad_vec4((int)D) + sfx_split_dwdt_vec4((int)D)) +
                  F * 32 +
                  4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 28;
-    else
-        bytes += n * (int64_t)(sfx_fp64_record_bytes((int)D, SFX_REC_WS) +
-                               sfx_fp64_record_bytes((int)D, SFX_REC_GREC)) +
-                 F * (8 + (int64_t)sfx_fp64_record_bytes((int)D, SFX_REC_DQ)) + 512;
+    else {
+        auto rec = [&](int what) { return (int64_t)sfx_fp64_record_bytes((int)D, what); };
+        bytes += n * (rec(SFX_REC_WS) + rec(SFX_REC_GREC)) + F * (8 + rec(SFX_REC_DQ)) + 512;
+        if(!b.ggeo) /* of a split mesh: face records and CSR of its own */
+            bytes += F * (rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO)) + (int64_t)b.nnz * 16 + 1280;
+    }
     return bytes;
 }
 
