@@ -57,6 +57,11 @@ __device__ __forceinline__ bool failed(const sfx_dev_error* e) {
            (*(volatile const unsigned long long*)&e->cell_key != ~0ull);
 }
 
+/* a face lower than f has failed: f cannot change the record */
+__device__ __forceinline__ bool below(const sfx_dev_error* e, int f) {
+    return *(volatile const unsigned long long*)&e->face_key < (unsigned long long)(unsigned)f << 8;
+}
+
 /* ---------------- time derivative (Exact :892-934 / HLLC :415-450) ------- */
 template <int D>
 __device__ __forceinline__ void time_derivative(double gamma, const double* W,
@@ -1809,7 +1814,10 @@ __global__ void __launch_bounds__(kExactBlock, 2)
                      eo.code, eo.status, write_branch);
 }
 
-/* the listed faces, one per thread; nothing to do when there are none */
+/* The listed faces, one per thread; nothing to do when there are none.  A
+ * failure of this step's other faces does not end it: the record names the
+ * lowest failing face, and that one may be listed (after a failure of an
+ * earlier step or phase the list is empty). */
 constexpr int kListedBlock = 128, kListedBlocks = 4 * 148;
 
 template <int D, int MODE>
@@ -1818,8 +1826,8 @@ __global__ void __launch_bounds__(kListedBlock)
     const int count = min(*(volatile const int*)m.listed_n, m.n_faces);
     for(int j = blockIdx.x * kListedBlock + threadIdx.x; j < count;
         j += kListedBlocks * kListedBlock) {
-        if(failed(m.err)) return;
         const int f = m.listed[j];
+        if(below(m.err, f)) continue;
         FaceProblem<D> q;
         if(!face_problem<D, MODE>(m, sp, dt, f, write_branch, q)) continue;
         double flux[D + 2];

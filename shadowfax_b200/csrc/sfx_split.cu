@@ -68,6 +68,11 @@ __device__ __forceinline__ bool failed(const sfx_dev_error* e) {
            (*(volatile const unsigned long long*)&e->cell_key != ~0ull);
 }
 
+/* a face lower than f has failed: f cannot change the record */
+__device__ __forceinline__ bool below(const sfx_dev_error* e, int f) {
+    return *(volatile const unsigned long long*)&e->face_key < (unsigned long long)(unsigned)f << 8;
+}
+
 /* FP32 reciprocal and square root as single hardware operations (1 to 2 ulp,
  * as the unit's / and sqrtf, which also carry code for subnormal operands):
  * a subnormal counts as zero here, a state 18 orders of magnitude below the
@@ -1781,7 +1786,11 @@ __device__ __forceinline__ bool sfaces_body(const sfx_dmesh& m, const sfx_solver
                                             const float dt, const int f,
                                             const LeftTile<D>& tile = LeftTile<D>{}) {
     constexpr int S = D + 2;
-    if(f >= sfx_flux_faces(m) || failed(m.err)) return false;
+    /* a queued face is solved even when another face of the step has failed: the
+     * record names the lowest one (after a failure of an earlier step or phase
+     * the queue is empty) */
+    if(f >= sfx_flux_faces(m) || (MODE == kSolveInline ? below(m.err, f) : failed(m.err)))
+        return false;
     FaceWork<D> w;
     /* by default HLLC forms dW/dt itself and the exact solver's kernels read
      * it (STORED_DW: from the per-cell record) */
