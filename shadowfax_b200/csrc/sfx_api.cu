@@ -140,7 +140,7 @@ int32_t slowq_capacity(int64_t n_faces) {
     return (int32_t)(n_faces > 0 ? n_faces : 1);
 }
 
-/* a one-member group's prefix sums and the word behind them */
+/* a one-member group's prefix sums and, last, the word behind them */
 constexpr int kSelfPre = 7;
 
 /* device table of a split mesh as a one-member launch group */
@@ -186,6 +186,11 @@ int run_phase(sfx_mesh* m, int phase, double dt, int write_branch, cudaStream_t 
             g.blocks[1] = b[1];
             sfx_split_blocks(m->d.dim, m->d.lanes, sfx_update_cells(m->d), 0, b);
             g.blocks[2] = b[2];
+            if(phase == 0 && g.blocks[0] == 0) {
+                /* no gradient launch to empty the queue (a part without cells) */
+                SFX_TRY(cuda_ok(cudaMemsetAsync(m->d.slowq_n, 0, sizeof(int32_t), s)));
+                SFX_TRY(cuda_ok(cudaMemsetAsync(m->self_pre + kSelfPre - 1, 0, sizeof(int32_t), s)));
+            }
         }
         return sfx_split_group_phase(&g, phase, &c->sp, s);
     }
