@@ -1402,7 +1402,7 @@ __device__ __forceinline__ void face_geom(const sfx_dmesh& m, int f, FaceGeom<D>
     for(int l = 0; l < D; ++l) q.n[l] = -dd[l] / dn;
 }
 
-/* kFaceArrays: field-major caller-owned arrays.  kFaceRecords: a mesh's
+/* kFaceArrays: field-major arrays (caller-owned, or of a mesh without records).  kFaceRecords: a mesh's
  * records, dW/dt from the cell's (a static mesh with one step).
  * kFaceMoving: records, face velocities and local time steps, dW/dt formed
  * here (at the boosted state; a cell in the middle of its step keeps its
@@ -1849,7 +1849,7 @@ __global__ void __launch_bounds__(kListedBlock)
  * 23 and 24 us. */
 constexpr int kApplyBlock = 128;
 
-template <int D>
+template <int D, bool REC>
 __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma) {
     using R = Rec<D>;
     constexpr int S = R::S;
@@ -1867,8 +1867,15 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma
 #pragma unroll
         for(int t = 0; t < U; ++t) e[t] = (unsigned)__ldg(m.aidx + (j + t < end ? j + t : j));
 #pragma unroll
-        for(int t = 0; t < U; ++t)
-            load_record<R::dq>(m.dQf + (size_t)(e[t] & ~kRightBit) * R::dq, v[t]);
+        for(int t = 0; t < U; ++t) {
+            const size_t f = e[t] & ~kRightBit;
+            if constexpr(REC) {
+                load_record<R::dq>(m.dQf + f * R::dq, v[t]);
+            } else {
+#pragma unroll
+                for(int k = 0; k < S; ++k) v[t][k] = __ldg(m.dQf + (size_t)k * m.n_faces + f);
+            }
+        }
 #pragma unroll
         for(int t = 0; t < U; ++t)
             if(t == 0 || j + t < end) {
@@ -1884,14 +1891,14 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma
         report_cell(m.err, i, SFX_ERR_NEG_STATE);
         return;
     }
-    double* ws = m.ws + (size_t)i * R::ws;
+    double* ws = REC ? m.ws + (size_t)i * R::ws : nullptr;
     if(m.local && m.tend[i] != m.t_next) {
         /* local time steps: a cell in the middle of its step takes the flux
          * of its active neighbours into Q; its W waits for the end of its
          * step (src/Simulation.cpp:791-836) */
 #pragma unroll
         for(int k = 0; k < S; ++k) m.Q[(size_t)k * n + i] = Q[k];
-        ws[S] = Q[0];
+        if(REC) ws[S] = Q[0];
         return;
     }
     /* get_W (ExactRiemannSolver.cpp:716-766 == HLLCRiemannSolver.cpp:495-535
@@ -1928,7 +1935,7 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(sfx_dmesh m, double gamma
         t[k] = W[k];
     }
     t[S] = Q[0];
-    store_record<8>(ws, t);
+    if(REC) store_record<8>(ws, t);
 }
 
 /* Host arrays are rows of one cell or face, device arrays field-major: the
@@ -2097,7 +2104,7 @@ __global__ void k_unpack_cells(sfx_dmesh m, const int32_t* idx, int count, const
         m.W[(size_t)q * m.n_cells + c] = in[t];
     else
         m.Q[c] = in[t];
-    m.ws[(size_t)c * Rec<3>::ws + q] = in[t]; /* W, then the mass: the same stride in 2D */
+    if(m.ws) m.ws[(size_t)c * Rec<3>::ws + q] = in[t]; /* W, then the mass: the same stride in 2D */
 }
 
 inline int grid_for(long long n, int block) {
@@ -2414,8 +2421,8 @@ int sfx_fp64_state_records(const sfx_dmesh* m, void* stream) {
 }
 
 /* k_grad_cells needs the records and face positions that are the cells' (see
- * there); other meshes take k_gradients, caller-owned arrays its field-major
- * form */
+ * there); other meshes take k_gradients, caller-owned arrays and meshes whose
+ * records did not fit its field-major form */
 template <int D>
 static void launch_gradients(const sfx_dmesh* m, double gamma, int nc, cudaStream_t s) {
     const int B = 128;
@@ -2491,11 +2498,15 @@ int sfx_fp64_apply(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream
     const int nc = sfx_update_cells(*m);
     if(nc == 0) return SFX_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    const int B = kApplyBlock;
-    if(m->dim == 3)
-        k_apply<3><<<grid_for(nc, B), B, 0, s>>>(*m, sp->gamma);
+    const int B = kApplyBlock, G = grid_for(nc, B);
+    if(m->dim == 3 && m->ws)
+        k_apply<3, true><<<G, B, 0, s>>>(*m, sp->gamma);
+    else if(m->dim == 3)
+        k_apply<3, false><<<G, B, 0, s>>>(*m, sp->gamma);
+    else if(m->ws)
+        k_apply<2, true><<<G, B, 0, s>>>(*m, sp->gamma);
     else
-        k_apply<2><<<grid_for(nc, B), B, 0, s>>>(*m, sp->gamma);
+        k_apply<2, false><<<G, B, 0, s>>>(*m, sp->gamma);
     sfx_count_launches(1);
     return cuda_status(cudaGetLastError());
 }

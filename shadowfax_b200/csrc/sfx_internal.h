@@ -42,8 +42,8 @@ struct sfx_dmesh {
                        cell lists its faces that way */
     double* W;      /* [S][n]    */
     double* Q;      /* [S][n]    */
-    double* grad;   /* [dim*S][n]: grad[(l*S + k)*n + i] = dW_k/dx_l; caller-owned
-                       arrays only (meshes keep them in grec) */
+    double* grad;   /* [dim*S][n]: grad[(l*S + k)*n + i] = dW_k/dx_l; caller-owned arrays
+                       and meshes without records only (the others keep them in grec) */
     /* faces */
     double* area;   /* [F]       */
     double* mid;    /* [dim][F]  */
@@ -56,7 +56,8 @@ struct sfx_dmesh {
                        (sfx_fp64.cu), otherwise [S][F] */
     /* plain-FP64 meshes: records of the cells' states and of their gradients
      * and dW/dt, and of the faces' gradient and flux geometry (sfx_fp64.cu).
-     * ws == NULL: caller-owned field-major arrays */
+     * ws == NULL: field-major arrays, caller-owned or of a mesh whose records did
+     * not fit on the device */
     double* ws;
     double* grec;
     double* ggeo;
