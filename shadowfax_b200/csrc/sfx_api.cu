@@ -140,6 +140,11 @@ int32_t slowq_capacity(int64_t n_faces) {
     return (int32_t)(n_faces > 0 ? n_faces : 1);
 }
 
+/* doubles of the split pass's dQ per face (store_dq, sfx_split.cu) */
+int64_t split_dq_doubles(int dim) {
+    return dim == 3 ? 4 : 3;
+}
+
 /* a one-member group's prefix sums and, last, the word behind them */
 constexpr int kSelfPre = 7;
 
@@ -375,7 +380,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
             A(&d.cw, 2 * n);
             A(&d.cg, (size_t)sfx_split_grad_vec4(dim) * n);
             A(&d.cdw, (size_t)sfx_split_dwdt_vec4(dim) * n);
-            A(&d.dq, 4 * F);
+            A(&d.dq, split_dq_doubles(dim) * F);
             d.slowq_cap = slowq_capacity(F);
             A(&d.slowq, (size_t)d.slowq_cap);
             A(&d.slowq_n, 1);
@@ -531,7 +536,8 @@ int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
     }
     if(precision == SFX_PREC_SPLIT) {
         /* fg, fr, an, dq, queue; cw, cg, cx, self table */
-        bytes += F * (32 + 4 * 12 + 8 * dim + 32) + 4 * slowq_capacity(F) + 4;
+        bytes += F * (32 + 4 * 12 + 8 * dim + 8 * split_dq_doubles(dim)) +
+                 4 * slowq_capacity(F) + 4;
         bytes += n * (32 + 16 * (sfx_split_grad_vec4((int)dim) + sfx_split_dwdt_vec4((int)dim)) +
                       16) + 256;
     }
@@ -776,7 +782,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         A(&d.cdw, (size_t)sfx_split_dwdt_vec4(dim) * n);
         A(&d.cx, n);
         A(&d.an, (size_t)dim * F);
-        A(&d.dq, 4 * F);
+        A(&d.dq, split_dq_doubles(dim) * F);
         d.slowq_cap = slowq_capacity(F);
         A(&d.slowq, (size_t)d.slowq_cap);
         A(&d.slowq_n, 1);
@@ -1197,7 +1203,7 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
     int64_t bytes = n * S * 24 + (S + 1) * 1024 * 8 + 64;
     if(precision == SFX_PREC_SPLIT)
         bytes += n * 32 + n * 16 * (sfx_split_grad_vec4((int)D) + sfx_split_dwdt_vec4((int)D)) +
-                 F * 32 +
+                 F * 8 * split_dq_doubles((int)D) +
                  4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 28;
     else {
         auto rec = [&](int what) { return (int64_t)sfx_fp64_record_bytes((int)D, what); };

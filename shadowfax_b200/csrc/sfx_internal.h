@@ -91,8 +91,8 @@ struct sfx_dmesh {
      * an [dim][F] FP64 area vector A n (n from x_L to x_R), for the pressure
      *     force, so that the forces on a cell cancel to FP64 round-off in a
      *     uniform region;
-     * dq [4 F]: the limited dQ received by the left cell, 32 bytes per face
-     *     (store_dq, sfx_split.cu). */
+     * dq [4 F] (2D [3 F]): the limited dQ received by the left cell, 32 (24)
+     *     bytes per face (store_dq, sfx_split.cu). */
     float4* fg;
     float* fr;
     float4* cw;
