@@ -475,17 +475,6 @@ __global__ void __launch_bounds__(128) k_gradients(sfx_dmesh m, double gamma) {
     }
 }
 
-/* a / b from y = 1 / b (rounded to nearest): two corrections of a y, the
- * second of them with an exact residual of a quotient within an ulp, give the
- * correctly rounded quotient (P. Markstein, "Computation of elementary
- * functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990)
- * where nothing under- or overflows; a zero quotient may lose its sign */
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-    double q = a * y;
-    q = __fma_rn(__fma_rn(-q, b, a), y, q);
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
-}
-
 /* 0, or a normal size between 2^-300 and 2^300: with plain_size lengths,
  * every dividend of the gradient is then 0 or between 2^-560 and 2^520 */
 __device__ __forceinline__ bool plain_state(double x) {
@@ -509,7 +498,7 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src) {
  * face sees the same c and |r| and the opposite r (the mesh qualifies when
  * every local face's right position is its right cell's position, gshare).
  * Bound by FP64 issue and the latency of the gathers.  The 2 D divisions by
- * |r| use the face's stored reciprocal (div_by: 5 operations; a zero term's
+ * |r| use the face's stored reciprocal (sfx_div_by: 5 operations; a zero term's
  * sign cannot change a sum that starts at +0), the limiter's minimum over the
  * faces takes two divisions per cell (sfx_limiter_min), and the face's
  * geometry and the neighbour's state come through a shared-memory ring filled
@@ -621,8 +610,8 @@ __global__ void __launch_bounds__(kGradBlock, D == 3 ? 5 : 6) k_grad_cells(sfx_d
         if(plain && y != 0.) {
 #pragma unroll
             for(int l = 0; l < D; ++l)
-                delta[l] = delta[l] + A * (div_by(dW * g[3 + l], rn, y) -
-                                           div_by(sW * g[3 + D + l], rn, y));
+                delta[l] = delta[l] + A * (sfx_div_by(dW * g[3 + l], rn, y) -
+                                           sfx_div_by(sW * g[3 + D + l], rn, y));
         } else {
 #pragma unroll
             for(int l = 0; l < D; ++l)
@@ -1818,7 +1807,7 @@ __global__ void __launch_bounds__(kExactBlock, 2)
  * failure of this step's other faces does not end it: the record names the
  * lowest failing face, and that one may be listed (after a failure of an
  * earlier step or phase the list is empty). */
-constexpr int kListedBlock = 128, kListedBlocks = 4 * 148;
+constexpr int kListedBlock = 128, kListedBlocks = 4 * kSfxSMs;
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(kListedBlock)
@@ -1842,9 +1831,9 @@ __global__ void __launch_bounds__(kListedBlock)
 /* One thread per cell: the cell's faces in ascending face order (aidx), the
  * order in which the reference's face loop adds them (a face of zero area, or
  * between two inactive cells, holds zeros, which change no sum), then Q and
- * get_W.  Bound by the latency of the dQ gathers: a face's dQ is one record
- * of 2 or 3 16-byte loads (field-major dQ touched a 32-byte sector per
- * double), U faces' loads in flight.  65,537 cells 3D 33 -> 23 us, 150,001
+ * get_W.  Bound by the latency of the dQ gathers: a face's dQ is one record, a
+ * 32-byte load in 2D and three of 16 bytes in 3D (field-major dQ touches a
+ * 32-byte sector per double), U faces' loads in flight.  65,537 cells 3D 33 -> 23 us, 150,001
  * cells 2D 20.5 -> 19.1 us (event-timed); one lane per cell and variable took
  * 23 and 24 us. */
 constexpr int kApplyBlock = 128;
@@ -2317,9 +2306,6 @@ int sfx_fp64_timestep_bins(const sfx_dmesh* m, double gamma, double cfl, uint64_
     return cudaGetLastError() == cudaSuccess ? SFX_OK : SFX_ERR_CUDA;
 }
 
-namespace {
-}  // namespace
-
 int sfx_fp64_move_velocities(const sfx_dmesh* m, double gamma, double dt, int periodic,
                              int faces, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
@@ -2345,9 +2331,6 @@ int sfx_fp64_drift(const sfx_dmesh* m, double dt, void* stream) {
     sfx_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? SFX_OK : SFX_ERR_CUDA;
 }
-
-namespace {
-}  // namespace
 
 void sfx_solver_params_init(sfx_solver_params* p, int kind, double g, double tol,
                             double cutoff) {
@@ -2466,7 +2449,7 @@ static int launch_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double 
         /* one wave of blocks waits for its longest face whichever way it is
          * sorted, and a second launch would add to that: the list from two
          * blocks on every SM */
-        const int list = nf > 2 * 148 * kExactBlock;
+        const int list = nf > 2 * kSfxSMs * kExactBlock;
         k_faces_exact<D, MODE><<<grid_for(nf, kExactBlock), kExactBlock, 0, s>>>(
                 *m, *sp, dt, write_branch, list);
         if(!list) return 1;

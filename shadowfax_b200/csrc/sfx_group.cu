@@ -199,7 +199,7 @@ extern "C" int sfx_group_step(sfx_group* g, int32_t nsteps, int32_t use_graph,
             int per_step = g->d_steps ? 1 : 0;
             for(int p = 0; p < 3; ++p) per_step += g->dev.blocks[p] > 0;
             /* the queued faces (both solvers: the exact solver's refused
-             * faces, HLLC's non-finite FP32 fluxes) */
+             * faces, HLLC's vacuum cases and non-finite FP32 fluxes) */
             if(g->dev.blocks[1] > 0) per_step += 1;
             sfx_count_launches(per_step * nsteps);
         }
@@ -309,8 +309,9 @@ extern "C" int sfx_group_tune(sfx_group* g, int32_t reps, int32_t* lanes_out) {
     for(int c = 0; c < 5 && !rc; ++c) {
         rc = sfx_group_set_lanes(g, cand[c]);
         if(rc) break;
-        /* timed on the gradient kernel, which only reads the states (the
-         * update kernel shares the setting); one untimed launch, then reps */
+        /* timed on the gradient kernel, which only reads the states (the update
+         * kernel takes a quarter of the lanes, at least one); one untimed
+         * launch, then reps */
         for(int r = 0; r <= reps && !rc; ++r) {
             if(r == 1) cudaEventRecord(e0, s);
             rc = sfx_split_group_phase(&g->dev, 0, sp, s);

@@ -186,6 +186,9 @@ struct sfx_solver_params {
 void sfx_solver_params_init(sfx_solver_params* p, int kind, double gamma,
                             double tol, double cutoff);
 
+/* streaming multiprocessors of a B200, the one device these kernels are built for */
+constexpr int kSfxSMs = 148;
+
 /* FP64 kernels (sfx_fp64.cu) */
 enum { SFX_REC_WS, SFX_REC_GREC, SFX_REC_DQ, SFX_REC_GGEO, SFX_REC_FGEO };
 int sfx_fp64_record_bytes(int dim, int what); /* bytes of one record */

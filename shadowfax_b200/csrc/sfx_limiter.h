@@ -1,7 +1,10 @@
 /*
+ * The divisions of the plain-FP64 gradients, for device code and for host-side
+ * tests of the same source: a quotient by a stored reciprocal (sfx_div_by) and
+ * the slope limiter's quotients.
+ *
  * The slope limiter's quotient for one face, plain-FP64 gradients
- * (VorCell::estimate_gradient, src/VorCell.cpp:486-530), for device code and
- * for host-side tests of the same source.
+ * (VorCell::estimate_gradient, src/VorCell.cpp:486-530).
  *
  * The reference forms q1 = a / dp and q2 = b / dp with a = W_max - W and
  * b = W_min - W (q1 = q2 = 1 where dp == 0) and keeps mx = (q1 < q2) ? q2 : q1.
@@ -22,6 +25,17 @@
 #else
 #define SFX_LIM_HD static inline
 #endif
+
+/* a / b from y = 1 / b (rounded to nearest): two corrections of a y, the
+ * second of them with an exact residual of a quotient within an ulp, give the
+ * correctly rounded quotient (P. Markstein, "Computation of elementary
+ * functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990)
+ * where nothing under- or overflows; a zero quotient may lose its sign */
+SFX_LIM_HD double sfx_div_by(double a, double b, double y) {
+    double q = a * y;
+    q = fma(fma(-q, b, a), y, q);
+    return fma(fma(-q, b, a), y, q);
+}
 
 /* the reference's two divisions and select */
 SFX_LIM_HD double sfx_limiter_ratio_ref(double a, double b, double dp) {

@@ -41,21 +41,21 @@ constexpr unsigned kRightBit = 0x80000000u;
 /* faces per lane whose midpoint - centroid the gradient kernel keeps in
  * shared memory between its two passes */
 constexpr int kGradSlots = 6;
-/* exact solver: "this face needs Brent's method", queued instead of solved */
+/* exact solver: fast_root did not settle the face, which is queued instead */
 constexpr int kDefer = 0x7f;
-/* how the exact solver treats a face whose p* needs a bracketing search:
- * search in this lane, or queue the face (kDefer) for a follow-up launch */
+/* a face launch leaves what it cannot settle in FP32 to the queue
+ * (kSolveDefer); the queue's launch solves it in FP64 (kSolveInline) */
 constexpr int kSolveInline = 0, kSolveDefer = 1;
-/* blocks of the group's queued-face launch (two waves of 128-thread blocks
- * on 148 SMs; the launch strides over each member's queue) */
-constexpr int kSlowGroupBlocks = 296;
-/* 2D HLLC face kernel: above one wave of 64-register blocks (four per SM on
- * 148 SMs) variant 0 takes the 48-register kernel, five blocks per SM, whose
+/* blocks of the group's queued-face launch (two 128-thread blocks per SM; the
+ * launch strides over each member's queue) */
+constexpr int kSlowGroupBlocks = 2 * kSfxSMs;
+/* 2D HLLC face kernel: above one wave of 64-register blocks (four per SM)
+ * variant 0 takes the 48-register kernel, five blocks per SM, whose
  * gathers have more warps to hide in: 12.0 us against 12.5 at 300,000 faces,
  * 36.6 against 39.8 at 1.2 million, 123 against 138 at 4.8 million; below a
  * wave (60,000 faces) 5.6 against 5.4.  In 3D it is slower at every size (35
  * against 31.5 us at 800,000 faces). */
-constexpr int kOneWaveHllc2d = 4 * 148;
+constexpr int kOneWaveHllc2d = 4 * kSfxSMs;
 
 __device__ __forceinline__ void report_face(sfx_dev_error* e, int f, int st) {
     atomicMin(&e->face_key, ((unsigned long long)(unsigned)f << 8) | (unsigned)st);
@@ -477,11 +477,6 @@ struct SFlux {
  * takes every LPC-th of the cell's faces, and the group combines its partial
  * sums / maxima / minima with shuffles.  All loads of a group are independent,
  * so a warp keeps 32 face gathers in flight instead of one. */
-template <int D>
-struct Lanes {
-    static constexpr int value = D == 3 ? 16 : 8;
-};
-
 template <int LPC>
 __device__ __forceinline__ float seg_sum(float v) {
 #pragma unroll
@@ -989,7 +984,7 @@ __device__ __noinline__ SFlux<D> shllc_fp64(float g, FaceStates<D> in, bool refl
 }
 
 /* HLLC on the predicted FP32 states.  kSolveDefer: in FP32; false for a
- * vacuum case or when that flux is not finite, and the face is then queued for the FP64 solve
+ * vacuum case or when that flux is not finite: the face is queued for the FP64 solve
  * (k_group_sfaces_slow).  kSolveInline: in FP64 (the queued faces).  The
  * FP64 solve stays out of the FP32 kernel: a call from it, or its code
  * inline, costs that kernel a stack frame and spills on every face. */
@@ -1064,19 +1059,6 @@ struct XS {
     }
 };
 
-/* p* for the face kernel: Newton's method in FP32 from the reference's
- * initial guess, then one FP64 Newton step from the FP32 root.  The face's
- * states are FP32 values; the FP32 root is within about 1e-6 of p*, and the
- * FP64 step (quadratic convergence) takes it to about 1e-12, inside the
- * iteration's 1e-8 tolerance.  f_K and the rarefaction powers z_K at the
- * final pressure are the FP64 values at the FP32 root carried along the
- * step to first order (error of the order of the step squared).  Two FP64
- * powers at most instead of one per FP64 iteration plus two per face.
- * Returns false, and the FP64 iteration runs from the start, outside the
- * range where FP32 is safe, when the FP32 iteration does not converge or
- * takes a Newton step to (nearly) zero pressure (where the reference's
- * iteration can stop at p = 0), when the FP64 step is not small, or when it
- * moves a side between shock and rarefaction. */
 /* x^(1/5) for normal x > 0 without a division or a power: w ~ x^(-1/5) from
  * the FP32 hardware log2/exp2, two Newton steps for w^-5 = x, w <- w (6 -
  * x w^5) / 5 (quadratic convergence from ~1e-7 to below 1e-16), then
@@ -1115,15 +1097,16 @@ __device__ __forceinline__ void side64(const sfx_solver_params& s, double p, dou
 }
 
 /* p* for the face kernel: Newton's method in FP32 from the reference's
- * initial guess, then one FP64 Newton step from the FP32 root.  The face's
- * states are FP32 values; the FP32 root is within about 1e-6 of p*, and the
- * FP64 step (quadratic convergence) takes it to about 1e-12, inside the
- * iteration's 1e-8 tolerance.  f_K and the rarefaction powers z_K at the
- * final pressure are the FP64 values at the FP32 root carried along the
- * step to first order (error of the order of the step squared).  Two FP64
- * powers at most instead of one per FP64 iteration plus two per face.
- * Returns false, and the FP64 iteration runs from the start, outside the
- * range where FP32 is safe, when the FP32 iteration takes a Newton step to
+ * initial guess, then FP64 Newton steps (at most four, usually one) from the
+ * FP32 root.  The face's states are FP32 values; the FP32 root is within about
+ * 1e-6 of p* where FP32 resolves f, and a last FP64 step of at most 1e-5 p
+ * (quadratic convergence) leaves about 1e-10, inside the iteration's 1e-8
+ * tolerance.  f_K and the rarefaction powers z_K at the final pressure are the
+ * FP64 values before that step carried along it to first order (error of the
+ * order of the step squared).  Two FP64 powers at most per step, usually two in
+ * all, instead of one per FP64 iteration plus two per face.
+ * Returns false, and the queue's FP64 iteration runs from the start, outside
+ * the range where FP32 is safe, when the FP32 iteration takes a Newton step to
  * (nearly) zero pressure where the reference's can stop at p = 0, or when four
  * FP64 steps leave no small step that keeps each side's wave. */
 template <bool G53 = false>
@@ -1217,7 +1200,7 @@ __device__ __forceinline__ bool fast_root(const sfx_solver_params& s, double rL,
     }
 }
 
-template <int D, int MODE>
+template <int D>
 __device__ int sexact(const sfx_solver_params& s, double* WL, double* WR, const double* n,
                       bool reflective, double* sol) {
     constexpr int S = D + 2;
@@ -1271,8 +1254,6 @@ __device__ int sexact(const sfx_solver_params& s, double* WL, double* WR, const 
         XS<D> x{s};
         const double pL = WL[D + 1], pR = WR[D + 1];
         double p = 0., fL = 0., zL = 0., fR = 0., zR = 0.;
-        if(MODE != kSolveDefer ||
-           !fast_root(s, WL[0], pL, WR[0], pR, aL, aR, vL, vR, p, fL, fR, zL, zR)) {
         /* p_K^-e (e = (g-1)/(2g)): (p/p_K)^e = p^e p_K^-e, one pow per
          * evaluation for both sides (0: not finite, pow of the ratio) */
         double iL = xpow(pL, -s.gm1d2g), iR = xpow(pR, -s.gm1d2g);
@@ -1342,7 +1323,6 @@ __device__ int sexact(const sfx_solver_params& s, double* WL, double* WR, const 
                 }
             }
             if(!conv && fg > 0.) {
-                if(MODE == kSolveDefer) return kDefer;
                 /* f(0) < 0 < f(pg).  The reference runs Brent's method on
                  * [0, pg] (ExactRiemannSolver.cpp:462-546), tens of
                  * iterations in one lane.  f is increasing and concave, so a
@@ -1381,7 +1361,6 @@ __device__ int sexact(const sfx_solver_params& s, double* WL, double* WR, const 
         if(!at_p) {
             double t0, t1;
             eval(p, t0, t1);
-        }
         }
         const double u = 0.5 * (vL + vR) + 0.5 * (fR - fL);
         if(u < 0.) {
@@ -1779,7 +1758,7 @@ __device__ __forceinline__ LeftTile<D> stage_left_cells(const sfx_dmesh& m, int 
 }
 
 /* one face; true when the face is left for the queued-face kernel (HLLC in
- * kSolveDefer mode whose FP32 flux is not finite) */
+ * kSolveDefer mode: a vacuum case, or an FP32 flux that is not finite) */
 template <int D, int SOLVER, int MODE, bool STORED_DW = SOLVER != SFX_SOLVER_HLLC,
           bool MOVING = false, bool TILE = false>
 __device__ __forceinline__ bool sfaces_body(const sfx_dmesh& m, const sfx_solver_params& sp,
@@ -1810,7 +1789,7 @@ __device__ __forceinline__ bool sfaces_body(const sfx_dmesh& m, const sfx_solver
             dWR[k] = w.WR[k];
         }
         static_assert(MODE == kSolveInline, "queued faces come from k_group_sfaces_exact");
-        status = sexact<D, MODE>(sp, dWL, dWR, dn, w.mirror, h);
+        status = sexact<D>(sp, dWL, dWR, dn, w.mirror, h);
         exact_flux<D>(sp.gamma, h, dn, w.v, MOVING, F);
     }
     face_dq<D>(m, f, w, F, status);
@@ -1821,19 +1800,19 @@ __device__ __forceinline__ bool sfaces_body(const sfx_dmesh& m, const sfx_solver
  * The exact face kernel works in three phases per block of 256 faces:
  *   1. every thread forms its face's predicted states (face_work) and
  *      classifies the face's wave pattern in FP32 from the signs of
- *      f(p_min) and f(p_max) (f increasing in p*): two rarefactions, two
- *      shocks, or a shock on the lower-pressure side and a rarefaction on the
- *      other (two classes, by which side that is).  Faces outside the range
- *      where the FP32 iteration is safe, and vacuum faces, go to the queue
+ *      f(p_min) and f(p_max) (f increasing in p*): two rarefactions (vacuum
+ *      faces too), two shocks, or a shock on the lower-pressure side and a
+ *      rarefaction on the other (two classes, by which side that is).  Faces
+ *      outside the range where the FP32 iteration is safe go to the queue
  *      solved by k_group_sfaces_slow;
  *   2. a counting sort of the block's faces by class (warp ballots, one scan
  *      of the 4 x 8 per-warp counts) through shared memory;
  *   3. thread t solves the block's t-th face in class order: p* by Newton in
- *      FP32 from the reference's guess plus one FP64 Newton step (fast_root),
- *      then the sampled half state in FP64.  A warp now takes one branch of
- *      the per-side shock/rarefaction code in every iteration.  A face whose
- *      FP32 iteration is refused, or whose state turns out to be a vacuum
- *      case in FP64, goes to the queue (warp-aggregated push).
+ *      FP32 from the reference's guess and up to four FP64 Newton steps
+ *      (fast_root), then the sampled half state in FP64; a face that is a
+ *      vacuum case in FP64 is sampled without p*.  A warp now takes one branch
+ *      of the per-side shock/rarefaction code in every iteration.  A face that
+ *      fast_root does not settle goes to the queue (warp-aggregated push).
  * Which thread solves a face changes nothing in its arithmetic, so reruns are
  * bitwise identical. */
 constexpr int kClassRR = 0, kClassSS = 1, kClassSR = 2, kClassRS = 3, kNClass = 4;
@@ -1875,8 +1854,8 @@ __device__ __forceinline__ int wave_class(const sfx_solver_params& s, const Face
 }
 
 /* phase 3: p* by fast_root and the sampled half state; kDefer when the face
- * needs the FP64 iteration or is a vacuum case, SFX_ERR_RIEMANN for an
- * unphysical half state, SFX_OK otherwise */
+ * needs the FP64 iteration, SFX_ERR_RIEMANN for an unphysical half state,
+ * SFX_OK otherwise */
 /* G53: gamma = 5/3, where the sampling's powers are integers in z_K or in
  * the fan's base: (p/p_K)^(1/g) = z_K^3, base^(2/(g-1)) = base^3,
  * base^(2g/(g-1)) = base^5 */
@@ -2294,8 +2273,9 @@ __global__ void __launch_bounds__(256, MINB)
 
 /* The queued faces of every member, one per thread.  Exact solver: the
  * FP64 iteration from the reference's guess (the monotone Newton search
- * where the reference runs Brent's method) and the vacuum cases.  HLLC: the
- * FP64 solve of faces whose FP32 flux was not finite.  Each block reads
+ * where the reference runs Brent's method), vacuum cases among states outside
+ * the FP32 range included.  HLLC: the FP64 solve of the vacuum cases and of faces
+ * whose FP32 flux was not finite.  Each block reads
  * the members' queue lengths (kSlowChunk members at a time, in parallel),
  * forms their prefix sums in shared memory and strides over the flattened
  * list, finding a slot's member by binary search: no thread walks the
@@ -2448,7 +2428,8 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
                 k_group_sfaces_slow<D><<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, g->pre, nm, *sp);
                 sfx_count_launches(1);
             } else {
-                /* HLLC; then the faces whose FP32 flux was not finite, in FP64 */
+                /* HLLC; then the vacuum cases and the faces whose FP32 flux was not
+                 * finite, in FP64 */
                 const int v = sfx_split_face_variant_kernel(sp, g->face_variant);
                 if(v == 2) {
                     k_group_sfaces<D, SFX_SOLVER_HLLC, 4, true><<<g->blocks[1], 256, 0, s>>>(
