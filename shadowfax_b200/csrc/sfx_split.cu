@@ -773,12 +773,19 @@ struct RT<float> {
     static __device__ __forceinline__ float sqrt_(float x) { return sqrt32(x); }
     static __device__ __forceinline__ float rcp_(float x) { return rcp32(x); }
     static __device__ __forceinline__ float max_(float x, float y) { return fmaxf(x, y); }
+    static __device__ __forceinline__ float pow_(float x, float y) { return powf(x, y); }
+    /* x / y to nearly half an ulp: one correction */
+    static __device__ __forceinline__ float div_(float x, float y) {
+        const float i = rcp32(y), q = x * i;
+        return fmaf(fmaf(-q, y, x), i, q);
+    }
 };
 template <>
 struct RT<double> {
     static __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
     static __device__ __forceinline__ double rcp_(double x) { return 1. / x; }
     static __device__ __forceinline__ double pow_(double x, double y) { return pow(x, y); }
+    static __device__ __forceinline__ double div_(double x, double y) { return x / y; }
     static __device__ __forceinline__ double max_(double x, double y) { return fmax(x, y); }
 };
 
@@ -787,10 +794,8 @@ struct TFlux {
     T m, mv[D], P, E;
 };
 
-/* VAC: with the vacuum cases; without them (the FP32 kernel, which carries no
- * power function then) false, for a face to be solved in FP64 */
-template <int D, typename T, bool VAC>
-__device__ __forceinline__ bool thllc(T g, const T* WL, const T* WRin, const T* n,
+template <int D, typename T>
+__device__ __forceinline__ void thllc(T g, const T* WL, const T* WRin, const T* n,
                                       bool reflective, TFlux<D, T>& F) {
     using R = RT<T>;
     constexpr int S = D + 2;
@@ -800,7 +805,7 @@ __device__ __forceinline__ bool thllc(T g, const T* WL, const T* WRin, const T* 
     F.E = zero;
 #pragma unroll
     for(int l = 0; l < D; ++l) F.mv[l] = zero;
-    if(WL[0] == zero && (reflective || WRin[0] == zero)) return true;
+    if(WL[0] == zero && (reflective || WRin[0] == zero)) return;
     /* the reflective right state is the left state with its normal velocity
      * reversed (only u_R enters below).  States are selected by value, element
      * by element: a select between two arrays' addresses would keep both
@@ -821,113 +826,62 @@ __device__ __forceinline__ bool thllc(T g, const T* WL, const T* WRin, const T* 
     const T irL = R::rcp_(WL[0]), irR = R::rcp_(WR[0]);
     const T aL = WL[0] != zero ? R::sqrt_(g * WL[D + 1] * irL) : zero;
     const T aR = WR[0] != zero ? R::sqrt_(g * WR[D + 1] * irR) : zero;
-    if(WL[0] == zero || WR[0] == zero || two * (aL + aR) / gm1 <= uR - uL) {
-        if constexpr(!VAC) {
-            return false;
-        } else {
-            /* exact vacuum solution at x/t = 0 */
-            T sol[S], vhalf = zero;
-            const T tdgp1 = two / (g + one), gm1dgp1 = gm1 / (g + one);
-            bool vac = false, fan = false;
-            bool sright = false; /* the sampled state is the right one */
-            if(WR[0] == zero) {
-                if(aL > uL) {
-                    if(uL + two * aL / gm1 > zero) {
-                        /* base > 0 in exact arithmetic on this branch */
-                        const T base = R::max_(zero, tdgp1 + gm1dgp1 / aL * uL);
-                        vhalf = tdgp1 * (aL + half * gm1 * uL) - uL;
-#pragma unroll
-                        for(int k = 0; k < S; ++k) sol[k] = WL[k];
-                        sol[0] = WL[0] * R::pow_(base, two / gm1);
-                        sol[D + 1] = WL[D + 1] * R::pow_(base, two * g / gm1);
-                        fan = true;
-                    } else {
-                        vac = true;
-                    }
-                }
-            } else if(WL[0] == zero) {
-                sright = true;
-                if(-uR < aR) {
-                    if(uR - two * aR / gm1 >= zero) {
-                        vac = true;
-                    } else {
-                        const T base = R::max_(zero, tdgp1 - gm1dgp1 / aR * uR);
-                        vhalf = tdgp1 * (-aR + half * gm1 * uR) - uR;
-#pragma unroll
-                        for(int k = 0; k < S; ++k) sol[k] = WR[k];
-                        sol[0] = WR[0] * R::pow_(base, two / gm1);
-                        sol[D + 1] = WR[D + 1] * R::pow_(base, two * g / gm1);
-                        fan = true;
-                    }
-                }
-            } else {
-                const T SR = uR - two * aR / gm1, SL = uL + two * aL / gm1;
-                if(SR > zero && SL < zero) {
-                    vac = true;
-                } else if(SL >= zero) {
-                    if(aL > uL) {
-                        const T base = R::max_(zero, tdgp1 + gm1dgp1 / aL * uL);
-                        vhalf = tdgp1 * (aL + half * gm1 * uL) - uL;
-#pragma unroll
-                        for(int k = 0; k < S; ++k) sol[k] = WL[k];
-                        sol[0] = WL[0] * R::pow_(base, two / gm1);
-                        sol[D + 1] = WL[D + 1] * R::pow_(base, two * g / gm1);
-                        fan = true;
-                    }
-                } else {
-                    sright = true;
-                    if(-uR < aR) {
-                        const T base = R::max_(zero, tdgp1 - gm1dgp1 / aR * uR);
-                        vhalf = tdgp1 * (-aR + half * gm1 * uR) - uR;
-#pragma unroll
-                        for(int k = 0; k < S; ++k) sol[k] = WR[k];
-                        sol[0] = WR[0] * R::pow_(base, two / gm1);
-                        sol[D + 1] = WR[D + 1] * R::pow_(base, two * g / gm1);
-                        fan = true;
-                    }
-                }
-            }
-            if(vac) return true;
-            if(!fan) {
-#pragma unroll
-                for(int k = 0; k < S; ++k) sol[k] = sright ? WR[k] : WL[k];
-            }
-#pragma unroll
-            for(int l = 0; l < D; ++l) sol[1 + l] += vhalf * n[l];
-            if(sol[0] == zero) return true;
-            T vsol = zero, v2 = zero;
-#pragma unroll
-            for(int l = 0; l < D; ++l) {
-                vsol += sol[1 + l] * n[l];
-                v2 += sol[1 + l] * sol[1 + l];
-            }
-            F.m = sol[0] * vsol;
-#pragma unroll
-            for(int l = 0; l < D; ++l) F.mv[l] = F.m * sol[1 + l];
-            F.P = sol[D + 1];
-            const T e = sol[D + 1] / gm1 / sol[0] + half * v2;
-            F.E = (sol[0] * e + sol[D + 1]) * vsol;
-            return true;
-        }
+    const bool vac = WL[0] == zero || WR[0] == zero || two * (aL + aR) / gm1 <= uR - uL;
+    bool left, star;
+    T SL = zero, SR = zero, Sstar = zero, mL = zero, mR = zero;
+    if(vac) {
+        left = WL[0] != zero && (WR[0] == zero || uL + two * aL / gm1 >= zero);
+        star = false;
+    } else {
+        const T rhobar = half * (WL[0] + WR[0]);
+        const T abar = half * (aL + aR);
+        const T pstar = R::max_(zero, half * (WL[D + 1] + WR[D + 1]) -
+                                              half * (uR - uL) * rhobar * abar);
+        const T gp = half * (g + one) / g;
+        /* w_K = a_K q_K = |S_K - u_K| */
+        const T wL = pstar > WL[D + 1]
+                             ? R::sqrt_(g * (WL[D + 1] + gp * (pstar - WL[D + 1])) * irL)
+                             : aL;
+        const T wR = pstar > WR[D + 1]
+                             ? R::sqrt_(g * (WR[D + 1] + gp * (pstar - WR[D + 1])) * irR)
+                             : aR;
+        SL = uL - wL;
+        SR = uR + wR;
+        mL = WL[0] * wL;
+        mR = WR[0] * wR;
+        Sstar = (WL[D + 1] - WR[D + 1] + mL * uL + mR * uR) * R::rcp_(mL + mR);
+        left = Sstar >= zero;
+        star = left ? (SL < zero) : (SR > zero);
     }
-    const T rhobar = half * (WL[0] + WR[0]);
-    const T abar = half * (aL + aR);
-    const T pstar = R::max_(zero, half * (WL[D + 1] + WR[D + 1]) - half * (uR - uL) * rhobar * abar);
-    const T gp = half * (g + one) / g;
-    /* w_K = a_K q_K = |S_K - u_K| */
-    const T wL = pstar > WL[D + 1] ? R::sqrt_(g * (WL[D + 1] + gp * (pstar - WL[D + 1])) * irL)
-                                   : aL;
-    const T wR = pstar > WR[D + 1] ? R::sqrt_(g * (WR[D + 1] + gp * (pstar - WR[D + 1])) * irR)
-                                   : aR;
-    const T SL = uL - wL;
-    const T SR = uR + wR;
-    const T mL = WL[0] * wL, mR = WR[0] * wR;
-    const T Sstar = (WL[D + 1] - WR[D + 1] + mL * uL + mR * uR) * R::rcp_(mL + mR);
-    const bool left = Sstar >= zero;
     T Wk[S];
 #pragma unroll
     for(int k = 0; k < S; ++k) Wk[k] = left ? WL[k] : WR[k];
-    const T uk = left ? uL : uR;
+    T uk = left ? uL : uR;
+    if(vac) {
+        /* the exact vacuum solution at x/t = 0 on the side that reaches it
+         * (HLLCRiemannSolver.cpp:44-156), the right one mirrored onto the left:
+         * the side's own state, its fan, or vacuum.  The fan's density and
+         * pressure are base^(2/(g-1)) and base^(2g/(g-1)) = that times base^2:
+         * one power (its cube at gamma = 5/3).  In this kernel, not in the queue,
+         * whose launch took 60 us however few faces it solved (its code is
+         * fetched for them alone): 450,000 faces in 2D, 3.4% and 40% of them
+         * vacuum, 89.5 and 103 -> 25.6 us; 530,000 in 3D 86 and 115 -> 31.8 us;
+         * without vacuum faces 57.5 -> 50.2 us (1.4 million, 2D), 85.2 -> 82.4
+         * (2.1 million, 3D). */
+        const T a = left ? aL : aR, v = left ? uL : -uR;
+        if(v < a) {
+            if(!(v + two * a / gm1 > zero)) return;
+            const T tdgp1 = two / (g + one);
+            const T base = R::max_(zero, tdgp1 + gm1 / (g + one) * R::div_(v, a));
+            const T z = g == T(5. / 3.) ? base * base * base : R::pow_(base, two / gm1);
+            const T uf = tdgp1 * (a + half * gm1 * v), shift = uf - v;
+            Wk[0] *= z;
+            Wk[D + 1] *= z * (base * base);
+#pragma unroll
+            for(int l = 0; l < D; ++l) Wk[1 + l] += (left ? shift : -shift) * n[l];
+            uk = left ? uf : -uf;
+        }
+    }
     const T Sk = left ? SL : SR;
     T v2 = zero;
 #pragma unroll
@@ -939,7 +893,7 @@ __device__ __forceinline__ bool thllc(T g, const T* WL, const T* WRin, const T* 
     T mk = Wk[0] * uk;
     F.P = Wk[D + 1];
     F.E = (re + Wk[D + 1]) * uk;
-    if(left ? (SL < zero) : (SR > zero)) {
+    if(star) {
         const T ds = Sstar - uk;
         const T i = R::rcp_(Sk - Sstar);
         const T Sfac = Sk * (left ? -mL : mR) * i;
@@ -950,7 +904,6 @@ __device__ __forceinline__ bool thllc(T g, const T* WL, const T* WRin, const T* 
     F.m = mk;
 #pragma unroll
     for(int l = 0; l < D; ++l) F.mv[l] = mk * Wk[1 + l];
-    return true;
 }
 
 __device__ __forceinline__ bool finite4(float a, float b, float c, float d) {
@@ -974,7 +927,7 @@ __device__ __noinline__ SFlux<D> shllc_fp64(float g, FaceStates<D> in, bool refl
     }
     for(int l = 0; l < D; ++l) dn[l] = in.n[l];
     TFlux<D, double> H;
-    thllc<D, double, true>((double)g, dL, dR, dn, reflective, H);
+    thllc<D, double>((double)g, dL, dR, dn, reflective, H);
     SFlux<D> F;
     F.m = (float)H.m;
     for(int l = 0; l < D; ++l) F.mv[l] = (float)H.mv[l];
@@ -984,7 +937,7 @@ __device__ __noinline__ SFlux<D> shllc_fp64(float g, FaceStates<D> in, bool refl
 }
 
 /* HLLC on the predicted FP32 states.  kSolveDefer: in FP32; false for a
- * vacuum case or when that flux is not finite: the face is queued for the FP64 solve
+ * when that flux is not finite, and the face is then queued for the FP64 solve
  * (k_group_sfaces_slow).  kSolveInline: in FP64 (the queued faces).  The
  * FP64 solve stays out of the FP32 kernel: a call from it, or its code
  * inline, costs that kernel a stack frame and spills on every face. */
@@ -1004,7 +957,7 @@ __device__ __forceinline__ bool shllc(float g, const float* WL, const float* WR,
         return true;
     }
     TFlux<D, float> G;
-    if(!thllc<D, float, false>(g, WL, WR, n, reflective, G)) return false;
+    thllc<D, float>(g, WL, WR, n, reflective, G);
     float mvs = 0.f;
 #pragma unroll
     for(int l = 0; l < D; ++l) mvs += G.mv[l];
@@ -1758,7 +1711,7 @@ __device__ __forceinline__ LeftTile<D> stage_left_cells(const sfx_dmesh& m, int 
 }
 
 /* one face; true when the face is left for the queued-face kernel (HLLC in
- * kSolveDefer mode: a vacuum case, or an FP32 flux that is not finite) */
+ * kSolveDefer mode whose FP32 flux is not finite) */
 template <int D, int SOLVER, int MODE, bool STORED_DW = SOLVER != SFX_SOLVER_HLLC,
           bool MOVING = false, bool TILE = false>
 __device__ __forceinline__ bool sfaces_body(const sfx_dmesh& m, const sfx_solver_params& sp,
@@ -2274,8 +2227,8 @@ __global__ void __launch_bounds__(256, MINB)
 /* The queued faces of every member, one per thread.  Exact solver: the
  * FP64 iteration from the reference's guess (the monotone Newton search
  * where the reference runs Brent's method), vacuum cases among states outside
- * the FP32 range included.  HLLC: the FP64 solve of the vacuum cases and of faces
- * whose FP32 flux was not finite.  Each block reads
+ * the FP32 range included.  HLLC: the FP64 solve of faces whose FP32 flux was not
+ * finite.  Each block reads
  * the members' queue lengths (kSlowChunk members at a time, in parallel),
  * forms their prefix sums in shared memory and strides over the flattened
  * list, finding a slot's member by binary search: no thread walks the
@@ -2428,8 +2381,7 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
                 k_group_sfaces_slow<D><<<kSlowGroupBlocks, kSlowBlock, 0, s>>>(g->tab, g->pre, nm, *sp);
                 sfx_count_launches(1);
             } else {
-                /* HLLC; then the vacuum cases and the faces whose FP32 flux was not
-                 * finite, in FP64 */
+                /* HLLC; then the faces whose FP32 flux was not finite, in FP64 */
                 const int v = sfx_split_face_variant_kernel(sp, g->face_variant);
                 if(v == 2) {
                     k_group_sfaces<D, SFX_SOLVER_HLLC, 4, true><<<g->blocks[1], 256, 0, s>>>(
