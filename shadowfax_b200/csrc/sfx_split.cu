@@ -50,11 +50,11 @@ constexpr int kSolveInline = 0, kSolveDefer = 1;
  * launch strides over each member's queue) */
 constexpr int kSlowGroupBlocks = 2 * kSfxSMs;
 /* 2D HLLC face kernel: above one wave of 64-register blocks (four per SM)
- * variant 0 takes the 48-register kernel, five blocks per SM, whose
- * gathers have more warps to hide in: 12.0 us against 12.5 at 300,000 faces,
- * 36.6 against 39.8 at 1.2 million, 123 against 138 at 4.8 million; below a
- * wave (60,000 faces) 5.6 against 5.4.  In 3D it is slower at every size (35
- * against 31.5 us at 800,000 faces). */
+ * variant 0 takes the 48-register kernel, five blocks per SM, whose gathers have
+ * more warps to hide in (face phase, both its launches): 17.4 us with either at
+ * 166,000 faces, 44.9 against 48.1 at 1.2 million, 87.4 against 97.3 at 3.0
+ * million; below a wave (121,000 faces) 16.4 against 15.2.  In 3D it is slower
+ * at every size (85.1 against 81.9 us at 2.1 million faces). */
 constexpr int kOneWaveHllc2d = 4 * kSfxSMs;
 
 __device__ __forceinline__ void report_face(sfx_dev_error* e, int f, int st) {
