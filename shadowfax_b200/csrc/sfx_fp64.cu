@@ -1945,6 +1945,19 @@ __global__ void __launch_bounds__(256) k_to_rows(const double* in, int64_t n, in
     for(int k = 0; k < w; ++k) rows[i * w + k] = in[k * n + i];
 }
 
+/* rows [count][w] from (IN: to) an array with element (i, k) at a[i * rs + k * cs] */
+template <bool IN>
+__global__ void __launch_bounds__(256) k_strided_rows(double* a, int64_t rs, int64_t cs,
+                                                      int64_t count, int w, double* rows) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(t >= count * w) return;
+    const int64_t i = t / w, k = t - i * w;
+    if(IN)
+        a[i * rs + k * cs] = rows[t];
+    else
+        rows[t] = a[i * rs + k * cs];
+}
+
 /* Q = get_Q(V, W): ExactRiemannSolver.cpp:776-804 / HLLCRiemannSolver.cpp:471-483 */
 template <int D>
 __global__ void k_init_Q(sfx_dmesh m, double gamma, int kind, const double* rows) {
@@ -2371,6 +2384,18 @@ int sfx_from_rows(const double* rows, int64_t n, int w, double* out, void* strea
 int sfx_to_rows(const double* in, int64_t n, int w, double* rows, void* stream) {
     if(n == 0) return SFX_OK;
     k_to_rows<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(in, n, w, rows);
+    sfx_count_launches(1);
+    return cuda_status(cudaGetLastError());
+}
+
+int sfx_strided_rows(double* a, int64_t rs, int64_t cs, int64_t count, int w, double* rows, int in,
+                     void* stream) {
+    if(count == 0) return SFX_OK;
+    const int G = grid_for(count * w, 256);
+    if(in)
+        k_strided_rows<true><<<G, 256, 0, (cudaStream_t)stream>>>(a, rs, cs, count, w, rows);
+    else
+        k_strided_rows<false><<<G, 256, 0, (cudaStream_t)stream>>>(a, rs, cs, count, w, rows);
     sfx_count_launches(1);
     return cuda_status(cudaGetLastError());
 }

@@ -53,7 +53,8 @@ struct sfx_dmesh {
     double* rpos;   /* [dim][F]  */
     double* vel;    /* [dim][F] or NULL */
     double* dQf;    /* limited dQ received by the left cell: plain-FP64 meshes [F] records
-                       (sfx_fp64.cu), otherwise [S][F] */
+                       (sfx_fp64.cu), without records [S][F]; split meshes rows [F][S] on
+                       their way to the host */
     /* plain-FP64 meshes: records of the cells' states and of their gradients
      * and dW/dt, and of the faces' gradient and flux geometry (sfx_fp64.cu).
      * ws == NULL: field-major arrays, caller-owned or of a mesh whose records did
@@ -208,6 +209,9 @@ int sfx_fp64_init_Q(const sfx_dmesh* m, const sfx_solver_params* sp, const doubl
 /* rows [n][w] <-> field-major [w][n], device arrays */
 int sfx_from_rows(const double* rows, int64_t n, int w, double* out, void* stream);
 int sfx_to_rows(const double* in, int64_t n, int w, double* rows, void* stream);
+/* rows [count][w] from (in: to) a device array with element (i, k) at a[i * rs + k * cs] */
+int sfx_strided_rows(double* a, int64_t rs, int64_t cs, int64_t count, int w, double* rows, int in,
+                     void* stream);
 /* totals of Q, and the error record after them: host_out[S + 2] (waits) */
 int sfx_fp64_totals(const sfx_dmesh* m, double* host_out, void* stream);
 /* halo records [count][S + 1] (W, then the mass Q[0]) of the listed cells */
@@ -241,7 +245,7 @@ int sfx_split_load_state(const sfx_dmesh* m, void* stream);
 int sfx_split_export_W(const sfx_dmesh* m, void* stream);
 /* the same as rows [n][S], for downloads */
 int sfx_split_W_rows(const sfx_dmesh* m, double* rows, void* stream);
-/* per-face dQ (FP32) widened into dQf (FP64 SoA), for parity checks */
+/* per-face dQ widened into dQf as rows [F][S], for parity checks */
 int sfx_split_export_dQ(const sfx_dmesh* m, void* stream);
 /* kernel launch counter behind sfx_launch_count (sfx_api.cu).  Launches made
  * while the calling thread captures a CUDA graph are not counted (the

@@ -462,7 +462,7 @@ __global__ void k_export_dQ(sfx_dmesh m) {
     if(f >= m.n_faces) return;
     double v[D + 2];
     load_dq<D>(m, f, v);
-    for(int k = 0; k < D + 2; ++k) m.dQf[(size_t)k * m.n_faces + f] = v[k];
+    for(int k = 0; k < D + 2; ++k) m.dQf[(size_t)f * (D + 2) + k] = v[k];
 }
 
 /* face flux split as: mass m, momentum m v + P n, energy E (the momentum's
