@@ -245,9 +245,26 @@ struct Carver {
     }
 };
 
-/* doubles of the staging rows: a state, and one row of gradients at least */
-size_t stage_doubles(const sfx_dmesh& d) {
-    return (size_t)std::max(d.n_cells, d.dim) * d.S;
+/* The staging rows: two states, or one and a row of gradients.  Plain FP64: in
+ * dQf when that is large enough (dq doubles), an array otherwise; split: one
+ * state in an array, the second in dq, where a state on its way in may go.
+ * stage_doubles: of the array (0: in dQf). */
+size_t stage_doubles(int64_t n, int dim, bool split, size_t dq) {
+    const size_t ns = (size_t)n * (dim + 2), row = (size_t)dim * (dim + 2);
+    if(split) return dq >= ns ? ns : 2 * ns;
+    return dq >= std::max(2 * ns, row) ? 0 : std::max(2 * ns, row);
+}
+
+void add_stage(Carver& arrays, sfx_dmesh& d, bool split, size_t dq) {
+    d.stage = d.stage2 = nullptr;
+    const size_t count = stage_doubles(d.n_cells, d.dim, split, dq);
+    if(count) arrays.add(&d.stage, count);
+}
+
+void set_stage(sfx_dmesh& d, bool split, size_t dq) {
+    const size_t ns = (size_t)d.n_cells * d.S;
+    if(!d.stage) d.stage = d.dQf;
+    d.stage2 = split && dq >= ns ? d.dq : d.stage + ns;
 }
 
 /* a plain-FP64 mesh's state and per-step scratch: the pass's records, or without
@@ -264,8 +281,22 @@ void add_fp64_state(Carver& arrays, sfx_dmesh& d, bool records) {
     arrays.add(&d.ws, n * rec_doubles(d.dim, SFX_REC_WS));
     arrays.add(&d.grec, n * rec_doubles(d.dim, SFX_REC_GREC));
     arrays.add(&d.dQf, F * rec_doubles(d.dim, SFX_REC_DQ));
-    arrays.add(&d.listed, F);
+    arrays.add(&d.listed, (size_t)sfx_fp64_list_room(F));
     arrays.add(&d.listed_n, 1);
+}
+
+/* doubles of a mesh's dQ scratch */
+size_t dq_doubles(const sfx_dmesh& d, bool split, bool records) {
+    const size_t F = (size_t)d.n_faces;
+    return F * (split ? split_dq_doubles(d.dim)
+                      : records ? rec_doubles(d.dim, SFX_REC_DQ) : (size_t)d.S);
+}
+
+/* rows of gradients that fit in a plain-FP64 mesh's staging rows */
+int64_t gradient_rows(const sfx_dmesh& d) {
+    const size_t dq = dq_doubles(d, false, d.ws != nullptr);
+    const size_t held = stage_doubles(d.n_cells, d.dim, false, dq);
+    return (int64_t)((held ? held : dq) / ((size_t)d.dim * d.S));
 }
 
 /* the arrays that add(arrays, records) names: with the plain-FP64 records, or,
@@ -351,7 +382,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     sfx_dmesh& d = m->d;
     const int64_t n = d.n_cells, F = d.n_faces;
     const int S = d.S, dim = d.dim;
-    d.W = d.Q = d.stage = d.grad = d.dQf = d.ws = d.grec = nullptr;
+    d.W = d.Q = d.grad = d.dQf = d.ws = d.grec = nullptr;
     d.listed = d.listed_n = nullptr;
     d.branch = nullptr;
     d.err = nullptr;
@@ -378,7 +409,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
         auto A = [&](auto** p, size_t c) { arrays.add(p, c); };
         A(&d.W, n * S);
         A(&d.Q, n * S);
-        A(&d.stage, stage_doubles(d));
+        add_stage(arrays, d, split, dq_doubles(d, split, records));
         A(&d.err, 1);
         A(&d.totals_scratch, (size_t)(S + 1) * 1024);
         if(split) {
@@ -405,6 +436,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
             A(&d.aidx, d.nnz);
         }
     });
+    if(!rc) set_stage(d, split, dq_doubles(d, split, d.ws != nullptr));
     if(!rc) rc = reset_err_on(m, s);
     if(!rc && split) rc = cuda_ok(cudaMemsetAsync(d.slowq_n, 0, sizeof(int32_t), s));
     if(!rc && split) rc = setup_self(m, s);
@@ -526,7 +558,10 @@ int sfx_ctx_synchronize(sfx_ctx* ctx) {
 int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
                               int64_t nnz, int32_t precision) {
     const int64_t S = dim + 2, n = n_cells, F = n_faces;
-    int64_t cells = n * (8 * (2 * dim + 2 + 3 * S) + 4) + 4;
+    const bool split = precision == SFX_PREC_SPLIT;
+    const size_t dq = (size_t)F * (split ? split_dq_doubles(dim) : rec_doubles(dim, SFX_REC_DQ));
+    int64_t cells = n * (8 * (2 * dim + 2 + 2 * S) + 4) + 4 +
+                    8 * (int64_t)stage_doubles(n, dim, split, dq);
     int64_t faces = F * (8 * (1 + 2 * dim) + 4 * 4);
     int64_t bytes = cells + faces + nnz * 4 + 8 * 8 * 1024 + 4096;
     if(precision != SFX_PREC_SPLIT) {
@@ -534,8 +569,8 @@ int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
          * order); face velocities */
         auto rec = [&](int what) { return (int64_t)sfx_fp64_record_bytes(dim, what); };
         bytes += n * (rec(SFX_REC_WS) + rec(SFX_REC_GREC)) +
-                 F * (rec(SFX_REC_DQ) + rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO) + 8 * dim + 4) +
-                 nnz * 4;
+                 F * (rec(SFX_REC_DQ) + rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO) + 8 * dim) +
+                 4 * sfx_fp64_list_room(F) + nnz * 4;
     } else {
         bytes += F * 8 * (dim + S); /* face velocities, dQf */
     }
@@ -759,7 +794,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         if(!aidx.empty()) A(&d.aidx, nnz);
         A(&d.W, n * S);
         A(&d.Q, n * S);
-        A(&d.stage, stage_doubles(d));
+        add_stage(arrays, d, split, dq_doubles(d, split, records));
         A(&d.area, F);
         A(&d.mid, F * dim);
         A(&d.left, F);
@@ -798,6 +833,7 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         sfx_mesh_free(m);
         return rc;
     }
+    set_stage(d, split, dq_doubles(d, split, d.ws != nullptr));
     cudaStream_t s = ctx->stream;
     /* the dQ scratch holds dim doubles per face, the state staging per cell */
     double* fstage = split ? d.dq : d.dQf;
@@ -824,7 +860,8 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
     if(!rc && split) rc = sfx_split_prepare(&d, s);
     if(!rc && split) rc = setup_self(m, s);
     if(!rc && d.ws) rc = sfx_fp64_face_records(&d, s);
-    if(!rc && d.ws) rc = sfx_fp64_state_records(&d, s);
+    if(!rc && d.ws)
+        rc = cuda_ok(cudaMemsetAsync(d.ws, 0, sizeof(double) * n * rec_doubles(dim, SFX_REC_WS), s));
     /* host staging buffers go out of scope: wait for the copies */
     if(!rc) rc = cuda_ok(cudaStreamSynchronize(s));
     if(rc != SFX_OK) {
@@ -859,19 +896,50 @@ int sfx_state_upload_WQ(sfx_mesh* m, const double* W, const double* Q) {
     if(!m || !W || !Q) return SFX_ERR_INVALID;
     const int64_t n = m->d.n_cells;
     cudaStream_t s = m->ctx->stream;
+    const sfx_dmesh& d = m->d;
     SFX_TRY(reset_err(m));
-    SFX_TRY(rows_in(m->d.W, W, n, m->d.S, m->d.stage, s));
-    SFX_TRY(rows_in(m->d.Q, Q, n, m->d.S, m->d.stage, s));
+    const size_t ns = (size_t)n * d.S;
+    SFX_TRY(h2d(d.stage, W, ns, s));
+    SFX_TRY(h2d(d.stage2, Q, ns, s));
     if(m->ctx->cfg.precision == SFX_PREC_SPLIT)
-        SFX_TRY(sfx_split_load_state(&m->d, s));
-    else if(m->d.ws)
-        SFX_TRY(sfx_fp64_state_records(&m->d, s));
+        SFX_TRY(sfx_split_load_state(&d, d.stage, d.stage2, s));
+    else
+        SFX_TRY(sfx_fp64_load_rows(&d, d.stage, d.stage2, s));
     return cuda_ok(cudaStreamSynchronize(s));
+}
+
+/* States of at most this many doubles are transposed on the host: 1,200 doubles of
+ * W and of Q take 24 us so (plain FP64, both in one copy) and 45 with two copies
+ * and the transposing launches; 8,000 take 41 (12,000 with the launches 60). */
+constexpr size_t kSmallState = 8192;
+
+static int download_small(sfx_mesh* m, double* W, double* Q) {
+    const sfx_dmesh& d = m->d;
+    const size_t n = (size_t)d.n_cells, ns = n * d.S;
+    cudaStream_t s = m->ctx->stream;
+    double t[2 * kSmallState + 64];
+    const bool split = m->ctx->cfg.precision == SFX_PREC_SPLIT;
+    /* plain FP64: W and Q, neighbours in the mesh's block, in one copy */
+    const double* from = split ? d.Q : d.W;
+    const size_t at = (size_t)(d.Q - from);
+    if(split) {
+        SFX_TRY(sfx_split_W_rows(&d, d.stage, s));
+        SFX_TRY(cuda_ok(cudaMemcpyAsync(W, d.stage, sizeof(double) * ns, cudaMemcpyDeviceToHost, s)));
+    }
+    SFX_TRY(cuda_ok(cudaMemcpyAsync(t, from, sizeof(double) * (at + ns), cudaMemcpyDeviceToHost, s)));
+    SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
+    for(size_t i = 0; i < n; ++i)
+        for(int k = 0; k < d.S; ++k) {
+            if(!split) W[i * d.S + k] = t[k * n + i];
+            Q[i * d.S + k] = t[at + k * n + i];
+        }
+    return SFX_OK;
 }
 
 int sfx_state_download(sfx_mesh* m, double* W, double* Q) {
     if(!m) return SFX_ERR_INVALID;
     cudaStream_t s = m->ctx->stream;
+    if(W && Q && (size_t)m->d.n_cells * m->d.S <= kSmallState) return download_small(m, W, Q);
     SFX_TRY(sfx_mesh_download_async(m, W, Q, s));
     return cuda_ok(cudaStreamSynchronize(s));
 }
@@ -984,7 +1052,7 @@ static int move_gradients(sfx_mesh* m, double* out, const double* in) {
     if(m->ctx->cfg.precision != SFX_PREC_FP64) return SFX_ERR_UNSUPPORTED;
     cudaStream_t s = m->ctx->stream;
     const int w = d.dim * d.S;
-    const int64_t n = d.n_cells, part = std::max<int64_t>(1, n / d.dim);
+    const int64_t n = d.n_cells, part = gradient_rows(d);
     const int64_t rs = d.grec ? (int64_t)rec_doubles(d.dim, SFX_REC_GREC) : 1;
     const int64_t cs = d.grec ? 1 : n;
     double* g = d.grec ? d.grec : d.grad;
@@ -1196,14 +1264,18 @@ int64_t sfx_mesh_clone_bytes(sfx_mesh* base, int32_t precision) {
     if(!base) return -1;
     const sfx_dmesh& b = base->d;
     const int64_t n = b.n_cells, F = b.n_faces, S = b.S, D = b.dim;
-    int64_t bytes = n * S * 24 + (S + 1) * 1024 * 8 + 64;
+    const bool split = precision == SFX_PREC_SPLIT;
+    const size_t dq = (size_t)F * (split ? split_dq_doubles((int)D) : rec_doubles((int)D, SFX_REC_DQ));
+    int64_t bytes = n * S * 16 + 8 * (int64_t)stage_doubles(n, (int)D, split, dq) +
+                    (S + 1) * 1024 * 8 + 64;
     if(precision == SFX_PREC_SPLIT)
         bytes += n * 32 + n * 16 * (sfx_split_grad_vec4((int)D) + sfx_split_dwdt_vec4((int)D)) +
                  F * 8 * split_dq_doubles((int)D) +
                  4 * (int64_t)slowq_capacity(F) + 4 + (int64_t)sizeof(sfx_group_entry) + 28;
     else {
         auto rec = [&](int what) { return (int64_t)sfx_fp64_record_bytes((int)D, what); };
-        bytes += n * (rec(SFX_REC_WS) + rec(SFX_REC_GREC)) + F * (8 + rec(SFX_REC_DQ)) + 512;
+        bytes += n * (rec(SFX_REC_WS) + rec(SFX_REC_GREC)) + F * (4 + rec(SFX_REC_DQ)) +
+                 4 * sfx_fp64_list_room(F) + 512;
         if(b.fg && !b.ggeo) /* of a split mesh: face records and CSR of its own */
             bytes += F * (rec(SFX_REC_GGEO) + rec(SFX_REC_FGEO)) + (int64_t)b.nnz * 16 + 1280;
     }
@@ -1278,7 +1350,7 @@ int sfx_mesh_upload_W_async(sfx_mesh* m, const double* W, void* stream) {
     SFX_TRY(reset_err_on(m, s));
     SFX_TRY(h2d(m->d.stage, W, (size_t)m->d.n_cells * m->d.S, s));
     SFX_TRY(sfx_fp64_init_Q(&m->d, &m->ctx->sp, m->d.stage, s));
-    if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_load_state(&m->d, s));
+    if(m->ctx->cfg.precision == SFX_PREC_SPLIT) SFX_TRY(sfx_split_load_state(&m->d, nullptr, nullptr, s));
     return SFX_OK;
 }
 

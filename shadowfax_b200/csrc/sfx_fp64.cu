@@ -338,15 +338,22 @@ __global__ void __launch_bounds__(256) k_csr_neighbours(sfx_dmesh m) {
     m.ent[j] = make_int2((int)e, nb);
 }
 
-/* W and Q[0] (field-major) -> ws */
+/* rows of W and Q -> W, Q (field-major) and, where the mesh has records, ws */
 template <int D>
-__global__ void k_state_records(sfx_dmesh m) {
+__global__ void __launch_bounds__(128) k_load_rows(sfx_dmesh m, const double* W, const double* Q) {
     constexpr int S = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= m.n_cells) return;
+#pragma unroll
+    for(int k = 0; k < S; ++k) {
+        m.W[(size_t)k * m.n_cells + i] = W[(size_t)i * S + k];
+        m.Q[(size_t)k * m.n_cells + i] = Q[(size_t)i * S + k];
+    }
+    if(!m.ws) return;
     double* w = m.ws + (size_t)i * Rec<D>::ws;
-    for(int k = 0; k < S; ++k) w[k] = m.W[(size_t)k * m.n_cells + i];
-    w[S] = m.Q[i];
+#pragma unroll
+    for(int k = 0; k < S; ++k) w[k] = W[(size_t)i * S + k];
+    w[S] = Q[(size_t)i * S];
 }
 
 /* ------------------------------ gradients ------------------------------ */
@@ -1808,6 +1815,9 @@ __global__ void __launch_bounds__(kExactBlock, 2)
  * lowest failing face, and that one may be listed (after a failure of an
  * earlier step or phase the list is empty). */
 constexpr int kListedBlock = 128, kListedBlocks = 4 * kSfxSMs;
+/* one wave of blocks waits for its longest face whichever way it is sorted, and a
+ * second launch would add to that: the list from two blocks on every SM */
+constexpr int kListFrom = 2 * kSfxSMs * kExactBlock;
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(kListedBlock)
@@ -2374,6 +2384,10 @@ int sfx_fp64_record_bytes(int dim, int what) {
     return (int)sizeof(double) * (dim == 3 ? v3 : v2)[what];
 }
 
+int64_t sfx_fp64_list_room(int64_t n_faces) {
+    return n_faces > kListFrom ? n_faces : 0;
+}
+
 int sfx_from_rows(const double* rows, int64_t n, int w, double* out, void* stream) {
     if(n == 0) return SFX_OK;
     k_from_rows<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(rows, n, w, out);
@@ -2418,12 +2432,13 @@ int sfx_fp64_face_records(const sfx_dmesh* m, void* stream) {
     return cuda_status(cudaGetLastError());
 }
 
-int sfx_fp64_state_records(const sfx_dmesh* m, void* stream) {
+int sfx_fp64_load_rows(const sfx_dmesh* m, const double* W, const double* Q, void* stream) {
+    if(m->n_cells == 0) return SFX_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if(m->dim == 3)
-        k_state_records<3><<<grid_for(m->n_cells, 128), 128, 0, s>>>(*m);
+        k_load_rows<3><<<grid_for(m->n_cells, 128), 128, 0, s>>>(*m, W, Q);
     else
-        k_state_records<2><<<grid_for(m->n_cells, 128), 128, 0, s>>>(*m);
+        k_load_rows<2><<<grid_for(m->n_cells, 128), 128, 0, s>>>(*m, W, Q);
     sfx_count_launches(1);
     return cuda_status(cudaGetLastError());
 }
@@ -2471,10 +2486,7 @@ static int launch_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double 
         k_faces<D, SFX_SOLVER_EXACT, MODE><<<G, B, 0, s>>>(*m, *sp, dt, write_branch);
         return 1;
     } else {
-        /* one wave of blocks waits for its longest face whichever way it is
-         * sorted, and a second launch would add to that: the list from two
-         * blocks on every SM */
-        const int list = nf > 2 * kSfxSMs * kExactBlock;
+        const int list = nf > kListFrom;
         k_faces_exact<D, MODE><<<grid_for(nf, kExactBlock), kExactBlock, 0, s>>>(
                 *m, *sp, dt, write_branch, list);
         if(!list) return 1;

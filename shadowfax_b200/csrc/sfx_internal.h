@@ -64,7 +64,7 @@ struct sfx_dmesh {
     double* ggeo;
     double* fgeo;
     /* plain-FP64 exact solver: the faces solved by the second launch of a step
-     * (room for every face) and their number */
+     * (room for sfx_fp64_list_room) and their number */
     int32_t* listed;
     int32_t* listed_n;
     int32_t gshare; /* every local face's right position equals its right cell's */
@@ -118,8 +118,11 @@ struct sfx_dmesh {
     double t_total;
     double* an;
     double* dq;
-    double* stage; /* [n][S] rows on their way between W or Q and the host; no kernel of a
-                      step touches it */
+    double* stage; /* rows on their way between the mesh and the host.  Plain FP64: inside
+                      dQf, dead between steps, where that holds two states; otherwise an
+                      array that no kernel of a step touches (a split mesh may be read on
+                      its context's stream while a group steps it on another) */
+    double* stage2; /* a second state's rows on their way in */
     /* exact solver, split pass: faces whose p* iteration falls back to
      * Brent's method are queued here by the face kernel (face ids; room for
      * every face; slowq_n counts them) and solved by a follow-up launch in
@@ -195,9 +198,12 @@ enum { SFX_REC_WS, SFX_REC_GREC, SFX_REC_DQ, SFX_REC_GGEO, SFX_REC_FGEO };
 int sfx_fp64_record_bytes(int dim, int what); /* bytes of one record */
 /* ent from idx and the face list */
 int sfx_fp64_csr_neighbours(const sfx_dmesh* m, void* stream);
-/* the face geometry records of an uploaded mesh; the state records from W, Q */
+/* the face geometry records of an uploaded mesh */
 int sfx_fp64_face_records(const sfx_dmesh* m, void* stream);
-int sfx_fp64_state_records(const sfx_dmesh* m, void* stream);
+/* faces the second launch of a step may be given (0: it has none) */
+int64_t sfx_fp64_list_room(int64_t n_faces);
+/* W, Q (and the state records) from rows [n][S] */
+int sfx_fp64_load_rows(const sfx_dmesh* m, const double* W, const double* Q, void* stream);
 int sfx_fp64_gradients(const sfx_dmesh* m, const sfx_solver_params* sp, void* stream);
 int sfx_fp64_faces(const sfx_dmesh* m, const sfx_solver_params* sp, double dt,
                    int write_branch, void* stream);
@@ -240,7 +246,8 @@ int sfx_fp64_riemann(int dim, const sfx_solver_params* sp, int n,
 
 /* FP32/FP64-split kernels (sfx_split.cu) */
 int sfx_split_prepare(const sfx_dmesh* m, void* stream);
-int sfx_split_load_state(const sfx_dmesh* m, void* stream);
+/* the cell records from W and Q; rows W, Q [n][S] != NULL: W and Q from those first */
+int sfx_split_load_state(const sfx_dmesh* m, const double* W, const double* Q, void* stream);
 /* W (FP64 SoA) from the FP32 cell records */
 int sfx_split_export_W(const sfx_dmesh* m, void* stream);
 /* the same as rows [n][S], for downloads */

@@ -349,15 +349,22 @@ __global__ void k_prep_cells(sfx_dmesh m) {
     m.cx[i] = make_float4(v[0], v[1], v[2], (float)m.vol[i]);
 }
 
-/* W (FP64 SoA) and Q (FP64 SoA) -> FP32 cell records */
+/* W (FP64 SoA) and Q (FP64 SoA), or rows of them stored there first, -> FP32
+ * cell records */
 template <int D>
-__global__ void k_load_state(sfx_dmesh m) {
+__global__ void k_load_state(sfx_dmesh m, const double* Wr, const double* Qr) {
     constexpr int S = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= m.n_cells) return;
     const int n = m.n_cells;
     float W[S];
-    for(int k = 0; k < S; ++k) W[k] = (float)m.W[(size_t)k * n + i];
+    for(int k = 0; k < S; ++k) {
+        if(Wr) {
+            m.W[(size_t)k * n + i] = Wr[(size_t)i * S + k];
+            m.Q[(size_t)k * n + i] = Qr[(size_t)i * S + k];
+        }
+        W[k] = (float)m.W[(size_t)k * n + i];
+    }
     store_cell<D>(m.cw, i, W, (float)m.Q[i], (float)m.tarea[i]);
 }
 
@@ -2442,12 +2449,12 @@ int sfx_split_prepare(const sfx_dmesh* m, void* stream) {
     return launched(m->n_faces ? 2 : 1);
 }
 
-int sfx_split_load_state(const sfx_dmesh* m, void* stream) {
+int sfx_split_load_state(const sfx_dmesh* m, const double* W, const double* Q, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if(m->dim == 3)
-        k_load_state<3><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m);
+        k_load_state<3><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m, W, Q);
     else
-        k_load_state<2><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m);
+        k_load_state<2><<<grid_for(m->n_cells, 256), 256, 0, s>>>(*m, W, Q);
     return launched(1);
 }
 
