@@ -49,6 +49,8 @@ struct sfx_mesh {
     int32_t* split_idx = nullptr;
     int2* split_ent = nullptr;
     unsigned long long* d_smin = nullptr; /* local time steps: smallest new step */
+    /* room for d.vgen, d.newpos and d.vel in the block of a small mesh (keeps_moving) */
+    double *kept_vgen = nullptr, *kept_newpos = nullptr, *kept_vel = nullptr;
 };
 
 namespace {
@@ -265,6 +267,13 @@ void set_stage(sfx_dmesh& d, bool split, size_t dq) {
     const size_t ns = (size_t)d.n_cells * d.S;
     if(!d.stage) d.stage = d.dQf;
     d.stage2 = split && dq >= ns ? d.dq : d.stage + ns;
+}
+
+/* Whether an upload sets aside the arrays of a moving step: a mesh whose first
+ * step_moving allocates them pays 250 to 350 us for it and as much when it is
+ * freed, more than the step; they are at most a megabyte here. */
+bool keeps_moving(int dim, int64_t n, int64_t F) {
+    return 8 * dim * (2 * n + F) <= 1 << 20;
 }
 
 /* a plain-FP64 mesh's state and per-step scratch: the pass's records, or without
@@ -582,6 +591,7 @@ int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
                       16) + 256;
     }
     bytes += nnz * 8; /* ent */
+    if(keeps_moving(dim, n, F)) bytes += 16 * dim * n;
     return bytes;
 }
 
@@ -802,6 +812,11 @@ int sfx_mesh_upload(sfx_ctx* ctx, const sfx_mesh_desc* desc, sfx_mesh** out) {
         A(&d.kind, F);
         A(&d.rpos, F * dim);
         if(d.has_velocity) A(&d.vel, F * dim);
+        if(keeps_moving(dim, n, F)) {
+            A(&m->kept_vgen, n * dim);
+            A(&m->kept_newpos, n * dim);
+            if(!d.has_velocity) A(&m->kept_vel, F * dim);
+        }
         A(&d.branch, F);
         A(&d.err, 1);
         A(&d.totals_scratch, (size_t)(S + 1) * 1024);
@@ -966,10 +981,13 @@ int sfx_step_moving(sfx_mesh* m, double dt, int32_t periodic, double* positions,
     const int64_t n = d.n_cells, F = d.n_faces;
     const int D = d.dim;
     const bool fresh = d.vel == nullptr;
+    if(!d.vgen) d.vgen = m->kept_vgen;
+    if(!d.newpos) d.newpos = m->kept_newpos;
+    if(!d.vel) d.vel = m->kept_vel;
     Carver first; /* one allocation: a moving mesh takes one step per tessellation */
     if(!d.vgen) first.add(&d.vgen, (size_t)D * n);
     if(!d.newpos) first.add(&d.newpos, (size_t)D * n);
-    if(fresh) first.add(&d.vel, (size_t)D * F);
+    if(!d.vel) first.add(&d.vel, (size_t)D * F);
     if(!first.slots.empty()) SFX_TRY(first.allocate(m));
     d.has_velocity = 1;
     SFX_TRY(reset_err(m));
@@ -1003,7 +1021,9 @@ static int ensure_local(sfx_mesh* m) {
         SFX_TRY(cuda_ok(cudaMemsetAsync(d.tend, 0, sizeof(uint64_t) * n, s)));
     }
     if(!d.vgen) {
-        SFX_TRY(dalloc(m, &d.vgen, (size_t)d.dim * n));
+        double* vgen = m->kept_vgen;
+        if(!vgen) SFX_TRY(dalloc(m, &vgen, (size_t)d.dim * n));
+        d.vgen = vgen;
         SFX_TRY(cuda_ok(cudaMemsetAsync(d.vgen, 0, sizeof(double) * d.dim * n, s)));
     }
     if(!m->d_smin) SFX_TRY(dalloc(m, &m->d_smin, 1));
