@@ -1962,7 +1962,14 @@ __device__ __forceinline__ void queue_faces(const sfx_dmesh& m, bool push, int f
 }
 
 /* ------------------------------- update ------------------------------- */
-template <int D, int LPC>
+/* Faces in flight per lane: 464,159 cells in 2D took 39 us with 1, 35 with 3, 38
+ * with 6 (64 registers).  In a launch of at most a block per SM registers are
+ * free, and a cell's gathers are two round trips instead of five: 3D, one lane a
+ * cell, a step of 1,000 to 6,000 cells (HLLC) 33.0 to 35.6 us with 3, 31.5 to 33.6
+ * with 8 or 16 (four lanes a cell and 1 face in flight: 32.1 to 34.3) */
+constexpr int kUpdateFaces = 3, kUpdateFacesSmall = 8;
+
+template <int D, int LPC, int U>
 __device__ __forceinline__ void sapply_body(const sfx_dmesh& m, const double gamma,
                                             const int t) {
     constexpr int S = D + 2;
@@ -1976,9 +1983,7 @@ __device__ __forceinline__ void sapply_body(const sfx_dmesh& m, const double gam
     const int end = live ? __ldg(m.off + i + 1) : 0;
     /* each lane sums every LPC-th face in FP64; the group then adds the lanes'
      * partial sums in a fixed tree, so reruns are bitwise identical */
-    /* faces in flight per lane: 1 took 39 us on 464,159 cells in 2D, 3 takes 35,
-     * 6 take 38 (64 registers) */
-    constexpr int U = 3;
+    /* U faces in flight (kUpdateFaces; the sum's order does not depend on it) */
     for(int j = beg + lane; j < end; j += U * LPC) {
         unsigned e[U];
         double v[U][S];
@@ -2307,12 +2312,12 @@ __global__ void __launch_bounds__(kSlowBlock)
     }
 }
 
-template <int D, int LPC>
+template <int D, int LPC, int U>
 __global__ void __launch_bounds__(256) k_group_sapply(const sfx_group_entry* tab, const int* pre,
                                                       int nm, double gamma) {
     const int mi = group_mesh_of_block(pre, nm);
     if(member_done(tab, mi)) return;
-    sapply_body<D, LPC>(tab[mi].m, gamma, (blockIdx.x - __ldg(pre + mi)) * blockDim.x + threadIdx.x);
+    sapply_body<D, LPC, U>(tab[mi].m, gamma, (blockIdx.x - __ldg(pre + mi)) * blockDim.x + threadIdx.x);
 }
 
 /* after a step: count the members' remaining steps down */
@@ -2415,9 +2420,14 @@ int group_phase(const sfx_group_dev* g, int phase, const sfx_solver_params* sp,
             }
         }
     } else {
-        if(g->blocks[2])
-            k_group_sapply<D, sfx_update_lanes(LPC)><<<g->blocks[2], 256, 0, s>>>(
-                    g->tab, g->pre + 2 * (nm + 1), nm, sp->gamma);
+        const int* pre2 = g->pre + 2 * (nm + 1);
+        constexpr int lanes = sfx_update_lanes(LPC);
+        if(D == 3 && lanes == 1 && g->blocks[2] > 0 && g->blocks[2] <= kSfxSMs)
+            k_group_sapply<D, lanes, kUpdateFacesSmall>
+                    <<<g->blocks[2], 256, 0, s>>>(g->tab, pre2, nm, sp->gamma);
+        else if(g->blocks[2])
+            k_group_sapply<D, lanes, kUpdateFaces>
+                    <<<g->blocks[2], 256, 0, s>>>(g->tab, pre2, nm, sp->gamma);
     }
     if(g->blocks[phase]) sfx_count_launches(1);
     return cudaGetLastError() == cudaSuccess ? SFX_OK : SFX_ERR_CUDA;
