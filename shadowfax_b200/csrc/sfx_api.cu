@@ -313,8 +313,8 @@ int64_t gradient_rows(const sfx_dmesh& d) {
 }
 
 /* the arrays that add(arrays, records) names: with the plain-FP64 records, or,
- * where those do not fit on the device, without (3D: 1,300 bytes per cell
- * instead of 3,550; the same bits from the kernels of caller-owned arrays: 419 us
+ * where those do not fit on the device, without (3D: 1,180 bytes per cell
+ * instead of 3,430; the same bits from the kernels of caller-owned arrays: 419 us
  * a step instead of 172 on 65,537 cells in 3D with HLLC, 838 instead of 376 with
  * the exact solver, 181 instead of 128 on 150,001 cells in 2D with HLLC) */
 template <typename Add>

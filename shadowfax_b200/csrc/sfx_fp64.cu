@@ -512,12 +512,13 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src) {
  * kGradStages faces ahead (lane k of a cell copies 16 bytes of the geometry
  * and one variable): no registers hold loads in flight.  Both loops divided
  * per face before, the first one in a kernel of its own that wrote 128 bytes
- * per face: 220 -> 83 us on 65,537 cells in 3D, 104 -> 63 us on 150,001 in 2D
- * (109 and 68 us without the ring; 88 and 66 without the kept midpoints).  96
- * registers in 3D: 102 left four blocks per SM instead of five (87 us), 80 spill
- * (86).  Two faces per ring stage: 85.  Cells sorted by face count so that a
- * warp's lanes run equally long: 83 us, but the update in that order lost
- * more than that to a lower L1 hit rate. */
+ * per face: 220 -> 83 us (event-timed; 80 in a profile) on 65,537 cells in 3D,
+ * 104 -> 63 us on 150,001 in 2D (109 and 68 us without the ring; 88 and 66
+ * without the kept midpoints).  96 registers in 3D: 102 left four blocks per SM
+ * instead of five (87 us), 80 spill (86).  Two faces per ring stage: 85.  Cells
+ * sorted by face count so that a warp's lanes run equally long: 83 us where this
+ * took 88, but the update in that order lost more than that to a lower L1 hit
+ * rate. */
 constexpr int kGradBlock = 128, kGradStages = 4;
 
 template <int D>

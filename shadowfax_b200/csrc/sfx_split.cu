@@ -873,8 +873,8 @@ __device__ __forceinline__ void thllc(T g, const T* WL, const T* WRin, const T* 
          * whose launch took 60 us however few faces it solved (its code is
          * fetched for them alone): 450,000 faces in 2D, 3.4% and 40% of them
          * vacuum, 89.5 and 103 -> 25.6 us; 530,000 in 3D 86 and 115 -> 31.8 us;
-         * without vacuum faces 57.5 -> 50.2 us (1.4 million, 2D), 85.2 -> 82.4
-         * (2.1 million, 3D). */
+         * a handful of vacuum faces 57.5 -> 50.2 us (1.4 million, 2D), 85.2 ->
+         * 81.6 (2.1 million, 3D). */
         const T a = left ? aL : aR, v = left ? uL : -uR;
         if(v < a) {
             if(!(v + two * a / gm1 > zero)) return;
