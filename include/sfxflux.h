@@ -187,7 +187,7 @@ int sfx_mesh_check(const sfx_mesh_desc* desc, int32_t precision);
 int sfx_mesh_free(sfx_mesh* mesh);
 /* bytes of device memory a mesh of this size takes (admission control).  A plain-FP64
  * mesh or clone that does not fit so is stored without the records its kernels
- * read (3D: 1,180 bytes per cell instead of 3,430), with the same results, slower. */
+ * read (3D: 1,220 bytes per cell instead of 3,470), with the same results, slower. */
 int64_t sfx_mesh_device_bytes(int32_t dim, int32_t n_cells, int32_t n_faces,
                               int64_t n_cell_faces, int32_t precision);
 

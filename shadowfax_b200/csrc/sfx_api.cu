@@ -251,26 +251,22 @@ struct Carver {
     }
 };
 
-/* The staging rows: two states, or one and a row of gradients.  Plain FP64: in
- * dQf when that is large enough (dq doubles), an array otherwise; split: one
- * state in an array, the second in dq, where a state on its way in may go.
- * stage_doubles: of the array (0: in dQf). */
+/* The staging rows: a state, and for plain FP64 at least one row of gradients and
+ * all of a small mesh's; a second state on its way in goes through the dQ scratch
+ * (dq doubles) when that holds it, otherwise behind the first. */
 size_t stage_doubles(int64_t n, int dim, bool split, size_t dq) {
     const size_t ns = (size_t)n * (dim + 2), row = (size_t)dim * (dim + 2);
-    if(split) return dq >= ns ? ns : 2 * ns;
-    return dq >= std::max(2 * ns, row) ? 0 : std::max(2 * ns, row);
+    const size_t rows = split ? 0 : std::max(row, std::min<size_t>(n * row, 16384));
+    return std::max(dq >= ns ? ns : 2 * ns, rows);
 }
 
 void add_stage(Carver& arrays, sfx_dmesh& d, bool split, size_t dq) {
-    d.stage = d.stage2 = nullptr;
-    const size_t count = stage_doubles(d.n_cells, d.dim, split, dq);
-    if(count) arrays.add(&d.stage, count);
+    arrays.add(&d.stage, stage_doubles(d.n_cells, d.dim, split, dq));
 }
 
 void set_stage(sfx_dmesh& d, bool split, size_t dq) {
     const size_t ns = (size_t)d.n_cells * d.S;
-    if(!d.stage) d.stage = d.dQf;
-    d.stage2 = split && dq >= ns ? d.dq : d.stage + ns;
+    d.stage2 = dq < ns ? d.stage + ns : split ? d.dq : d.dQf;
 }
 
 /* Whether an upload sets aside the arrays of a moving step: a mesh whose first
@@ -305,16 +301,9 @@ size_t dq_doubles(const sfx_dmesh& d, bool split, bool records) {
                       : records ? rec_doubles(d.dim, SFX_REC_DQ) : (size_t)d.S);
 }
 
-/* rows of gradients that fit in a plain-FP64 mesh's staging rows */
-int64_t gradient_rows(const sfx_dmesh& d) {
-    const size_t dq = dq_doubles(d, false, d.ws != nullptr);
-    const size_t held = stage_doubles(d.n_cells, d.dim, false, dq);
-    return (int64_t)((held ? held : dq) / ((size_t)d.dim * d.S));
-}
-
 /* the arrays that add(arrays, records) names: with the plain-FP64 records, or,
- * where those do not fit on the device, without (3D: 1,180 bytes per cell
- * instead of 3,430; the same bits from the kernels of caller-owned arrays: 419 us
+ * where those do not fit on the device, without (3D: 1,220 bytes per cell
+ * instead of 3,470; the same bits from the kernels of caller-owned arrays: 419 us
  * a step instead of 172 on 65,537 cells in 3D with HLLC, 838 instead of 376 with
  * the exact solver, 181 instead of 128 on 150,001 cells in 2D with HLLC) */
 template <typename Add>
@@ -395,7 +384,7 @@ int clone_impl(sfx_ctx* ctx, sfx_mesh* base, cudaStream_t s, bool wait, sfx_mesh
     sfx_dmesh& d = m->d;
     const int64_t n = d.n_cells, F = d.n_faces;
     const int S = d.S, dim = d.dim;
-    d.W = d.Q = d.grad = d.dQf = d.ws = d.grec = nullptr;
+    d.W = d.Q = d.stage = d.stage2 = d.grad = d.dQf = d.ws = d.grec = nullptr;
     d.listed = d.listed_n = nullptr;
     d.branch = nullptr;
     d.err = nullptr;
@@ -1073,7 +1062,7 @@ int sfx_mesh_get_timesteps(sfx_mesh* m, uint64_t* start, uint64_t* end) {
 }
 
 /* host gradients [n][dim*S] from or to the mesh's records (gradients [l][k] first) or
- * field-major arrays, through the staging rows, n / dim cells at a time (a copy of
+ * field-major arrays, through the staging rows, as many cells at a time as fit (a copy of
  * the records with the host picking the gradients out took 920 us to set and 680
  * to get for 30,000 cells in 2D; these take 128 and 178) */
 static int move_gradients(sfx_mesh* m, double* out, const double* in) {
@@ -1081,17 +1070,22 @@ static int move_gradients(sfx_mesh* m, double* out, const double* in) {
     if(m->ctx->cfg.precision != SFX_PREC_FP64) return SFX_ERR_UNSUPPORTED;
     cudaStream_t s = m->ctx->stream;
     const int w = d.dim * d.S;
-    const int64_t n = d.n_cells, part = gradient_rows(d);
+    const int64_t n = d.n_cells;
+    /* on their way in through the dQ scratch when that holds them all */
+    const size_t dq = dq_doubles(d, false, d.ws != nullptr);
+    const bool whole = in && dq >= (size_t)(n * w);
+    double* rows = whole ? d.dQf : d.stage;
+    const int64_t part = whole ? n : (int64_t)(stage_doubles(n, d.dim, false, dq) / w);
     const int64_t rs = d.grec ? (int64_t)rec_doubles(d.dim, SFX_REC_GREC) : 1;
     const int64_t cs = d.grec ? 1 : n;
     double* g = d.grec ? d.grec : d.grad;
     for(int64_t i = 0; i < n; i += part) {
         const int64_t count = std::min(part, n - i);
         const size_t bytes = sizeof(double) * (size_t)(count * w);
-        if(in) SFX_TRY(h2d(d.stage, in + i * w, (size_t)(count * w), s));
-        SFX_TRY(sfx_strided_rows(g + i * rs, rs, cs, count, w, d.stage, in != nullptr, s));
+        if(in) SFX_TRY(h2d(rows, in + i * w, (size_t)(count * w), s));
+        SFX_TRY(sfx_strided_rows(g + i * rs, rs, cs, count, w, rows, in != nullptr, s));
         if(out)
-            SFX_TRY(cuda_ok(cudaMemcpyAsync(out + i * w, d.stage, bytes, cudaMemcpyDeviceToHost, s)));
+            SFX_TRY(cuda_ok(cudaMemcpyAsync(out + i * w, rows, bytes, cudaMemcpyDeviceToHost, s)));
     }
     return cuda_ok(cudaStreamSynchronize(s));
 }
@@ -1239,7 +1233,6 @@ int sfx_flux_pass(sfx_mesh* m, double dt, double* grad, double* dQ_face,
         for(int64_t f = 0; f < F; ++f)
             for(int k = 0; k < S; ++k)
                 dQ_face[f * S + k] = m->d.ws ? tq[f * rec + k] : tq[(size_t)k * F + f];
-    /* last: the gradients' way to the host may go through dQf */
     if(grad && !split) SFX_TRY(sfx_mesh_get_gradients(m, grad));
     sfx_stats local;
     return check_err(m, st ? st : &local);

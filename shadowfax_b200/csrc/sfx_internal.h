@@ -118,10 +118,9 @@ struct sfx_dmesh {
     double t_total;
     double* an;
     double* dq;
-    double* stage; /* rows on their way between the mesh and the host.  Plain FP64: inside
-                      dQf, dead between steps, where that holds two states; otherwise an
-                      array that no kernel of a step touches (a split mesh may be read on
-                      its context's stream while a group steps it on another) */
+    double* stage;  /* rows on their way between the mesh and the host; no kernel of a step
+                       touches them (a state may be read on one stream while a step runs on
+                       another) */
     double* stage2; /* a second state's rows on their way in */
     /* exact solver, split pass: faces whose p* iteration falls back to
      * Brent's method are queued here by the face kernel (face ids; room for
