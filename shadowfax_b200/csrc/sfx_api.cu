@@ -1217,24 +1217,28 @@ int sfx_flux_pass(sfx_mesh* m, double dt, double* grad, double* dQ_face,
             for(int q = 0; q < D * S; ++q) grad[i * D * S + q] = tf[(size_t)i * G * 4 + q];
     }
     if(branch && split && F) SFX_TRY(cuda_ok(cudaMemsetAsync(m->d.branch, 0, 4 * F, s)));
-    /* dQ: rows (split, and the 2D records are rows), 3D records, or field-major */
-    const bool direct = split || (m->d.ws && D == 2);
-    const size_t rec = m->d.ws ? rec_doubles(D, SFX_REC_DQ) : (size_t)S;
-    std::unique_ptr<double[]> tq;
-    if(dQ_face && !direct) tq.reset(new(std::nothrow) double[F * rec + 1]);
-    if(dQ_face && !direct && !tq) return SFX_ERR_NOMEM;
-    if(dQ_face)
-        SFX_TRY(cuda_ok(cudaMemcpyAsync(direct ? dQ_face : tq.get(), m->d.dQf,
-                                        sizeof(double) * (size_t)F * (direct ? S : rec),
+    /* dQ: rows as they are (split, and the 2D records), or formed through the staging
+     * rows from the 3D records or field-major arrays */
+    if(dQ_face && (split || (m->d.ws && D == 2))) {
+        SFX_TRY(cuda_ok(cudaMemcpyAsync(dQ_face, m->d.dQf, sizeof(double) * (size_t)F * S,
                                         cudaMemcpyDeviceToHost, s)));
+    } else if(dQ_face) {
+        const int64_t rs = m->d.ws ? (int64_t)rec_doubles(D, SFX_REC_DQ) : 1;
+        const int64_t cs = m->d.ws ? 1 : F;
+        const size_t dq = dq_doubles(m->d, split, m->d.ws != nullptr);
+        const int64_t part = (int64_t)stage_doubles(n, D, split, dq) / S;
+        for(int64_t f = 0; f < F; f += part) {
+            const int64_t count = std::min(part, F - f);
+            SFX_TRY(sfx_strided_rows(m->d.dQf + f * rs, rs, cs, count, S, m->d.stage, 0, s));
+            SFX_TRY(cuda_ok(cudaMemcpyAsync(dQ_face + f * S, m->d.stage,
+                                            sizeof(double) * (size_t)(count * S),
+                                            cudaMemcpyDeviceToHost, s)));
+        }
+    }
     if(branch && F)
         SFX_TRY(cuda_ok(cudaMemcpyAsync(branch, m->d.branch, sizeof(int32_t) * F,
                                         cudaMemcpyDeviceToHost, s)));
     SFX_TRY(cuda_ok(cudaStreamSynchronize(s)));
-    if(dQ_face && !direct)
-        for(int64_t f = 0; f < F; ++f)
-            for(int k = 0; k < S; ++k)
-                dQ_face[f * S + k] = m->d.ws ? tq[f * rec + k] : tq[(size_t)k * F + f];
     if(grad && !split) SFX_TRY(sfx_mesh_get_gradients(m, grad));
     sfx_stats local;
     return check_err(m, st ? st : &local);
